@@ -137,7 +137,7 @@ class DecodeRunner:
         return StepInfo(n_tokens=B, n_seqs=B, max_q_len=1, max_kv_len=self.max_len,
                         tokens=self.view("tokens"), positions=self.view("positions"), tok_seq=self.view("tok_seq"),
                         cu_seqlens=self.view("cu_seqlens"), start_pos=self.view("start_pos"), slots=self.view("slots"),
-                        want_rows=self.view("want_rows"), page_tables=tables, slots_long=self.slots_long)
+                        want_rows=self.view("want_rows"), page_tables=tables, slots_long=self.slots_long, wants_every_row=True)
 
     # ------------------------------------------------------------------ one step's body
     def _body(self) -> None:

@@ -19,7 +19,7 @@ from ..config.model_config import ModelConfig
 from ..config.registry import build_model_spec, build_part
 from ..config.specs import ModelSpec
 from ..parts.base import CacheNeed, MixerMemory, Part, Runtime, StateSpec
-from ..parts.block import finish_deferred
+from ..parts.block import finish_deferred, norm_into
 from ..weights.loader import load_weights
 from .step_info import StepInfo
 
@@ -130,8 +130,10 @@ class Model:
         n_want = step.want_rows.numel()
         if n_want == 0:
             return rt.empty(0, self.config.vocab_size, dtype=torch.float32)
-        rows_x = rt.empty(n_want, x.shape[1], dtype=torch.float32)
-        rows_p = rt.empty(n_want, x.shape[1], dtype=torch.float32) if pending is not None else None
-        kernels.gather_rows(x, pending, step.want_rows, rows_x, rows_p)
-        h = self.parts.final_norm.forward(rows_x, rows_p)
-        return self.parts.head.forward(h)
+        if step.wants_every_row and pending is None:
+            rows_x, rows_p = x, None
+        else:
+            rows_x = rt.empty(n_want, x.shape[1], dtype=torch.float32)
+            rows_p = rt.empty(n_want, x.shape[1], dtype=torch.float32) if pending is not None else None
+            kernels.gather_rows(x, pending, step.want_rows, rows_x, rows_p)
+        return self.parts.head.forward(norm_into(self.parts.final_norm, self.parts.head, rows_x, rows_p))

@@ -14,7 +14,7 @@ from ..csrc import build as _build
 __all__ = [
     "KernelError", "KVView", "require_cuda", "dtype_code", "embed", "add_rmsnorm", "rope_table", "qkv_post",
     "attention_simt", "silu_mul", "gather_rows", "linear_simt", "argmax", "sample", "uniform_of", "core",
-    "launch_count", "reset_launch_count", "library_launch_count", "count_library_launches", "attention_mma_available", "attention_mma", "attention_mma_plan", "attention_decode_cluster_limit", "attention_decode_splits", "attention_decode_clusters_resident", "attention_tcgen05", "attention_tcgen05_takes", "attention_tcgen05_blocks", "attention_library", "gemm_tcgen05", "gemm_qkv_cluster_splits", "gemm_qkv_clusters_resident", "gemm_tcgen05_rows", "gemm_rows_takes", "gemm_rows_add_plan", "gemm_add_plan", "gemm_tcgen05_pair", "gemm_pair_takes", "gemm_prompt", "library_gemm", "gemm_status", "check_gemm_status", "set_pdl", "PinnedCopy", "decode_advance",
+    "launch_count", "reset_launch_count", "library_launch_count", "count_library_launches", "attention_mma_available", "attention_mma", "attention_mma_plan", "attention_decode_cluster_limit", "attention_decode_splits", "attention_decode_clusters_resident", "attention_tcgen05", "attention_tcgen05_takes", "attention_tcgen05_blocks", "attention_library", "gemm_tcgen05", "gemm_few", "gemm_few_plan", "gemm_qkv_cluster_splits", "gemm_qkv_clusters_resident", "gemm_tcgen05_rows", "gemm_rows_takes", "gemm_rows_add_plan", "gemm_add_plan", "gemm_tcgen05_pair", "gemm_pair_takes", "gemm_prompt", "library_gemm", "gemm_status", "check_gemm_status", "set_pdl", "PinnedCopy", "decode_advance",
     "layernorm", "qk_norm_rope_cache", "softcap", "convert", "causal_conv", "gated_delta_rule", "gated_rmsnorm", "block_gates",
     "linear_scan", "gates_scan_step", "gates_scan_step_takes",
     "moe_route", "moe_plan", "moe_plan_rows", "grouped_linear", "moe_gather", "moe_combine", "scaled_add", "scaled_add_experts", "gla", "gla_slices", "latent_prepare",
@@ -136,6 +136,7 @@ def core() -> ctypes.CDLL:
             "mlc_linear_simt": [P, I, P, I, P, I, I, I, I, P, LL, I, P],
             "mlc_attention_combine": [P, P, LL, I, I, P, I, P, I, P],
             "mlc_gemm_tcgen05": [P, P, P, I, I, I, I, I, I, I, P, P, I, P, P, P, P, I, I, I, I, P, P, P, LL, I, I, I, F, F, P],
+            "mlc_gemm_few": [P, P, F, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, P, I, I, I, I, P, P, P, LL, I, I, I, F, F, P],
             "mlc_gemm_tcgen05_rows": [P, P, P, I, I, I, I, I, I, I, P, I, P, P, P, P, I, I, I, I, P, P, P, LL, I, I, I, F, F, P],
             "mlc_gemm_tcgen05_pair": [P, P, P, I, I, I, I, I, I, I, P, I, I, F, F, P],
             "mlc_gemm_tcgen05_rows_grouped": [P, P, P, I, I, I, I, I, I, P, I, P, I, I, F, F, P],
@@ -1561,6 +1562,77 @@ def gemm_qkv_cluster_splits(n_tok: int, n_out: int, k: int, resident: tuple = No
         if per >= 12 and (splits - 1) * per < k_blocks and tiles <= fit:
             return splits
     return 1
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> Optional[tuple]:
+    """How csrc/gemm_few.cu takes a product (`plan` of `gemm_few`), or None where the tcgen05 form is the better one.
+
+    A warp takes `units` units of 64 columns; fewer warps with more units each have fewer parts to add up, more warps have
+    more loads under way.  The lines below were drawn on a B200 from sweeps over (warps, units, tiles, blocks, splits) in
+    chains of like kernels at the Qwen2-0.5B, 1.5B and 7B sizes (us, against the tcgen05 form, with its norm where there is one):
+      ADD      blocks x splits of about two an SM, at least 7 and at most 26 units a split.  8 rows: 896 x 896 1.5 against
+               2.3, 896 x 4,864 2.7 against 3.5, 1,536 x 8,960 5.8 against 6.6, 3,584 x 3,584 5.3 against 6.7; but 3,584 x
+               18,944 25.5 against 24.0: not above 40 M weights.  16 rows: 896 x 4,864 3.2 against 3.7, but 3,584 x 3,584 7.8
+               against 6.8 and 1,536 x 8,960 7.9 against 6.7: not above 5 M.  32 rows: 896 x 4,864 4.2 against 4.7.
+      QKV      a block per tile (at most one an SM).  8 rows: 1,152 x 896 2.5 against 6.6, 2,048 x 1,536 3.8 against 8.3,
+               4,608 x 3,584 9.2 against 13.5; 16 rows: 3.0, 4.6, 12.2 against 6.7, 8.5, 13.3; 32 rows: 1,152 x 896 5.2
+               against 7.0.
+      others   8 rows: 9,728 x 896 with SiLU 5.2 against 7.5, 17,920 x 1,536 10.6 against 13.1, 37,888 x 3,584 44.9 against
+               48.1, the head's 151,936 x 896 44.6 against 47.4; 16 rows: 6.4 against 7.5, 12.6 against 13.6, 3,584
+               columns slower; 24 rows: 9.1 against 8.9."""
+    if n_tok < 1 or n_tok > 32 or k < 64 or k % 64:
+        return None
+    units, tiles = k // 64, (n_out + 15) // 16
+    if epilogue == EPI_ADD:
+        if n_out * k > (40_000_000 if n_tok <= 8 else 5_000_000):
+            return None
+        splits = (units + 27) // 28 if tiles >= n_sms else max(1, min(units // 7, 2 * n_sms // tiles), (units + 25) // 26)
+        per = (units + splits - 1) // splits
+        splits = (units + per - 1) // per
+        uw = max(1 if per <= 2 else 2, (per + 13) // 14)
+        if uw > 2:
+            return None
+        rt = 2 if tiles < n_sms and tiles * splits > 2 * n_sms else 1
+        return ((per + uw - 1) // uw, uw, rt, min((tiles + rt - 1) // rt, n_sms), splits)
+    if epilogue == EPI_QKV:
+        uw = (units + 7) // 8 if n_tok <= 8 and units <= 24 else (units + 15) // 16
+        if uw > (4 if n_tok <= 16 else 1):
+            return None
+        return ((units + uw - 1) // uw, uw, 1, min(tiles, n_sms), 1)
+    uw = (units + 15) // 16
+    if uw > (4 if n_tok <= 8 else 2 if n_tok <= 16 else 0):
+        return None
+    rt = {1: 3, 2: 2}.get(uw, 1) if n_tok <= 8 else 1
+    blocks = n_sms if n_tok <= 8 and uw > 1 else 2 * n_sms
+    return ((units + uw - 1) // uw, uw, rt, min((tiles + rt - 1) // rt, blocks), 1)
+
+
+def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, plan: tuple, gain: Optional[torch.Tensor] = None,
+             eps: float = 0.0, bias: Optional[torch.Tensor] = None, positions: Optional[torch.Tensor] = None,
+             tok_seq: Optional[torch.Tensor] = None, rope: Optional[torch.Tensor] = None, q_heads: int = 0, kv_heads: int = 0,
+             head_dim: int = 0, kv: Optional[KVView] = None, glu=None) -> None:
+    """The product of up to 32 rows with the epilogues of `gemm_tcgen05` (see csrc/gemm_few.cu).  x: bfloat16 [n, K], or with
+    `gain` the float32 residual stream, whose RMS norm is multiplied.  `plan`: (warps of a block, units of 64 columns per warp,
+    tiles of 16 rows of w at a time, blocks that walk them, blocks that share the K range), as `gemm_few_plan` gives it."""
+    require_cuda(x, w, out, gain, bias, positions, tok_seq, rope)
+    n_tok, K = x.shape
+    n_out = w.shape[0]
+    if x.dtype != (torch.bfloat16 if gain is None else torch.float32) or w.dtype != torch.bfloat16:
+        raise KernelError("the few-row product takes bfloat16 weights and bfloat16 rows, or a float32 stream and its norm's gain")
+    if w.shape[1] != K or (gain is not None and (gain.dtype != torch.float32 or gain.numel() != K)):
+        raise KernelError(f"shapes do not agree: x {tuple(x.shape)}, w {tuple(w.shape)}")
+    wanted = {EPI_STORE: n_tok * n_out, EPI_ADD: n_tok * n_out, EPI_SILU_MUL: n_tok * (n_out // 2)}.get(epilogue, n_tok * q_heads * head_dim)
+    assert out.numel() == wanted and (epilogue != EPI_ADD or out.dtype == torch.float32)
+    if kv is not None:
+        assert kv.k_pool.dtype == out.dtype
+        cache = (kv.k_pool.data_ptr(), kv.v_pool.data_ptr(), kv.page_table.data_ptr(), kv.entry_offset, kv.pages_per_seq, kv.page_size)
+    else:
+        cache = (None, None, None, 0, 0, 1)
+    _check(core().mlc_gemm_few(x.data_ptr(), _ptr(gain), eps, w.data_ptr(), out.data_ptr(), dtype_code(out.dtype), n_tok, n_out, K,
+                               epilogue, *plan, _ptr(bias), _ptr(positions), _ptr(tok_seq), _ptr(rope),
+                               rope.shape[0] if rope is not None else 0, q_heads, kv_heads, head_dim, *cache, *_glu_args(glu),
+                               _stream()), "few-row matrix product")
 
 
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 0, n_splits: int = 1,

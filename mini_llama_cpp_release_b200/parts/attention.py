@@ -22,6 +22,7 @@ from ..config.registry import register_part, build_part
 from ..config.specs import PartSpec
 from .base import CacheNeed, MixerMemory, Part, TensorSpec
 from .linear import Linear
+from .norm import normed_rows
 
 
 @register_part("mixer", "gqa_attention")
@@ -103,11 +104,20 @@ class GQAttention(Part):
         b = self.qkv.nbytes() + self.o.nbytes()
         return b + (self.bias.numel() * 4 if self.bias is not None else 0)
 
+    def _few_plan(self, n: int, rows: int):
+        return kernels.gemm_few_plan(n, rows, self.hidden, kernels.bindings.EPI_QKV, self.runtime.n_sms) if self.fused else None
+
+    def takes_normed_stream(self, n: int) -> bool:
+        """Whether `forward` may be given a `NormedStream` of n rows: whichever rows of the projection it will use.  (A class
+        with a forward of its own is given finished rows.)"""
+        return type(self).forward is GQAttention.forward and all(self._few_plan(n, r) is not None for r in (self.H * self.hd, (self.H + 2 * self.KV) * self.hd))
+
     # ---- the step
     accumulates = True        # forward(..., residual=x) may add the branch into the float32 stream and return None
 
-    def forward(self, h: torch.Tensor, step, memory: MixerMemory, residual: Optional[torch.Tensor] = None):
+    def forward(self, h, step, memory: MixerMemory, residual: Optional[torch.Tensor] = None):
         rt = self.runtime
+        h, gain, eps = normed_rows(h)
         n = h.shape[0]
         if hasattr(self.position, "prepare"):
             self.position.prepare(step.max_kv_len)
@@ -126,6 +136,10 @@ class GQAttention(Part):
             kernels.gemm_tcgen05_rows(h, proj.weight, q, kernels.bindings.EPI_QKV, bias=bias, positions=step.positions,
                                       tok_seq=step.tok_seq, rope=table, q_heads=self.H, kv_heads=kv_heads, head_dim=self.hd,
                                       kv=memory.kv if memory.writes_cache else None, n_sms=rt.n_sms)
+        elif self.fused and (plan := self._few_plan(n, proj.weight.shape[0])) is not None:
+            kernels.gemm_few(h, proj.weight, q, kernels.bindings.EPI_QKV, plan, gain, eps, bias=bias, positions=step.positions,
+                             tok_seq=step.tok_seq, rope=table, q_heads=self.H, kv_heads=kv_heads, head_dim=self.hd,
+                             kv=memory.kv if memory.writes_cache else None)
         elif self.fused:
             # short epilogues in more blocks beat one long one; the few tiles' K range shared out over clusters of blocks
             splits = kernels.gemm_qkv_cluster_splits(n, proj.weight.shape[0], self.hidden) if n <= 64 else 1

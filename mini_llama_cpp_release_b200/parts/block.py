@@ -18,6 +18,14 @@ from ..config.specs import PartSpec
 from .base import MixerMemory, Part, TensorSpec
 
 
+def norm_into(norm, reader, x: torch.Tensor, pending: Optional[torch.Tensor]):
+    """The norm of the stream (which takes `pending` first) for the part that reads it; with nothing pending the reader's
+    product may form the norm itself."""
+    if pending is None and hasattr(norm, "into"):
+        return norm.into(reader, x)
+    return norm.forward(x, pending)
+
+
 @register_part("block", "prenorm")
 class PreNormBlock(Part):
     """The feed-forward (with its norm) may be absent."""
@@ -53,11 +61,11 @@ class PreNormBlock(Part):
         else:
             if left is not None:
                 left.finish()
-            h = self.mixer_norm.forward(x, pending)
+            h = norm_into(self.mixer_norm, mixer, x, pending)
         a = mixer.forward(h, step, memory, residual=x) if getattr(mixer, "accumulates", False) else mixer.forward(h, step, memory)
         if ffn is None:
             return x, a
-        h2 = self.feed_forward_norm.forward(x, a)
+        h2 = norm_into(self.feed_forward_norm, ffn, x, a)
         if getattr(ffn, "defers_sum", False) and not getattr(ffn, "identity", 0) and not getattr(ffn, "sum_is_plain", False):
             step.handover[DEFERRED] = DeferredBranch(x, expert_rows=ffn.forward(h2, step, deferred=True))
             return x, None

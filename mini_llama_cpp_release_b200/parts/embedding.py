@@ -12,7 +12,7 @@ from ..config.registry import build_part, register_part
 from ..config.specs import PartSpec
 from .base import Part, TensorSpec
 from .linear import Linear
-from .norm import RMSNorm
+from .norm import RMSNorm, normed_rows
 
 
 @register_part("embedding", "token_embedding")
@@ -79,8 +79,13 @@ class LinearHead(Part):
     def weight_bytes(self) -> int:
         return self.proj.nbytes()
 
-    def forward(self, h: torch.Tensor) -> torch.Tensor:
-        logits = self.proj(h, torch.float32)
+    def takes_normed_stream(self, n: int) -> bool:
+        """Whether `forward` may be given a `NormedStream` of n rows.  (A class with a forward of its own is given finished rows.)"""
+        return type(self).forward is LinearHead.forward and self.proj.few_plan(n) is not None
+
+    def forward(self, h) -> torch.Tensor:
+        h, gain, eps = normed_rows(h)
+        logits = self.proj(h, torch.float32) if gain is None else self.proj.of_norm(h, gain, eps)
         if self.softcap is not None:
             kernels.softcap(logits, self.softcap)
         return logits

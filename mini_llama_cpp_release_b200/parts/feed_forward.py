@@ -13,6 +13,7 @@ from ..config.registry import build_part, register_part
 from ..config.specs import PartSpec
 from .base import Part, TensorSpec
 from .linear import Linear
+from .norm import normed_rows
 
 
 
@@ -60,10 +61,20 @@ class SwiGLU(Part):
 
     accumulates = True        # forward(..., residual=x) may add the branch into the float32 stream and return None
 
-    def forward(self, h: torch.Tensor, step=None, residual=None):
+    def _few_plan(self, n: int):
+        return kernels.gemm_few_plan(n, 2 * self.inter, self.hidden, kernels.bindings.EPI_SILU_MUL, self.runtime.n_sms) if self.fused else None
+
+    def takes_normed_stream(self, n: int) -> bool:
+        """Whether `forward` may be given a `NormedStream` of n rows.  (A class with a forward of its own is given finished rows.)"""
+        return type(self).forward is SwiGLU.forward and self._few_plan(n) is not None
+
+    def forward(self, h, step=None, residual=None):
         rt = self.runtime
+        h, gain, eps = normed_rows(h)
         a = rt.empty(h.shape[0], self.inter)
-        if self.fused and kernels.gemm_rows_takes(h.shape[0], 2 * self.inter, self.hidden):
+        if (plan := self._few_plan(h.shape[0])) is not None:
+            kernels.gemm_few(h, self.gate_up.weight, a, kernels.bindings.EPI_SILU_MUL, plan, gain, eps, glu=self.activation)
+        elif self.fused and kernels.gemm_rows_takes(h.shape[0], 2 * self.inter, self.hidden):
             kernels.gemm_prompt(h, self.gate_up.weight, a, kernels.bindings.EPI_SILU_MUL, n_sms=rt.n_sms, glu=self.activation)    # prompts
         elif self.fused:
             kernels.gemm_tcgen05(h, self.gate_up.weight, a, kernels.bindings.EPI_SILU_MUL, n_sms=rt.n_sms, glu=self.activation)

@@ -68,6 +68,18 @@ class Linear:
     def nbytes(self) -> int:
         return self.weight.numel() * self.weight.element_size()
 
+    def few_plan(self, n_rows: int, epilogue: int = 0):
+        """The plan of the few-row product (csrc/gemm_few.cu), or None where another kernel takes these rows."""
+        if not self.tensor_core_ok:
+            return None
+        return kernels.gemm_few_plan(n_rows, self.out_features, self.in_features, epilogue, self.runtime.n_sms)
+
+    def of_norm(self, stream: torch.Tensor, gain: torch.Tensor, eps: float) -> torch.Tensor:
+        """float32 [n, out]: the product of the float32 stream's RMS norm, for a row count that has a `few_plan`."""
+        out = self.runtime.empty(stream.shape[0], self.out_features, dtype=torch.float32)
+        kernels.gemm_few(stream, self.weight, out, kernels.bindings.EPI_STORE, self.few_plan(stream.shape[0]), gain, eps)
+        return out
+
     def can_add_into_stream(self, n_rows: int) -> bool:
         """Whether `add_into` has a kernel for these operands: the tcgen05 products (atomic adds for few rows; plain or
         atomic adds for more), else the library's product with the stream as the matrix it adds to."""
@@ -86,6 +98,9 @@ class Linear:
         if m > SMALL_BATCH:
             kernels.library_gemm(x, self.weight, stream, accumulate=True)
             return
+        if (plan := self.few_plan(m, kernels.bindings.EPI_ADD)) is not None:
+            kernels.gemm_few(x, self.weight, stream, kernels.bindings.EPI_ADD, plan)
+            return
         splits = split_count(self.out_features, self.in_features, m, self.runtime.n_sms, max_splits=add_split_cap(m))
         kernels.gemm_tcgen05(x, self.weight, stream, kernels.bindings.EPI_ADD, splits, n_sms=self.runtime.n_sms)
 
@@ -100,6 +115,10 @@ class Linear:
             kernels.linear_simt(x, self.weight, out)
             return out
         kernels.require_cuda(x)
+        if (plan := self.few_plan(m)) is not None:
+            out = rt.empty(m, self.out_features, dtype=out_dtype)
+            kernels.gemm_few(x, self.weight, out, kernels.bindings.EPI_STORE, plan)
+            return out
         if self.tensor_core_ok and m <= SMALL_BATCH:
             splits = split_count(self.out_features, self.in_features, m, rt.n_sms) if (partial_ok and out_dtype == torch.float32) else 1
             out = rt.empty(splits, m, self.out_features, dtype=out_dtype)

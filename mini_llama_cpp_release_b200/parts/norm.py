@@ -7,6 +7,7 @@ addition rides in the next norm's kernel, in float32, and the stream itself stay
 """
 from __future__ import annotations
 
+from dataclasses import dataclass
 from typing import Optional
 
 import torch
@@ -14,6 +15,19 @@ import torch
 from .. import kernels
 from ..config.registry import register_part
 from .base import Part, TensorSpec
+
+
+@dataclass(frozen=True)
+class NormedStream:
+    """The RMS norm of the float32 stream x, not yet computed: the product that reads it computes it along the way."""
+    x: torch.Tensor
+    gain: torch.Tensor
+    eps: float
+
+
+def normed_rows(h):
+    """(rows, gain, eps) of a product's input: the rows themselves, or a stream whose norm is wanted (gain not None)."""
+    return (h.x, h.gain, h.eps) if isinstance(h, NormedStream) else (h, None, 0.0)
 
 
 @register_part("norm", "rmsnorm")
@@ -47,6 +61,14 @@ class RMSNorm(Part):
         out = self.runtime.empty(*x.shape, dtype=out_dtype or self.runtime.dtype)
         kernels.add_rmsnorm(x, delta, self.gain, self.eps, out)
         return out
+
+    def into(self, reader, x: torch.Tensor):
+        """The norm of x for `reader`, the part that multiplies it: left to the reader's product where it says that it
+        can form the norm itself (`takes_normed_stream`)."""
+        takes = getattr(reader, "takes_normed_stream", None)
+        if takes is not None and self.runtime.dtype == torch.bfloat16 and takes(x.shape[0]):
+            return NormedStream(x, self.gain, self.eps)
+        return self.forward(x)
 
     def forward_pair(self, x: torch.Tensor, other: Optional["RMSNorm"], delta: Optional[torch.Tensor] = None, expert_rows=None):
         """This norm and another of the same size and eps on the same x, which takes `delta` and the weighted sum of
