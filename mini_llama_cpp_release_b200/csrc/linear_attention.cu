@@ -206,6 +206,96 @@ gla_walk_kernel(GlaArgs a) {
 }
 
 
+// Steps of one token per sequence: a warp per (sequence, head, eight columns), a column's rows spread over its lanes, so that
+// the state streams through in whole lines and nothing but a warp's sum stands between its arrival and the output.  The
+// state was written by the step before, so its loads do not wait for the kernel before this one.  Bound by the state's bytes:
+// B200, 8 sequences, 6 heads of 128 x 257 (12.6 MB in and out), 5.5 us, the walk 32 us.
+constexpr int GLS_COLS = 8;
+
+template <int RPL, bool SILU>          // rows of a column per lane: dim <= 32 * RPL
+__global__ void __launch_bounds__(128)
+gla_step_kernel(GlaArgs a) {
+    grid_launch_dependents();
+    const int lane = threadIdx.x & 31;
+    const int col0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * GLS_COLS, head = blockIdx.y, seq = blockIdx.z;
+    const int dim = a.dim, vdim = a.vdim;
+    if (col0 >= vdim) return;
+    float* const S_base = a.state + (long long)a.slots[seq] * a.state_stride + (long long)head * vdim * dim;
+    float S[GLS_COLS][RPL];
+#pragma unroll
+    for (int c = 0; c < GLS_COLS; ++c)
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+            const int row = lane + 32 * i;
+            S[c][i] = (col0 + c < vdim && row < dim) ? S_base[(long long)(col0 + c) * dim + row] : 0.0f;
+        }
+    grid_dependency_wait();
+    for (int t = a.cu_seqlens[seq], t1 = a.cu_seqlens[seq + 1]; t < t1; ++t) {
+        const float* qk = a.qk + (long long)t * a.qk_stride + (head / a.qk_share) * dim;
+        const float one = a.const_decay != nullptr ? a.const_decay[head] : a.head_decay != nullptr ? a.head_decay[(long long)t * a.H + head] : 1.0f;
+        const bool per_row = a.const_decay == nullptr && a.head_decay == nullptr;
+        float q[RPL], k[RPL], d[RPL], v = 0.0f;
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+            const int row = lane + 32 * i;
+            q[i] = k[i] = 0.0f;
+            d[i] = one;
+            if (row < dim) {
+                q[i] = qk[a.q_col + row];
+                k[i] = qk[a.k_col + row];
+                if (per_row) d[i] = a.decay[(long long)t * a.H * dim + head * dim + row];
+            }
+        }
+        if (lane < GLS_COLS) {
+            if (col0 + lane < a.v_cols) v = a.vsrc[(long long)t * a.v_stride + a.v_col + head * a.v_cols + col0 + lane];
+            else if (col0 + lane < vdim) v = 1.0f;
+            if (a.v_scale != nullptr) v *= a.v_scale[(long long)t * a.H + head];
+            if (SILU) v = silu_f(v);
+        }
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+            if (SILU) {
+                q[i] = silu_f(q[i]);
+                k[i] = silu_f(k[i]);
+            }
+            q[i] *= a.q_scale;
+        }
+        float acc[GLS_COLS];
+#pragma unroll
+        for (int c = 0; c < GLS_COLS; ++c) {
+            const float vc = __shfl_sync(0xffffffffu, v, c);
+            acc[c] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) {
+                S[c][i] = fmaf(d[i], S[c][i], k[i] * vc);
+                acc[c] = fmaf(S[c][i], q[i], acc[c]);
+            }
+        }
+        float mine = 0.0f;
+#pragma unroll
+        for (int c = 0; c < GLS_COLS; ++c) {
+            const float sum = warp_sum(acc[c]);
+            if (lane == c) mine = sum;
+        }
+        if (lane < GLS_COLS && col0 + lane < vdim) a.out[(long long)t * a.H * vdim + head * vdim + col0 + lane] = mine;
+    }
+#pragma unroll
+    for (int c = 0; c < GLS_COLS; ++c)
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+            const int row = lane + 32 * i;
+            if (col0 + c < vdim && row < dim) S_base[(long long)(col0 + c) * dim + row] = S[c][i];
+        }
+}
+
+template <bool SILU>
+static int launch_gla_step(const GlaArgs& a, int n_seqs, cudaStream_t s) {
+    const dim3 grid((a.vdim + 4 * GLS_COLS - 1) / (4 * GLS_COLS), a.H, n_seqs);
+    auto k = a.dim <= 32 ? gla_step_kernel<1, SILU> : a.dim <= 64 ? gla_step_kernel<2, SILU> : a.dim <= 128 ? gla_step_kernel<4, SILU> : gla_step_kernel<8, SILU>;
+    cudaError_t e = launch_pdl(k, grid, dim3(128), 0, s, a);
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
 // The state-space layer ("Mamba-2"; Dao and Gu, "Transformers are SSMs: Generalized Models and Efficient Algorithms Through
 // Structured State Space Duality"): per head a state S [N][vdim] with one decay per token and head,
 //   dt = softplus(z_dt + bias),   S_t = exp(-exp(A_log) · dt) S_{t-1} + dt · B_t x_tᵀ,   y_t = S_tᵀ C_t + D x_t
@@ -272,12 +362,20 @@ static int launch_gla(const GlaArgs& a, dim3 grid, cudaStream_t s) {
     return 0;
 }
 
-int gla_walk(GlaArgs a, int n_seqs, int n_tokens, int rows, bool silu, cudaStream_t s) {
+int gla_walk(GlaArgs a, int n_seqs, int n_tokens, int rows, bool silu, cudaStream_t s, float* chunks, int max_q_len) {
     if (a.H <= 0 || a.dim <= 0 || a.dim > 256 || a.vdim <= 0 || a.v_cols <= 0 || a.v_cols > a.vdim || n_seqs > 65535 ||
         a.qk_share < 1 || a.H % a.qk_share)
         return MLC_ERR_BAD_SIZE;
     if (silu && (a.v_scale != nullptr || a.v_cols != a.vdim)) return MLC_ERR_UNSUPPORTED;      // SiLU would act on the scaled v
     if (rows != 2 && rows != 4 && rows != 8 && rows != 16 && rows != 32) return MLC_ERR_BAD_SIZE;
+    if (chunks != nullptr) {
+        if (silu || 8 * rows < a.dim || (a.const_decay == nullptr && a.head_decay == nullptr) || ((uintptr_t)chunks & 15) ||
+            gla_chunk_floats(n_seqs, n_tokens, max_q_len, a.H, a.dim, a.vdim) == 0)
+            return MLC_ERR_UNSUPPORTED;
+        return gla_chunks(a, n_seqs, n_tokens, max_q_len, chunks, s);
+    }
+    // as many tokens as sequences: as a rule one each
+    if (n_tokens == n_seqs && 8 * rows >= a.dim && a.H <= 65535) return silu ? launch_gla_step<true>(a, n_seqs, s) : launch_gla_step<false>(a, n_seqs, s);
     a.col_slabs = (a.vdim + GLA_COLS - 1) / GLA_COLS;
     a.out_slice = (long long)n_tokens * a.H * a.vdim;
     const dim3 grid(a.H, n_seqs, a.col_slabs * ((a.dim + 8 * rows - 1) / (8 * rows)));
@@ -305,18 +403,25 @@ extern "C" int mlc_gla_rows(int n_seqs, int H, int dim, int vdim, int n_sms) {
     return rows;
 }
 
+// Floats of 16-byte aligned scratch memory with which a step of these sizes takes the prompt's form of the walk over one decay
+// per token and head (gla_chunks.cu), 0: the walk.  max_q_len: the longest run of a sequence.
+extern "C" long long mlc_gla_chunk_floats(int n_seqs, int n_tokens, int max_q_len, int H, int dim, int vdim) {
+    return gla_chunk_floats(n_seqs, n_tokens, max_q_len, H, dim, vdim);
+}
+
 // The walk over one decay per token, head and key channel, or over the state-space layer's (one per token and head).
 static int walk_over(const float* qk, long long qk_stride, int q_col, int k_col, const float* v, long long v_stride, int v_col,
                      const float* decay, float q_scale, float* state, long long state_stride, const int* slots,
                      const int* cu_seqlens, int n_seqs, int n_tokens, int H, int dim, int vdim, int rows, float* out,
-                     cudaStream_t s, int qk_share = 1, const float* head_decay = nullptr, const float* v_scale = nullptr) {
+                     cudaStream_t s, int qk_share = 1, const float* head_decay = nullptr, const float* v_scale = nullptr,
+                     float* chunks = nullptr, int max_q_len = 0) {
     GlaArgs a = {};
     a.qk = qk; a.qk_stride = qk_stride; a.q_col = q_col; a.k_col = k_col;
     a.vsrc = v; a.v_stride = v_stride; a.v_col = v_col;
     a.decay = decay; a.head_decay = head_decay; a.v_scale = v_scale; a.q_scale = q_scale;
     a.state = state; a.state_stride = state_stride; a.slots = slots; a.cu_seqlens = cu_seqlens; a.out = out;
     a.H = H; a.dim = dim; a.vdim = a.v_cols = vdim; a.qk_share = qk_share;
-    return gla_walk(a, n_seqs, n_tokens, rows, false, s);
+    return gla_walk(a, n_seqs, n_tokens, rows, false, s, chunks, max_q_len);
 }
 
 // proj: float32 rows (stride proj_stride) holding q (H x dim) at q_col, k (H x dim) at k_col, v (H x vdim) at v_col.
@@ -361,12 +466,13 @@ extern "C" int mlc_forget_gate_attention(const float* proj, long long proj_strid
 // float32 rows (what the convolution and its activation left) holding x (H x vdim) at column 0, B (G x N) at b_col and C
 // (G x N) at c_col; head h reads group h / (H / G).  dt, decay: float32 [n][H] scratch that this call fills.  state: float32, a
 // slot's row holds H*vdim*N floats ([head][column][row]).  rows: what mlc_gla_rows gave for (n_seqs, H, N, vdim).  walk: float32
-// [ceil(N / (8 * rows))][n][H*vdim] scratch (the walk's partial outputs).  out [n][H*vdim] of out_dtype: the gated, normed y.
+// [ceil(N / (8 * rows))][n][H*vdim] scratch (the walk's partial outputs).  chunks: null, or
+// the memory mlc_gla_chunk_floats asked for, with rows that cover N.  out [n][H*vdim] of out_dtype: the gated, normed y.
 extern "C" int mlc_state_space(const float* proj, long long proj_stride, int z_col, int dt_col, const float* xbc, long long xbc_stride,
                                int b_col, int c_col, const float* dt_bias, const float* A_log, const float* D, const float* gain,
                                float eps, int norm_groups, float* dt, float* decay, float* state, long long state_stride,
-                               const int* slots, const int* cu_seqlens, int n_seqs, int n_tokens, int H, int G, int N, int vdim,
-                               int rows, float* walk, void* out, int out_dtype, void* stream) {
+                               const int* slots, const int* cu_seqlens, int n_seqs, int n_tokens, int max_q_len, int H, int G, int N,
+                               int vdim, int rows, float* walk, float* chunks, void* out, int out_dtype, void* stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || N <= 0 || N > 256 || vdim <= 0 || n_seqs > 65535) return MLC_ERR_BAD_SIZE;
     const int inner = H * vdim;
@@ -376,7 +482,7 @@ extern "C" int mlc_state_space(const float* proj, long long proj_stride, int z_c
     state_space_steps_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(proj, proj_stride, dt_col, dt_bias, A_log, total, H, dt, decay);
     MLC_LAUNCH_CHECK();
     const int rc = walk_over(xbc, xbc_stride, c_col, b_col, xbc, xbc_stride, 0, nullptr, 1.0f, state, state_stride, slots, cu_seqlens,
-                            n_seqs, n_tokens, H, N, vdim, rows, walk, s, H / G, decay, dt);
+                            n_seqs, n_tokens, H, N, vdim, rows, walk, s, H / G, decay, dt, chunks, max_q_len);
     if (rc != 0) return rc;
     const int slices = (N + 8 * rows - 1) / (8 * rows);
     const int warps = inner >= 1024 ? 8 : 4;

@@ -35,7 +35,13 @@ struct GlaArgs {
 };
 
 // Launches the walk for n_seqs sequences of n_tokens tokens together; `rows` is what mlc_gla_rows gave; `silu`: q, k and v
-// pass SiLU as they are read.  Returns 0 or an error code.
-int gla_walk(GlaArgs a, int n_seqs, int n_tokens, int rows, bool silu, cudaStream_t s);
+// pass SiLU as they are read.  With `chunks`, scratch memory of the size mlc_gla_chunk_floats gave (which is not 0), rows
+// that cover the head, one decay per token and head, and no `silu`, the prompt's form instead (gla_chunks.cu).  Returns 0 or
+// an error code.
+int gla_walk(GlaArgs a, int n_seqs, int n_tokens, int rows, bool silu, cudaStream_t s, float* chunks = nullptr, int max_q_len = 0);
+
+// The prompt's form: floats of scratch memory it wants for a step of these sizes (0: the walk is to be taken), and its launch.
+long long gla_chunk_floats(int n_seqs, int n_tokens, int max_q_len, int H, int dim, int vdim);
+int gla_chunks(GlaArgs a, int n_seqs, int n_tokens, int max_q_len, float* scratch, cudaStream_t s);
 
 }  // namespace mlc

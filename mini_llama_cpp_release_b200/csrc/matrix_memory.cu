@@ -302,11 +302,13 @@ using namespace mlc;
 // (H x vdim) side by side from column q_col on, and of the gate (H x vdim) at g_col; `silu_first` overwrites q, k and v with
 // their SiLU (one more launch) instead of leaving it to the walk.  decay float32 [H], gain float32 [H*vdim].  state: float32, a slot's row holds
 // H*vdim*dim floats ([head][column][row]).  rows: what mlc_gla_rows gave.  walk: float32 [ceil(dim / (8 * rows))][n][H*vdim]
-// scratch.  out [n][H*vdim] of out_dtype.
+// scratch.  chunks: null, or the memory mlc_gla_chunk_floats asked for (then with silu_first, and rows that cover dim).
+// max_q_len: the longest run of a sequence.  out [n][H*vdim] of out_dtype.
 extern "C" int mlc_decay_attention(float* proj, long long proj_stride, int q_col, int g_col, int silu_first,
                                    const float* decay, const float* gain, float eps, float out_scale, float* state,
                                    long long state_stride, const int* slots, const int* cu_seqlens, int n_seqs, int n_tokens,
-                                   int H, int dim, int vdim, int rows, float* walk, void* out, int out_dtype, void* stream) {
+                                   int max_q_len, int H, int dim, int vdim, int rows, float* walk, float* chunks, void* out,
+                                   int out_dtype, void* stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (H <= 0 || vdim <= 0 || (long long)H * vdim > 16384 || rows < 1) return MLC_ERR_BAD_SIZE;
     if (out_dtype != MLC_DTYPE_F32 && out_dtype != MLC_DTYPE_BF16) return MLC_ERR_BAD_DTYPE;
@@ -325,7 +327,7 @@ extern "C" int mlc_decay_attention(float* proj, long long proj_stride, int q_col
     a.const_decay = decay; a.q_scale = 1.0f;
     a.state = state; a.state_stride = state_stride; a.slots = slots; a.cu_seqlens = cu_seqlens; a.out = walk;
     a.H = H; a.dim = dim; a.vdim = a.v_cols = vdim; a.qk_share = 1;
-    const int rc = gla_walk(a, n_seqs, n_tokens, rows, !silu_first, s);
+    const int rc = gla_walk(a, n_seqs, n_tokens, rows, !silu_first, s, chunks, max_q_len);
     if (rc != 0) return rc;
     const int slices = (dim + 8 * rows - 1) / (8 * rows), inner = H * vdim;
     const long long slice = (long long)n_tokens * inner;
@@ -338,12 +340,14 @@ extern "C" int mlc_decay_attention(float* proj, long long proj_stride, int q_col
 // each), the input and forget gates' logits (H each) at their columns.  i_bias, f_bias float32 [H], gain float32 [H*vdim].
 // state: float32, a slot's row holds H*(vdim+1)*dim floats ([head][column][row], the last column n), then H running maxima.
 // gates: float32 [3][n][H] scratch.  rows: what mlc_gla_rows gave for (n_seqs, H, dim, vdim + 1).  walk: float32
-// [ceil(dim / (8 * rows))][n][H*(vdim+1)] scratch.  out [n][H*vdim] of out_dtype.  max_q_len: the longest run of a sequence.
+// [ceil(dim / (8 * rows))][n][H*(vdim+1)] scratch.  chunks: null, or the memory
+// mlc_gla_chunk_floats asked for (for vdim + 1 columns; then with rows that cover dim).  out [n][H*vdim] of out_dtype.
+// max_q_len: the longest run of a sequence.
 extern "C" int mlc_matrix_memory(const float* proj, long long proj_stride, int q_col, int k_col, int v_col, int g_col, int i_col,
                                  int f_col, const float* i_bias, const float* f_bias, float cap, const float* gain, float eps,
                                  float* state, long long state_stride, const int* slots, const int* cu_seqlens, int n_seqs,
                                  int n_tokens, int max_q_len, int H, int dim, int vdim, int rows, float* gates, float* walk,
-                                 void* out, int out_dtype, void* stream) {
+                                 float* chunks, void* out, int out_dtype, void* stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (H <= 0 || dim <= 0 || vdim <= 0 || vdim > 1024 || n_seqs > 65535 || rows < 1 || !(cap > 0.0f)) return MLC_ERR_BAD_SIZE;
     if (out_dtype != MLC_DTYPE_F32 && out_dtype != MLC_DTYPE_BF16) return MLC_ERR_BAD_DTYPE;
@@ -361,7 +365,7 @@ extern "C" int mlc_matrix_memory(const float* proj, long long proj_stride, int q
     a.head_decay = decay; a.v_scale = take; a.q_scale = 1.0f / sqrtf((float)dim);
     a.state = state; a.state_stride = state_stride; a.slots = slots; a.cu_seqlens = cu_seqlens; a.out = walk;
     a.H = H; a.dim = dim; a.vdim = vdim + 1; a.v_cols = vdim; a.qk_share = 1;
-    const int rc = gla_walk(a, n_seqs, n_tokens, rows, false, s);
+    const int rc = gla_walk(a, n_seqs, n_tokens, rows, false, s, chunks, max_q_len);
     if (rc != 0) return rc;
     const int slices = (dim + 8 * rows - 1) / (8 * rows);
     const long long slice = per * (vdim + 1);

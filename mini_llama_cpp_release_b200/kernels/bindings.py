@@ -112,8 +112,8 @@ def core() -> ctypes.CDLL:
             "mlc_moe_route": [P, I, P, P, I, I, I, I, I, P, P, P],
             "mlc_moe_plan": [P, I, I, I, I, I, P, P, P, P],
             "mlc_moe_plan_table": [P, P, F, P, I, I, I, I, I, P, P, P, P],
-            "mlc_decay_attention": [P, LL, I, I, I, P, P, F, F, P, LL, P, P, I, I, I, I, I, I, P, P, I, P],
-            "mlc_matrix_memory": [P, LL, I, I, I, I, I, I, P, P, F, P, F, P, LL, P, P, I, I, I, I, I, I, I, P, P, P, I, P],
+            "mlc_decay_attention": [P, LL, I, I, I, P, P, F, F, P, LL, P, P, I, I, I, I, I, I, I, P, P, P, I, P],
+            "mlc_matrix_memory": [P, LL, I, I, I, I, I, I, P, P, F, P, F, P, LL, P, P, I, I, I, I, I, I, I, P, P, P, P, I, P],
             "mlc_rms_pair": [P, P, I, P, P, P, I, P, P, F, I, I, P, P, I, P],
             "mlc_embed_rms": [P, I, P, I, I, F, P, F, P, P],
             "mlc_diff_combine": [P, I, P, LL, F, F, F, I, I, I, I, P, P],
@@ -126,7 +126,7 @@ def core() -> ctypes.CDLL:
             "mlc_tanh_norm": [P, P, I, P, P, I, P, P, F, F, P, P, F, I, I, P, I, P],
             "mlc_glu": [P, I, I, I, I, I, F, F, P, I, P],
             "mlc_sigmoid_gate": [P, I, P, LL, I, I, I, I, P],
-            "mlc_state_space": [P, LL, I, I, P, LL, I, I, P, P, P, P, F, I, P, P, P, LL, P, P, I, I, I, I, I, I, I, P, P, I, P],
+            "mlc_state_space": [P, LL, I, I, P, LL, I, I, P, P, P, P, F, I, P, P, P, LL, P, P, I, I, I, I, I, I, I, I, P, P, P, I, P],
             "mlc_forget_gate_attention": [P, LL, I, I, I, P, P, P, P, P, LL, P, P, I, I, I, I, I, I, P, P],
             "mlc_scaled_add": [P, P, I, P, P, I, P, LL, I, P],
             "mlc_scaled_add_experts": [P, P, I, P, P, P, P, I, P, LL, I, P],
@@ -154,6 +154,8 @@ def core() -> ctypes.CDLL:
         lib.mlc_linear_simt_scratch_floats.restype = c_longlong
         lib.mlc_gla_rows.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.mlc_gla_rows.restype = c_int
+        lib.mlc_gla_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
+        lib.mlc_gla_chunk_floats.restype = c_longlong
         lib.mlc_set_pdl.argtypes = [c_int]
         lib.mlc_set_pdl.restype = c_int
         lib.mlc_uniform_of.argtypes = [c_ulonglong, c_int, c_int]
@@ -797,6 +799,22 @@ def gla_slices(n_seqs: int, heads: int, dim: int, vdim: int, device: torch.devic
     return (dim + 8 * rows - 1) // (8 * rows)
 
 
+def _head_decay_plan(step, n: int, heads: int, dim: int, vdim: int, device: torch.device) -> Tuple[int, int, Optional[torch.Tensor]]:
+    """For a walk over one decay per token and head: rows of the state per thread, slices of partial outputs, and scratch
+    memory if the step takes the prompt's form (csrc/gla_chunks.cu).  That form and the step of single tokens want the whole
+    head in one slice."""
+    lib = core()
+    need = lib.mlc_gla_chunk_floats(step.n_seqs, n, step.max_q_len, heads, dim, vdim)
+    if need > 0 or n == step.n_seqs:
+        rows = 4
+        while 8 * rows < dim:
+            rows *= 2
+    else:
+        rows = lib.mlc_gla_rows(step.n_seqs, heads, dim, vdim, _sm_count(device))
+    chunks = torch.empty(need, dtype=torch.float32, device=device) if need > 0 else None
+    return rows, (dim + 8 * rows - 1) // (8 * rows), chunks
+
+
 def gla(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, z: torch.Tensor, z_bias: Optional[torch.Tensor], tau: float,
         state: torch.Tensor, step, heads: int, dim: int, vdim: int, out: torch.Tensor) -> None:
     """S <- diag(sigmoid(z + bias)^(1/tau)) S + k vT, o = ST q dim^-1/2 over the step's tokens; q, k (heads x dim) and v
@@ -857,8 +875,7 @@ def state_space(proj: torch.Tensor, z_col: int, dt_col: int, xbc: torch.Tensor, 
     _require_rows(xbc)
     n = proj.shape[0]
     lib = core()
-    rows = lib.mlc_gla_rows(step.n_seqs, heads, n_state, vdim, _sm_count(out.device))
-    slices = (n_state + 8 * rows - 1) // (8 * rows)
+    rows, slices, chunks = _head_decay_plan(step, n, heads, n_state, vdim, out.device)
     inner = heads * vdim
     assert state.shape[1] == inner * n_state and tuple(out.shape) == (n, inner) and gain.numel() == inner
     for t in (dt_bias, A_log, D):
@@ -868,9 +885,9 @@ def state_space(proj: torch.Tensor, z_col: int, dt_col: int, xbc: torch.Tensor, 
     _check(lib.mlc_state_space(proj.data_ptr(), proj.stride(0), z_col, dt_col, xbc.data_ptr(), xbc.stride(0), b_col, c_col,
                                dt_bias.data_ptr(), A_log.data_ptr(), D.data_ptr(), gain.data_ptr(), float(eps), int(norm_groups),
                                dt.data_ptr(), decay.data_ptr(), state.data_ptr(), state.stride(0), step.slots.data_ptr(),
-                               step.cu_seqlens.data_ptr(), step.n_seqs, n, heads, groups, n_state, vdim, rows, walk.data_ptr(),
-                               out.data_ptr(), dtype_code(out.dtype), _stream()), "state-space layer")
-    count_launches(2)
+                               step.cu_seqlens.data_ptr(), step.n_seqs, n, step.max_q_len, heads, groups, n_state, vdim, rows,
+                               walk.data_ptr(), _ptr(chunks), out.data_ptr(), dtype_code(out.dtype), _stream()), "state-space layer")
+    count_launches(2 + (2 if chunks is not None else 0))
 
 
 # ------------------------------------------------------------------ memories that decay per head (csrc/matrix_memory.cu)
@@ -885,17 +902,16 @@ def decay_attention(proj: torch.Tensor, q_col: int, g_col: int, decay: torch.Ten
     _require_rows(proj)
     n = proj.shape[0]
     lib = core()
-    rows = lib.mlc_gla_rows(step.n_seqs, heads, dim, vdim, _sm_count(out.device))
-    slices = (dim + 8 * rows - 1) // (8 * rows)
+    rows, slices, chunks = _head_decay_plan(step, n, heads, dim, vdim, out.device)
     assert decay.dtype == gain.dtype == torch.float32 and decay.numel() == heads and gain.numel() == heads * vdim
     assert state.shape[1] == heads * vdim * dim and tuple(out.shape) == (n, heads * vdim)
     walk = torch.empty(slices * n * heads * vdim, dtype=torch.float32, device=out.device)
-    silu_first = n > 64                 # a prompt: SiLU once per value, not once per block of the walk that reads it
+    silu_first = n > 64 or chunks is not None      # a prompt: SiLU once per value, not once per block of the walk that reads it
     _check(lib.mlc_decay_attention(proj.data_ptr(), proj.stride(0), q_col, g_col, 1 if silu_first else 0, decay.data_ptr(), gain.data_ptr(),
                                    float(eps), float(out_scale), state.data_ptr(), state.stride(0), step.slots.data_ptr(),
-                                   step.cu_seqlens.data_ptr(), step.n_seqs, n, heads, dim, vdim, rows, walk.data_ptr(),
-                                   out.data_ptr(), dtype_code(out.dtype), _stream()), "linear attention with a constant decay")
-    count_launches(2 if silu_first else 1)
+                                   step.cu_seqlens.data_ptr(), step.n_seqs, n, step.max_q_len, heads, dim, vdim, rows,
+                                   walk.data_ptr(), _ptr(chunks), out.data_ptr(), dtype_code(out.dtype), _stream()), "linear attention with a constant decay")
+    count_launches((2 if silu_first else 1) + (2 if chunks is not None else 0))
 
 
 def matrix_memory(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, g_col: int, i_col: int, f_col: int, i_bias: torch.Tensor,
@@ -911,8 +927,7 @@ def matrix_memory(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, g_col:
     _require_rows(proj)
     n = proj.shape[0]
     lib = core()
-    rows = lib.mlc_gla_rows(step.n_seqs, heads, dim, vdim + 1, _sm_count(out.device))
-    slices = (dim + 8 * rows - 1) // (8 * rows)
+    rows, slices, chunks = _head_decay_plan(step, n, heads, dim, vdim + 1, out.device)
     assert all(t.dtype == torch.float32 for t in (i_bias, f_bias, gain)) and i_bias.numel() == f_bias.numel() == heads
     assert gain.numel() == heads * vdim and tuple(out.shape) == (n, heads * vdim)
     assert state.shape[1] == heads * (vdim + 1) * dim + heads
@@ -920,9 +935,9 @@ def matrix_memory(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, g_col:
     _check(lib.mlc_matrix_memory(proj.data_ptr(), proj.stride(0), q_col, k_col, v_col, g_col, i_col, f_col, i_bias.data_ptr(),
                                  f_bias.data_ptr(), float(cap), gain.data_ptr(), float(eps), state.data_ptr(), state.stride(0),
                                  step.slots.data_ptr(), step.cu_seqlens.data_ptr(), step.n_seqs, n, step.max_q_len, heads, dim,
-                                 vdim, rows, scratch.data_ptr(), scratch[3 * n * heads:].data_ptr(), out.data_ptr(),
+                                 vdim, rows, scratch.data_ptr(), scratch[3 * n * heads:].data_ptr(), _ptr(chunks), out.data_ptr(),
                                  dtype_code(out.dtype), _stream()), "matrix memory with exponential gates")
-    count_launches(2)
+    count_launches(2 + (2 if chunks is not None else 0))
 
 
 # ------------------------------------------------------------------ dynamic tanh norm, gated units, sigmoid gate (csrc/tanh_norm.cu)
