@@ -47,15 +47,25 @@ struct AttnArgs {
     int n_splits;
 };
 
+// Floats from one row of a tile to the next: whole 16-byte pieces, an odd number of them, so that the lanes of a warp, each
+// reading a piece of a key of its own, hit all banks.  What lies between a row's end and its last whole piece is zero.
+__host__ __device__ __forceinline__ int att_pitch(int hd) { return 4 * (((hd + 3) / 4) | 1); }
+
+// What bounds it: with the few rows of a decode step, the chain of a tile's loads, scores, softmax and weighted values; so
+// loads are 16 bytes, the next tile's are in flight while a tile is used, and a key's (a value's) entries pass a lane's
+// registers once for all four rows of its warp.  B200, float32, 3 sequences of about 100 keys, 14 heads of 64 on 2: 82 us a
+// launch with entry-by-entry loads and a row at a time, now 22.
 template <typename T, int ATT_ACC>        // ATT_ACC: output entries a lane holds per row, head size <= 32 * ATT_ACC
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attention_simt_kernel(AttnArgs a, PagedKV c) {
     extern __shared__ float smem[];
     const int hd = c.head_dim;
-    float* Qs = smem;                              // [16][hd]
-    float* Ks = Qs + ATT_ROWS * hd;                // [32][hd+1]
-    float* Vs = Ks + ATT_TILE * (hd + 1);          // [32][hd]
+    const int ld = att_pitch(hd);                  // a row's floats in shared memory
+    float* Qs = smem;                              // [16][ld]
+    float* Ks = Qs + ATT_ROWS * ld;                // [32][ld]
+    float* Vs = Ks + ATT_TILE * ld;                // [32][ld]
     __shared__ long long key_off[ATT_TILE];
+    __shared__ __align__(16) float Ps[ATT_WARPS][ATT_TILE][ATT_ROWS_PER_WARP];   // a warp's probabilities of a tile
 
     const int b = blockIdx.z;
     int y = blockIdx.y;
@@ -73,11 +83,11 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
     const T* q = (const T*)a.q;
 
     // stage the block's query rows
-    for (int idx = threadIdx.x; idx < ATT_ROWS * hd; idx += blockDim.x) {
-        const int r = idx / hd, d = idx % hd;
+    for (int idx = threadIdx.x; idx < ATT_ROWS * ld; idx += blockDim.x) {
+        const int r = idx / ld, d = idx % ld;
         const int t = r / a.heads_per_block, hg = chunk * a.heads_per_block + r % a.heads_per_block;
         float v = 0.0f;
-        if (t < n_tok && hg < a.group) {
+        if (t < n_tok && hg < a.group && d < hd) {
             const long long row = (long long)(seq_tok0 + tok0 + t) * a.q_heads + (kvh * a.group + hg);
             v = to_float(q[row * hd + d]);
         }
@@ -115,57 +125,140 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
 
     const T* kp = (const T*)c.k_pool;
     const T* vp = (const T*)c.v_pool;
-    for (int v = my_begin; v < my_end; ++v) {
-        const int tile = v < head_tiles ? v : tile_begin + (v - head_tiles);
-        __syncthreads();   // previous tile's readers are done (and Qs is staged)
-        if (threadIdx.x < ATT_TILE) {
-            const int kpos = tile * ATT_TILE + threadIdx.x;
-            key_off[threadIdx.x] = ((kpos >= lo_block || kpos < keep) && kpos <= p_last) ? paged_offset(c, b, kpos, kvh) : -1;
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < ATT_TILE * hd; idx += blockDim.x) {
-            const int j = idx / hd, d = idx % hd;
-            const long long off = key_off[j];
-            float kv = 0.0f, vv = 0.0f;
+    auto tile_of = [&](int v) { return v < head_tiles ? v : tile_begin + (v - head_tiles); };
+    // a float32 cache whose rows are whole 16-byte pieces: a thread's pieces of the next tile wait in registers
+    const bool wide = sizeof(T) == 4 && ATT_ACC <= 8 && (hd & 3) == 0 && ((((uintptr_t)kp) | ((uintptr_t)vp)) & 15) == 0 && (c.entry_offset & 3) == 0;
+    constexpr int PIECES = ATT_ACC <= 8 ? 4 : 1;      // up to 64 entries per head: 32 keys x 16 pieces on 128 threads
+    const int row_pieces = hd >> 2;
+    const bool ahead = wide && hd <= 64;
+    float4 kr[PIECES], vr[PIECES];
+    auto offset_of = [&](int tile, int j) -> long long {
+        const int kpos = tile * ATT_TILE + j;
+        return ((kpos >= lo_block || kpos < keep) && kpos <= p_last) ? paged_offset(c, b, kpos, kvh) : -1;
+    };
+    auto fetch = [&](int v) {
+        const int tile = tile_of(v);
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) {
+            const int idx = threadIdx.x + u * ATT_WARPS * 32, j = idx / row_pieces, d = (idx - j * row_pieces) * 4;
+            kr[u] = vr[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const long long off = j < ATT_TILE ? offset_of(tile, j) : -1;
             if (off >= 0) {
-                kv = to_float(kp[off + d]);
-                vv = to_float(vp[off + d]);
+                kr[u] = *reinterpret_cast<const float4*>((const float*)kp + off + d);
+                vr[u] = *reinterpret_cast<const float4*>((const float*)vp + off + d);
             }
-            Ks[j * (hd + 1) + d] = kv;
-            Vs[j * hd + d] = vv;
+        }
+    };
+    if (ahead && my_begin < my_end) fetch(my_begin);
+    for (int v = my_begin; v < my_end; ++v) {
+        const int tile = tile_of(v);
+        __syncthreads();   // previous tile's readers are done (and Qs is staged)
+        if (ahead) {
+#pragma unroll
+            for (int u = 0; u < PIECES; ++u) {
+                const int idx = threadIdx.x + u * ATT_WARPS * 32, j = idx / row_pieces, d = (idx - j * row_pieces) * 4;
+                if (j < ATT_TILE) {
+                    *reinterpret_cast<float4*>(Ks + j * ld + d) = kr[u];
+                    *reinterpret_cast<float4*>(Vs + j * ld + d) = vr[u];
+                }
+            }
+            if (v + 1 < my_end) fetch(v + 1);
+        } else {
+            if (threadIdx.x < ATT_TILE) key_off[threadIdx.x] = offset_of(tile, threadIdx.x);
+            __syncthreads();
+            if (wide) {
+                for (int idx = threadIdx.x; idx < ATT_TILE * row_pieces; idx += blockDim.x) {
+                    const int j = idx / row_pieces, d = (idx - j * row_pieces) * 4;
+                    const long long off = key_off[j];
+                    float4 kv = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv = kv;
+                    if (off >= 0) {
+                        kv = *reinterpret_cast<const float4*>((const float*)kp + off + d);
+                        vv = *reinterpret_cast<const float4*>((const float*)vp + off + d);
+                    }
+                    *reinterpret_cast<float4*>(Ks + j * ld + d) = kv;
+                    *reinterpret_cast<float4*>(Vs + j * ld + d) = vv;
+                }
+            } else {
+                for (int idx = threadIdx.x; idx < ATT_TILE * ld; idx += blockDim.x) {
+                    const int j = idx / ld, d = idx % ld;
+                    const long long off = key_off[j];
+                    float kv = 0.0f, vv = 0.0f;
+                    if (off >= 0 && d < hd) {
+                        kv = to_float(kp[off + d]);
+                        vv = to_float(vp[off + d]);
+                    }
+                    Ks[idx] = kv;
+                    Vs[idx] = vv;
+                }
+            }
         }
         __syncthreads();
 
+        // scores of the warp's four rows against the lane's key, each summed in ascending order of the entries
         const int kpos = tile * ATT_TILE + lane;
+        float dot[ATT_ROWS_PER_WARP];
+#pragma unroll
+        for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) dot[i] = 0.0f;
+        const float* const qw = Qs + warp * ATT_ROWS_PER_WARP * ld;
+        const float* const kl = Ks + lane * ld;
+#pragma unroll 4
+        for (int d = 0; d < hd; d += 4) {
+            const float4 kk = *reinterpret_cast<const float4*>(kl + d);
+            float4 qq[ATT_ROWS_PER_WARP];
+#pragma unroll
+            for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) qq[i] = *reinterpret_cast<const float4*>(qw + i * ld + d);
+            // row after row, not term after term: the multiply-adds of one sum wait for one another
+#pragma unroll
+            for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) dot[i] = fmaf(qq[i].x, kk.x, dot[i]);
+#pragma unroll
+            for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) dot[i] = fmaf(qq[i].y, kk.y, dot[i]);
+#pragma unroll
+            for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) dot[i] = fmaf(qq[i].z, kk.z, dot[i]);
+#pragma unroll
+            for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) dot[i] = fmaf(qq[i].w, kk.w, dot[i]);
+        }
+        bool any = false;
+        float corr[ATT_ROWS_PER_WARP];
 #pragma unroll
         for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) {
-            if (!row_ok[i]) continue;
-            const bool in_range = (kpos >= row_lo[i] || kpos < keep) && kpos <= row_hi[i];
+            const bool in_range = row_ok[i] && (kpos >= row_lo[i] || kpos < keep) && kpos <= row_hi[i];
             float s = -INFINITY;
             if (in_range) {
-                const float* qr = Qs + (warp * ATT_ROWS_PER_WARP + i) * hd;
-                const float* kr = Ks + lane * (hd + 1);
-                float dot = 0.0f;
-                for (int d = 0; d < hd; ++d) dot += qr[d] * kr[d];
-                s = dot * a.scale;
+                s = dot[i] * a.scale;
                 if (a.softcap > 0.0f) s = a.softcap * tanhf(s / a.softcap);
             }
             const float tile_max = warp_max(s);
-            if (tile_max == -INFINITY) continue;
-            const float m_new = fmaxf(m[i], tile_max);
-            const float p = in_range ? expf(s - m_new) : 0.0f;
-            const float corr = (m[i] == -INFINITY) ? 0.0f : expf(m[i] - m_new);
-            l[i] = l[i] * corr + warp_sum(p);
-            m[i] = m_new;
+            float p = 0.0f;
+            corr[i] = 1.0f;
+            if (tile_max != -INFINITY) {              // the same for the whole warp
+                const float m_new = fmaxf(m[i], tile_max);
+                p = in_range ? expf(s - m_new) : 0.0f;
+                corr[i] = (m[i] == -INFINITY) ? 0.0f : expf(m[i] - m_new);
+                l[i] = l[i] * corr[i] + warp_sum(p);
+                m[i] = m_new;
+                any = true;
+            }
+            Ps[warp][lane][i] = p;
+        }
+        __syncwarp();
+        if (!any) continue;
 #pragma unroll
-            for (int k = 0; k < ATT_ACC; ++k) acc[i][k] *= corr;
-            for (int j = 0; j < ATT_TILE; ++j) {
-                const float pj = __shfl_sync(0xffffffffu, p, j);
-                const float* vr = Vs + j * hd;
+        for (int i = 0; i < ATT_ROWS_PER_WARP; ++i)
 #pragma unroll
-                for (int k = 0; k < ATT_ACC; ++k) {
-                    const int d = lane + 32 * k;
-                    if (d < hd) acc[i][k] += pj * vr[d];
+            for (int k = 0; k < ATT_ACC; ++k) acc[i][k] *= corr[i];
+#pragma unroll 4
+        for (int j = 0; j < ATT_TILE; ++j) {
+            const float4 pj = *reinterpret_cast<const float4*>(&Ps[warp][j][0]);
+            const float* vl = Vs + j * ld;
+#pragma unroll
+            for (int k = 0; k < ATT_ACC; ++k) {
+                const int d = lane + 32 * k;
+                if (d < hd) {
+                    const float vv = vl[d];
+                    acc[0][k] = fmaf(pj.x, vv, acc[0][k]);
+                    acc[1][k] = fmaf(pj.y, vv, acc[1][k]);
+                    acc[2][k] = fmaf(pj.z, vv, acc[2][k]);
+                    acc[3][k] = fmaf(pj.w, vv, acc[3][k]);
                 }
             }
         }
@@ -281,7 +374,7 @@ static int launch_attention_simt(const void* q, void* out, int dtype, const int*
     if (gy > 65535) return MLC_ERR_BAD_SIZE;
     PagedKV c{k_pool, v_pool, page_table, entry_offset, pages_per_seq, page_size, kv_heads, hd};
     dim3 grid((max_q_len + a.tokens_per_block - 1) / a.tokens_per_block, (unsigned)gy, n_seqs);
-    const size_t smem = (size_t)(ATT_ROWS * hd + ATT_TILE * (hd + 1) + ATT_TILE * hd) * sizeof(float);
+    const size_t smem = (size_t)(ATT_ROWS + 2 * ATT_TILE) * att_pitch(hd) * sizeof(float);
     cudaError_t e;
     // one instance per element type and accumulator count; each remembers how much shared memory it was allowed
 #define MLC_SIMT_LAUNCH(T, ACC)                                                                                          \

@@ -14,16 +14,16 @@
 // or on which kernel took the step.
 //
 // Three shapes of work:
-//   many rows (prompts)   tiles of 128 x 128 outputs, 8 x 8 per thread; operands come in
+//   many rows (prompts)   tiles of 128 x 128 or 64 x 64 outputs, 8 x 8 per thread; operands come in
 //                         16-byte loads into registers one K step ahead and go through a
 //                         double-buffered shared-memory tile;
-//   some rows             the same with tiles of 64 x 64, 4 x 4 per thread;
-//   few rows (decoding)   tiles of 16 rows x 64 columns.  Such a product is a stream of
-//                         weights with almost no arithmetic, and with few columns it has
-//                         too few tiles to keep the memory system busy: each block then
-//                         takes one chunk of K for its tile and leaves the chunk's sums in
-//                         scratch memory, and a second kernel adds the chunks in order.
-#include "common.cuh"
+//   few rows (decoding)   of a float32 matrix whose rows are 16-byte aligned: a stream of weights with almost no
+//                         arithmetic, `linear_few_kernel` below;
+//   few rows, other types or alignments   tiles of 16 rows x 64 columns.
+// Where the tiles alone would leave SMs idle, each block of the tiled kernel takes one chunk of K for its tile and
+// leaves the chunk's sums in scratch memory, and a second kernel adds the chunks in order.
+// 230 rows of x, B200, in brackets 128 x 128 tiles without chunks: 9,728 x 896 160 us (266), 896 x 4,864 89 us (350).
+#include "tcgen05.cuh"      // mbarriers with bounded waits, TMA tile loads, tensor maps, shared-memory addresses of a cluster's blocks
 
 namespace mlc {
 
@@ -82,13 +82,26 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
     const int k_begin = PARTIAL ? blockIdx.z * LS_CHUNK : 0;
     const int k_end = PARTIAL ? min(K, k_begin + LS_CHUNK) : K;
     const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
+    // a thread's rows and columns in groups of up to four side by side, the groups spread over the tile: neighbouring
+    // threads' 16-byte reads of a group are neighbours in shared memory and hit all banks once
+    constexpr int GM = TM < 4 ? TM : 4, GN = TN < 4 ? TN : 4;
+    auto row_of = [&](int i) { return (i / GM) * (BM / (TM / GM)) + ty * GM + i % GM; };
+    auto col_of = [&](int j) { return (j / GN) * (BN / (TN / GN)) + tx * GN + j % GN; };
     const bool x_vec = rows_vectorizable(x, K), w_vec = rows_vectorizable(w, K);
 
-    float total[TM][TN], acc[TM][TN];
+    // the totals of the 64 x 64 tile lie in shared memory, a column per thread: its blocks are small, and what hides their
+    // loads is how many of them an SM's registers hold
+    constexpr bool PARKED = !PARTIAL && BM == 64;
+    __shared__ float parked[PARKED ? TM * TN : 1][PARKED ? THREADS : 1];
+    float total[PARKED ? 1 : TM][PARKED ? 1 : TN], acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) total[i][j] = acc[i][j] = 0.0f;
+        for (int j = 0; j < TN; ++j) {
+            acc[i][j] = 0.0f;
+            if constexpr (PARKED) parked[i * TN + j][threadIdx.x] = 0.0f;
+            else total[i][j] = 0.0f;
+        }
 
     float4 xr[XV], wr[WV];
     auto fetch = [&](int k0) {
@@ -132,9 +145,9 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
         for (int kk = 0; kk < steps; ++kk) {
             float a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = xs[buf][kk][ty * TM + i];
+            for (int i = 0; i < TM; ++i) a[i] = xs[buf][kk][row_of(i)];
 #pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = ws[buf][kk][tx * TN + j];
+            for (int j = 0; j < TN; ++j) b[j] = ws[buf][kk][col_of(j)];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -145,7 +158,8 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    total[i][j] += acc[i][j];
+                    if constexpr (PARKED) parked[i * TN + j][threadIdx.x] += acc[i][j];
+                    else total[i][j] += acc[i][j];
                     acc[i][j] = 0.0f;
                 }
         }
@@ -157,13 +171,14 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        const int m = m0 + ty * TM + i;
+        const int m = m0 + row_of(i);
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tx * TN + j;
+            const int n = n0 + col_of(j);
             if (n >= N) continue;
-            if (PARTIAL) part[((long long)blockIdx.z * M + m) * N + n] = acc[i][j];
+            if constexpr (PARTIAL) part[((long long)blockIdx.z * M + m) * N + n] = acc[i][j];
+            else if constexpr (PARKED) y[(long long)m * N + n] = from_float<TY>(parked[i * TN + j][threadIdx.x]);
             else y[(long long)m * N + n] = from_float<TY>(total[i][j]);
         }
     }
@@ -175,40 +190,296 @@ __global__ void linear_simt_add_chunks_kernel(const float* __restrict__ part, TY
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= MN) return;
     float total = 0.0f;
+#pragma unroll 8
     for (int c = 0; c < n_chunks; ++c) total += part[(long long)c * MN + i];
     y[i] = from_float<TY>(total);
 }
 
+// ------------------------------------------------------------------ up to 16 rows of x, float32 operands, aligned rows
+// The order of summation wants one thread to walk a chunk of K, 256 multiply-adds that wait for one another, so the chunks go
+// to different warps: a warp takes 32 rows of W, one per lane, TOKENS rows of x and one chunk (or `pw` of them one after the
+// other), and the chunks' sums meet in shared memory, where they are added in ascending order; beyond eight warps' worth of
+// chunks the blocks of a cluster share them out and read one another's sums.  Neither a scratch array nor a second kernel is
+// needed.
+// Weights and tokens come by TMA into a ring of a warp's own, in boxes of 32 floats a row (seen as 64 16-bit elements, the
+// width of the other kernels' boxes) whose 16-byte pieces are swapped by the row's number modulo 8: a warp's reads, one row
+// per lane, hit all banks; the tokens' reads are broadcasts.  Warps do not wait for one another before the end of a tile,
+// and the ring runs on from tile to tile.
+// What bounds it: memory for large matrices; for small ones the launch, the first trip to memory and a chunk's chain (1,024
+// cycles at least); from nine rows on the tokens' reads.  B200, one kernel of a chain in a graph, 3 rows, in brackets tiles of
+// 16 x 64 with the chunks' sums in scratch memory and a second kernel: 1,152 x 896 5.4 us, 896 x 896 5.4, 896 x 4,864 8.5,
+// 9,728 x 896 8.2 (17 and 2 for the second kernel on the average of the four), 151,936 x 896 84 us = 6.5 TB/s (257).  With a ring of four
+// stages an SM holds one block instead of two: 9,728 x 896 12.1 us, 151,936 x 896 95.
+constexpr int LF_BOX = 32;              // elements of K in a stage
+constexpr int LF_ROW_BYTES = 128;
+constexpr int LF_ROWS = 32;
+constexpr int LF_SLOTS = 3;
+constexpr int LF_MAX_WARPS = 8;
+constexpr int LF_MAX_CLUSTER = 8;
+constexpr int LF_MAX_PW = 4;
+
+__host__ __device__ constexpr int lf_slot_bytes(int tokens) { return LF_ROWS * LF_ROW_BYTES + (tokens + 7) / 8 * 1024; }      // boxes begin on 1024-byte boundaries
+
+__device__ __forceinline__ float load_cluster_float(unsigned cluster_addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
+
+template <typename TY, int TOKENS>
+__global__ void __launch_bounds__(32 * LF_MAX_WARPS)
+linear_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, TY* __restrict__ y, int M, int N,
+                  int K, int n_chunks, int pw, int cluster, int tiles, int* status) {
+    constexpr int SLOT_BYTES = lf_slot_bytes(TOKENS), W_BYTES = LF_ROWS * LF_ROW_BYTES;
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    extern __shared__ unsigned char lf_smem[];
+    unsigned char* const smem = lf_smem + ((1024u - (smem_u32(lf_smem) & 1023u)) & 1023u);
+    unsigned char* const ring = smem + warp * LF_SLOTS * SLOT_BYTES;                                // [SLOTS][W box, x box]
+    float* const sums = reinterpret_cast<float*>(smem + warps * LF_SLOTS * SLOT_BYTES);             // [2][warps * pw][TOKENS][LF_ROWS]
+    __shared__ __align__(8) unsigned long long full_bars[LF_MAX_WARPS * LF_SLOTS];
+    const unsigned ring_at = smem_u32(ring), bars = smem_u32(full_bars) + 8u * (unsigned)(warp * LF_SLOTS);
+    const int rank = cluster > 1 ? (int)cluster_rank() : 0;
+    const int first_tile = blockIdx.x / cluster, tile_step = gridDim.x / cluster;
+    const int chunk0 = (rank * warps + warp) * pw, chunk1 = min(n_chunks, chunk0 + pw);
+    const int k_begin = chunk0 * LS_CHUNK, k_end = min(K, chunk1 * LS_CHUNK);
+    const int stages = k_end > k_begin ? (k_end - k_begin + LF_BOX - 1) / LF_BOX : 0;               // of one tile
+    const int my_tiles = first_tile < tiles ? (tiles - first_tile + tile_step - 1) / tile_step : 0;
+    const int total_stages = my_tiles * stages;
+
+    grid_launch_dependents();
+    int ask_tile = first_tile, ask_stage = 0;
+    auto ask = [&](int slot, bool weights, bool tokens) {
+        const int c = 2 * (k_begin + ask_stage * LF_BOX);
+        const unsigned at = ring_at + (unsigned)(slot * SLOT_BYTES), bar = bars + 8u * (unsigned)slot;
+        if (weights) {
+            mbar_expect_tx(bar, W_BYTES + TOKENS * LF_ROW_BYTES);
+            tma_load_2d(at, &map_w, c, ask_tile * LF_ROWS, bar);
+        }
+        if (tokens) tma_load_2d(at + W_BYTES, &map_x, c, 0, bar);
+    };
+    auto next = [&]() {
+        if (++ask_stage == stages) {
+            ask_stage = 0;
+            ask_tile += tile_step;
+        }
+    };
+    const int early = min(LF_SLOTS, total_stages);
+    if (lane == 0) {
+        for (int s = 0; s < LF_SLOTS; ++s) mbar_init(bars + 8u * s, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int s = 0; s < early; ++s, next()) ask(s, true, false);          // the weights depend on nothing
+    }
+    __syncwarp();
+    grid_dependency_wait();
+    if (lane == 0) {
+        ask_tile = first_tile;
+        ask_stage = 0;
+        for (int s = 0; s < early; ++s, next()) ask(s, false, true);
+    }
+
+    int slot = 0, round = 0, done = 0, parity = 0;
+    bool ok = true;
+    for (int tile = first_tile; tile < tiles; tile += tile_step, parity ^= 1) {
+        float* const mine = sums + ((parity * warps + warp) * pw) * TOKENS * LF_ROWS;
+        float acc[TOKENS];
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) acc[t] = 0.0f;
+        for (int s = 0; s < stages && ok; ++s) {
+            ok = __all_sync(0xffffffffu, mbar_wait(bars + 8u * (unsigned)slot, (unsigned)round & 1u, status, 61));
+            if (!ok) break;
+            const unsigned char* const wr = ring + slot * SLOT_BYTES + lane * LF_ROW_BYTES;
+            const unsigned char* const xr = ring + slot * SLOT_BYTES + W_BYTES;
+            float4 wv[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) wv[q] = *reinterpret_cast<const float4*>(wr + ((q ^ (lane & 7)) << 4));
+            // what lies beyond K has arrived as zeros, which change no sum
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+#pragma unroll
+                for (int g = 0; g < TOKENS; g += 4) {
+                    float4 xv[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) xv[t] = *reinterpret_cast<const float4*>(xr + (g + t) * LF_ROW_BYTES + ((q ^ ((g + t) & 7)) << 4));
+                    // token after token, not term after term: the multiply-adds of one sum wait for one another
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) acc[g + t] = fmaf(xv[t].x, wv[q].x, acc[g + t]);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) acc[g + t] = fmaf(xv[t].y, wv[q].y, acc[g + t]);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) acc[g + t] = fmaf(xv[t].z, wv[q].z, acc[g + t]);
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) acc[g + t] = fmaf(xv[t].w, wv[q].w, acc[g + t]);
+                }
+            }
+            if ((s + 1) % (LS_CHUNK / LF_BOX) == 0 || s + 1 == stages) {       // a chunk is complete
+#pragma unroll
+                for (int t = 0; t < TOKENS; ++t) {
+                    mine[((s / (LS_CHUNK / LF_BOX)) * TOKENS + t) * LF_ROWS + lane] = acc[t];
+                    acc[t] = 0.0f;
+                }
+            }
+            __syncwarp();                                            // the slot has been read
+            if (lane == 0 && done + LF_SLOTS < total_stages) {
+                ask(slot, true, true);
+                next();
+            }
+            ++done;
+            if (++slot == LF_SLOTS) {
+                slot = 0;
+                ++round;
+            }
+        }
+        // the other set of sums takes the next tile's, so one barrier a tile is enough
+        const bool all_ok = __syncthreads_and(ok);
+        if (cluster == 1 && all_ok) {
+            for (int o = threadIdx.x; o < TOKENS * LF_ROWS; o += blockDim.x) {
+                const int n = tile * LF_ROWS + o % LF_ROWS, m = o / LF_ROWS;
+                if (m >= M || n >= N) continue;
+                const float* const at = sums + parity * warps * pw * TOKENS * LF_ROWS + o;
+                float total = 0.0f;
+#pragma unroll 8
+                for (int c = 0; c < n_chunks; ++c) total += at[c * TOKENS * LF_ROWS];
+                y[(long long)m * N + n] = from_float<TY>(total);
+            }
+        }
+        ok = all_ok;
+    }
+    if (cluster > 1) {                                               // one tile per cluster; its blocks share out the outputs
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const unsigned sums_at = smem_u32(sums);
+        const int per = warps * pw;
+        for (int o = rank * blockDim.x + threadIdx.x; o < TOKENS * LF_ROWS; o += cluster * blockDim.x) {
+            const int n = first_tile * LF_ROWS + o % LF_ROWS, m = o / LF_ROWS;
+            if (m >= M || n >= N || !ok) continue;
+            float total = 0.0f;
+#pragma unroll 8
+            for (int c = 0; c < n_chunks; ++c) {
+                const int r = c / per;
+                total += load_cluster_float(cluster_map(sums_at + (unsigned)((c - r * per) * TOKENS * LF_ROWS + o) * 4u, r));
+            }
+            y[(long long)m * N + n] = from_float<TY>(total);
+        }
+        // nobody leaves while another block may still read its sums
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+
+// K's chunks over the warps of a block, the blocks of a cluster and, only beyond those, a warp's time.
+struct FewPlan { int warps, cluster, pw; };
+static FewPlan few_plan(int K) {
+    const int n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
+    const int pw = (n_chunks + LF_MAX_WARPS * LF_MAX_CLUSTER - 1) / (LF_MAX_WARPS * LF_MAX_CLUSTER), shares = (n_chunks + pw - 1) / pw;
+    const int cluster = (shares + LF_MAX_WARPS - 1) / LF_MAX_WARPS;
+    return FewPlan{(shares + cluster - 1) / cluster, cluster, pw};
+}
+
+template <typename TY, int TOKENS>
+static int launch_few(const float* x, const float* w, TY* y, int M, int N, int K, int* status, int n_sms, cudaStream_t s) {
+    const int tiles = (N + LF_ROWS - 1) / LF_ROWS, n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
+    const FewPlan p = few_plan(K);
+    static_assert((size_t)LF_MAX_WARPS * (LF_SLOTS * lf_slot_bytes(TOKENS) + 2 * (TOKENS > 8 ? 1 : LF_MAX_PW) * TOKENS * LF_ROWS * sizeof(float)) + 2048 <= 227 * 1024, "shared memory of a block");
+    const size_t smem = (size_t)p.warps * (LF_SLOTS * lf_slot_bytes(TOKENS) + 2 * p.pw * TOKENS * LF_ROWS * sizeof(float)) + 1024 /* alignment slack */;
+    if (smem + 1024 > 227 * 1024) return MLC_ERR_BAD_SIZE;           // (takes_few has seen to it)
+    CUtensorMap mx, mw;
+    int rc = cached_map_2d(&mx, x, M, 2LL * K, 64, TOKENS);
+    if (rc) return rc;
+    rc = cached_map_2d(&mw, w, N, 2LL * K, 64, LF_ROWS);
+    if (rc) return rc;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(linear_few_kernel<TY, TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const long long resident = (long long)n_sms * (long long)(227 * 1024 / (smem + 1024));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.cluster > 1 ? (long long)tiles * p.cluster : tiles < resident ? tiles : resident));
+    cfg.blockDim = dim3(32 * p.warps);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.cluster > 1 ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, linear_few_kernel<TY, TOKENS>, mx, mw, y, M, N, K, n_chunks, p.pw, p.cluster, tiles, status);
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+// Whether the product takes the kernel above.
+static bool takes_few(int x_dtype, int w_dtype, const void* x, const void* w, int M, int K) {
+    return x_dtype == MLC_DTYPE_F32 && w_dtype == MLC_DTYPE_F32 && M <= 16 && (K & 3) == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 &&
+           few_plan(K).pw <= (M > 8 ? 1 : LF_MAX_PW);
+}
+
+template <typename TY>
+static int launch_few_rows(const float* x, const float* w, TY* y, int M, int N, int K, int* status, int n_sms, cudaStream_t s) {
+    if (M <= 4) return launch_few<TY, 4>(x, w, y, M, N, K, status, n_sms, s);
+    if (M <= 8) return launch_few<TY, 8>(x, w, y, M, N, K, status, n_sms, s);
+    return launch_few<TY, 16>(x, w, y, M, N, K, status, n_sms, s);
+}
+
+// The tile of a product of more than 16 rows: 128 x 128 where those fill the GPU four times over (a block has an SM almost
+// for itself, so a short last wave costs a whole tile), else 64 x 64; and whether its blocks take single chunks of K.
+struct TilePlan { bool large; bool chunks; long long scratch; };
+constexpr long long LS_MAX_SCRATCH = 32LL << 20;          // floats: 128 MB
+static TilePlan tile_plan(int M, int N, int K, int n_sms) {
+    const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128), t64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
+    const int n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
+    const long long need = (long long)n_chunks * M * N;
+    TilePlan p{t128 >= 4LL * n_sms, false, 0};
+    p.chunks = !p.large && t64 < 3LL * n_sms && n_chunks > 1 && n_chunks <= 65535 && need <= LS_MAX_SCRATCH;
+    if (p.chunks) p.scratch = need;
+    return p;
+}
+
 template <typename TX, typename TW, typename TY>
 static int launch_linear(const void* x, const void* w, void* y, float* scratch, long long scratch_floats, int M, int N, int K,
-                         int n_sms, cudaStream_t s) {
+                         int* status, int n_sms, cudaStream_t s) {
     const TX* xp = (const TX*)x;
     const TW* wp = (const TW*)w;
     TY* yp = (TY*)y;
-    if (M > 64) {
-        dim3 grid((N + 127) / 128, (M + 127) / 128);
-        if (grid.y > 65535) return MLC_ERR_BAD_SIZE;
-        linear_simt_kernel<TX, TW, TY, 128, 128, 8, 8, false><<<grid, 256, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
-    } else if (M > 16) {
-        dim3 grid((N + 63) / 64, (M + 63) / 64);
-        linear_simt_kernel<TX, TW, TY, 64, 64, 4, 4, false><<<grid, 256, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
+    const int n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
+    const long long MN = (long long)M * N;
+    bool chunks = false;
+    if (M > 16) {
+        const TilePlan p = tile_plan(M, N, K, n_sms);
+        chunks = p.chunks && scratch != nullptr && scratch_floats >= p.scratch;
+        if (p.large || (M + 63) / 64 > 65535) {
+            dim3 grid((N + 127) / 128, (M + 127) / 128);
+            if (grid.y > 65535) return MLC_ERR_BAD_SIZE;
+            linear_simt_kernel<TX, TW, TY, 128, 128, 8, 8, false><<<grid, 256, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
+        } else if (chunks) {
+            dim3 grid((N + 63) / 64, (M + 63) / 64, n_chunks);
+            linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, true><<<grid, 64, 0, s>>>(xp, wp, yp, scratch, M, N, K);
+        } else {
+            dim3 grid((N + 63) / 64, (M + 63) / 64);
+            linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, false><<<grid, 64, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
+        }
     } else {
-        const int n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
+        if constexpr (sizeof(TX) == 4 && sizeof(TW) == 4) {
+            if (takes_few(MLC_DTYPE_F32, MLC_DTYPE_F32, x, w, M, K)) return launch_few_rows<TY>(xp, wp, yp, M, N, K, status, n_sms, s);
+        }
         const int tiles = (N + 63) / 64;
-        const long long need = (long long)n_chunks * M * N;
         // few tiles: a block per (tile, chunk) and a second kernel that adds the chunks, if the caller gave room for them
-        if (tiles < 4 * n_sms && n_chunks > 1 && n_chunks <= 65535 && scratch != nullptr && scratch_floats >= need) {
+        chunks = tiles < 4 * n_sms && n_chunks > 1 && n_chunks <= 65535 && scratch != nullptr && scratch_floats >= n_chunks * MN;
+        if (chunks) {
             dim3 grid(tiles, 1, n_chunks);
             linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, true><<<grid, 128, 0, s>>>(xp, wp, yp, scratch, M, N, K);
-            MLC_LAUNCH_CHECK();
-            const long long MN = (long long)M * N;
-            linear_simt_add_chunks_kernel<TY><<<(unsigned)((MN + 255) / 256), 256, 0, s>>>(scratch, yp, MN, n_chunks);
         } else {
             dim3 grid(tiles, 1);
             linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, false><<<grid, 128, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
         }
     }
     MLC_LAUNCH_CHECK();
+    if (chunks) {
+        linear_simt_add_chunks_kernel<TY><<<(unsigned)((MN + 255) / 256), 256, 0, s>>>(scratch, yp, MN, n_chunks);
+        MLC_LAUNCH_CHECK();
+    }
     return 0;
 }
 
@@ -216,32 +487,34 @@ static int launch_linear(const void* x, const void* w, void* y, float* scratch, 
 
 using namespace mlc;
 
-// Floats of scratch memory a product of these sizes can use (0: none): room for each K chunk's sums when few rows meet
-// few columns.  Without it the product still runs, with fewer blocks.
-extern "C" long long mlc_linear_simt_scratch_floats(int M, int N, int K, int n_sms) {
-    if (M <= 0 || M > 16 || N <= 0 || K <= LS_CHUNK) return 0;
-    if ((N + 63) / 64 >= 4 * n_sms) return 0;
+// Floats of scratch memory a product of these sizes can use (0: none): room for each K chunk's sums when the tiles alone
+// are few.  Without it the product still runs, with fewer blocks.
+extern "C" long long mlc_linear_simt_scratch_floats(const void* x, int x_dtype, const void* w, int w_dtype, int M, int N, int K, int n_sms) {
+    if (M <= 0 || N <= 0 || K <= LS_CHUNK || n_sms < 1) return 0;
+    if (M > 16) return tile_plan(M, N, K, n_sms).scratch;
+    if (takes_few(x_dtype, w_dtype, x, w, M, K) || (N + 63) / 64 >= 4 * n_sms) return 0;
     return (long long)((K + LS_CHUNK - 1) / LS_CHUNK) * M * N;
 }
 
 // x [M][K] of x_dtype, w [N][K] of w_dtype, y [M][N] of y_dtype; all row-major and dense.  scratch: null, or
-// `scratch_floats` floats of device memory (see mlc_linear_simt_scratch_floats).
+// `scratch_floats` floats of device memory (see mlc_linear_simt_scratch_floats).  status: one int on the device, 0 before the
+// call; a bounded wait that ran out leaves 61 there.
 extern "C" int mlc_linear_simt(const void* x, int x_dtype, const void* w, int w_dtype, void* y, int y_dtype,
-                               int M, int N, int K, float* scratch, long long scratch_floats, int n_sms, void* stream) {
+                               int M, int N, int K, float* scratch, long long scratch_floats, int* status, int n_sms, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || n_sms < 1) return MLC_ERR_BAD_SIZE;
+    if (K <= 0 || n_sms < 1 || status == nullptr) return MLC_ERR_BAD_SIZE;
     if ((x_dtype | w_dtype | y_dtype) & ~1) return MLC_ERR_BAD_DTYPE;
     cudaStream_t s = (cudaStream_t)stream;
     const int code = x_dtype * 4 + w_dtype * 2 + y_dtype;
     switch (code) {
-        case 0: return launch_linear<float, float, float>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 1: return launch_linear<float, float, bf16>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 2: return launch_linear<float, bf16, float>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 3: return launch_linear<float, bf16, bf16>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 4: return launch_linear<bf16, float, float>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 5: return launch_linear<bf16, float, bf16>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 6: return launch_linear<bf16, bf16, float>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
-        case 7: return launch_linear<bf16, bf16, bf16>(x, w, y, scratch, scratch_floats, M, N, K, n_sms, s);
+        case 0: return launch_linear<float, float, float>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 1: return launch_linear<float, float, bf16>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 2: return launch_linear<float, bf16, float>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 3: return launch_linear<float, bf16, bf16>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 4: return launch_linear<bf16, float, float>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 5: return launch_linear<bf16, float, bf16>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 6: return launch_linear<bf16, bf16, float>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
+        case 7: return launch_linear<bf16, bf16, bf16>(x, w, y, scratch, scratch_floats, M, N, K, status, n_sms, s);
     }
     return MLC_ERR_BAD_DTYPE;
 }

@@ -133,7 +133,7 @@ def core() -> ctypes.CDLL:
             "mlc_gla": [P, LL, I, I, I, P, P, F, P, LL, P, P, I, I, I, I, I, I, P, P],
             "mlc_latent_prepare": [P, LL, P, LL, I, I, I, P, F, P, P, P, I, I, I, I, I, I, I, P, I, I, P, P, LL, I, I, P],
             "mlc_head_project": [P, I, LL, LL, P, I, LL, LL, LL, P, I, LL, LL, I, I, I, I, P, LL, P],
-            "mlc_linear_simt": [P, I, P, I, P, I, I, I, I, P, LL, I, P],
+            "mlc_linear_simt": [P, I, P, I, P, I, I, I, I, P, LL, P, I, P],
             "mlc_attention_combine": [P, P, LL, I, I, P, I, P, I, P],
             "mlc_gemm_tcgen05": [P, P, P, I, I, I, I, I, I, I, P, P, I, P, P, P, P, I, I, I, I, P, P, P, LL, I, I, I, F, F, P],
             "mlc_gemm_few": [P, P, F, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P, P, I, I, I, I, P, P, P, LL, I, I, I, F, F, P],
@@ -150,7 +150,7 @@ def core() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = c_int
-        lib.mlc_linear_simt_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
+        lib.mlc_linear_simt_scratch_floats.argtypes = [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int]
         lib.mlc_linear_simt_scratch_floats.restype = c_longlong
         lib.mlc_gla_rows.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.mlc_gla_rows.restype = c_int
@@ -332,12 +332,12 @@ def linear_simt(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, n_sms: int = 
     if n_sms <= 0:
         n_sms = _sm_count(x.device)
     lib = core()
-    need = lib.mlc_linear_simt_scratch_floats(m, n, k, n_sms)
+    need = lib.mlc_linear_simt_scratch_floats(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype), m, n, k, n_sms)
     scratch = torch.empty(need, dtype=torch.float32, device=x.device) if need > 0 else None
     if scratch is not None:
         count_launches(1)                       # the kernel that adds the chunks
     _check(lib.mlc_linear_simt(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype), y.data_ptr(),
-                               dtype_code(y.dtype), m, n, k, _ptr(scratch), need, n_sms, _stream()), "linear")
+                               dtype_code(y.dtype), m, n, k, _ptr(scratch), need, gemm_status(x.device).data_ptr(), n_sms, _stream()), "linear")
 
 
 _argmax_scratch = {}
@@ -1315,7 +1315,8 @@ def check_gemm_status(device: torch.device) -> None:
                    12: "the attention kernel's tensor-core issuer", 13: "the attention kernel's softmax rows",
                    21: "the prompt product's TMA loader", 22: "the prompt product's tensor-core issuer",
                    23: "the prompt product's epilogue", 31: "the single-token attention kernel's wait for keys and values", 41: "the paired prompt product's TMA loader",
-                   42: "the paired prompt product's tensor-core issuer or relay", 43: "the paired prompt product's epilogue"}.get(code, str(code))
+                   42: "the paired prompt product's tensor-core issuer or relay", 43: "the paired prompt product's epilogue",
+                   61: "the float32 few-row product's wait for its operands"}.get(code, str(code))
             raise KernelError(f"a tcgen05 kernel gave up waiting on a barrier ({who}); its output is not valid")
 
 
