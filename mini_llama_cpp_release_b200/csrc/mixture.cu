@@ -298,10 +298,11 @@ moe_plan_kernel(const int* __restrict__ ids, const int* __restrict__ tokens, con
     __syncthreads();
     if (threadIdx.x == 0) {
         int at = 0;
+        const int stretches = (n_pairs + per - 1) / per;             // that hold pairs: one in a decode step
         for (int e = 0; e < E; ++e) {
             start[e] = at;
             int c = 0;
-            for (int w = 0; w < 32; ++w) {
+            for (int w = 0; w < stretches; ++w) {
                 const int here = cnt[w * E + e];
                 cnt[w * E + e] = at + c;
                 c += here;

@@ -17,7 +17,7 @@ __all__ = [
     "launch_count", "reset_launch_count", "library_launch_count", "count_library_launches", "attention_mma_available", "attention_mma", "attention_mma_plan", "attention_decode_cluster_limit", "attention_decode_splits", "attention_decode_clusters_resident", "attention_tcgen05", "attention_tcgen05_takes", "attention_tcgen05_blocks", "attention_library", "gemm_tcgen05", "gemm_few", "gemm_few_plan", "gemm_qkv_cluster_splits", "gemm_qkv_clusters_resident", "gemm_tcgen05_rows", "gemm_rows_takes", "gemm_rows_add_plan", "gemm_add_plan", "gemm_tcgen05_pair", "gemm_pair_takes", "gemm_prompt", "library_gemm", "gemm_status", "check_gemm_status", "set_pdl", "PinnedCopy", "decode_advance",
     "layernorm", "qk_norm_rope_cache", "softcap", "convert", "causal_conv", "gated_delta_rule", "gated_rmsnorm", "block_gates",
     "linear_scan", "gates_scan_step", "gates_scan_step_takes",
-    "moe_route", "moe_plan", "moe_plan_rows", "grouped_linear", "moe_gather", "moe_combine", "scaled_add", "scaled_add_experts", "gla", "gla_slices", "latent_prepare",
+    "moe_route", "moe_plan", "moe_plan_rows", "grouped_linear", "gemm_few_grouped", "gemm_few_grouped_takes", "moe_gather", "moe_combine", "scaled_add", "scaled_add_experts", "gla", "gla_slices", "latent_prepare",
     "head_project", "gemm_tcgen05_grouped", "GROUPED_TILE",
     "group_norm", "activation", "forget_gate_attention", "moe_route_scored",
     "tanh_norm", "glu", "sigmoid_gate", "state_space",
@@ -112,6 +112,7 @@ def core() -> ctypes.CDLL:
             "mlc_moe_route": [P, I, P, P, I, I, I, I, I, P, P, P],
             "mlc_moe_plan": [P, I, I, I, I, I, P, P, P, P],
             "mlc_moe_plan_table": [P, P, F, P, I, I, I, I, I, P, P, P, P],
+            "mlc_gemm_few_grouped": [P, P, P, P, P, I, I, I, I, I, I, I, F, F, I, P],
             "mlc_decay_attention": [P, LL, I, I, I, P, P, F, F, P, LL, P, P, I, I, I, I, I, I, I, P, P, P, I, P],
             "mlc_matrix_memory": [P, LL, I, I, I, I, I, I, P, P, F, P, F, P, LL, P, P, I, I, I, I, I, I, I, P, P, P, P, I, P],
             "mlc_rms_pair": [P, P, I, P, P, P, I, P, P, F, I, I, P, P, I, P],
@@ -154,6 +155,8 @@ def core() -> ctypes.CDLL:
         lib.mlc_linear_simt_scratch_floats.restype = c_longlong
         lib.mlc_gla_rows.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.mlc_gla_rows.restype = c_int
+        lib.mlc_gemm_few_grouped_max_k.argtypes = []
+        lib.mlc_gemm_few_grouped_max_k.restype = c_int
         lib.mlc_gla_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
         lib.mlc_gla_chunk_floats.restype = c_longlong
         lib.mlc_set_pdl.argtypes = [c_int]
@@ -1649,6 +1652,27 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int,
                                epilogue, *plan, _ptr(bias), _ptr(positions), _ptr(tok_seq), _ptr(rope),
                                rope.shape[0] if rope is not None else 0, q_heads, kv_heads, head_dim, *cache, *_glu_args(glu),
                                _stream()), "few-row matrix product")
+
+
+def gemm_few_grouped_takes(n_pairs: int, n_out: int, k: int) -> bool:
+    """Whether csrc/gemm_few_grouped.cu takes the experts' product of `n_pairs` (token, choice) pairs."""
+    return 1 <= n_pairs <= 16 and k % 64 == 0 and 0 < k <= core().mlc_gemm_few_grouped_max_k() and n_out % 2 == 0
+
+
+def gemm_few_grouped(x: torch.Tensor, src_tok: Optional[torch.Tensor], w: torch.Tensor, tile_group: torch.Tensor, group_rows: int,
+                     out: torch.Tensor, epilogue: int, n_sms: int, glu=None) -> None:
+    """out[row] = w[tile_group[row // group_rows]] x[src_tok[row]] (x[row] without src_tok) for the runs of a `moe_plan` with
+    tiles of `group_rows` <= 16 rows; w bfloat16 [E, N, K], epilogue EPI_STORE or EPI_SILU_MUL."""
+    require_cuda(x, src_tok, w, tile_group, out)
+    E, n_out, K = w.shape
+    groups = tile_group.numel()
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or epilogue not in (EPI_STORE, EPI_SILU_MUL):
+        raise KernelError("the experts' few-row product takes bfloat16 operands and the store and gated epilogues")
+    assert x.shape[1] == K and tile_group.dtype == torch.int32 and out.shape == (groups * group_rows, n_out // 2 if epilogue == EPI_SILU_MUL else n_out)
+    assert (x.shape[0] == groups * group_rows) if src_tok is None else (src_tok.dtype == torch.int32 and src_tok.numel() == groups * group_rows)
+    _check(core().mlc_gemm_few_grouped(x.data_ptr(), _ptr(src_tok), w.data_ptr(), tile_group.data_ptr(), out.data_ptr(),
+                                       dtype_code(out.dtype), groups, int(group_rows), n_out, K, 1 if epilogue == EPI_SILU_MUL else 0,
+                                       *_glu_args(glu), n_sms, _stream()), "experts' few-row product")
 
 
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int = 0, n_splits: int = 1,

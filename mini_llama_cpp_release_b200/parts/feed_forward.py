@@ -288,7 +288,11 @@ class MixtureOfExperts(Part):
         n = h.shape[0]
         by_table = self.routing == "table"
         ids, weights = (None, rt.empty(n, self.top, dtype=torch.float32)) if by_table else self.route(h)
-        tile = kernels.GROUPED_TILE if self.fused else self.TILE
+        # few pairs: the experts' weights stream through the few-row product, which gathers the rows itself; a run then has
+        # at most as many rows as there are pairs, and is padded to one or two tiles of eight
+        few = (self.fused and self.gated and not self.weight_on_input and kernels.gemm_few_grouped_takes(n * self.top, 2 * self.inter, self.hidden)
+               and kernels.gemm_few_grouped_takes(n * self.top, self.hidden, self.inter))
+        tile = (8 if n * self.top <= 8 else 16) if few else kernels.GROUPED_TILE if self.fused else self.TILE
         rows = kernels.moe_plan_rows(n * self.top, self.E, tile)
         row_of = rt.empty(n, self.top, dtype=torch.int32)
         src_tok = rt.empty(rows, dtype=torch.int32)
@@ -300,7 +304,10 @@ class MixtureOfExperts(Part):
         y = rt.empty(rows, self.hidden, dtype=torch.float32)
         act = rt.empty(rows, self.inter)
         on_input = (weights, row_of) if self.weight_on_input else (None, None)
-        if self.fused:
+        if few:
+            kernels.gemm_few_grouped(h, src_tok, self.gate_up, tile_expert, tile, act, kernels.bindings.EPI_SILU_MUL, rt.n_sms, glu=self.glu)
+            kernels.gemm_few_grouped(act, None, self.down, tile_expert, tile, y, kernels.bindings.EPI_STORE, rt.n_sms)
+        elif self.fused:
             hs = rt.empty(rows, self.hidden)
             kernels.moe_gather(h, src_tok, hs, *on_input)            # the sorted rows, dense, as the product's TMA loads want them
             if self.gated:
