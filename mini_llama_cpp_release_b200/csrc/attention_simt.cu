@@ -58,6 +58,8 @@ __host__ __device__ __forceinline__ int att_pitch(int hd) { return 4 * (((hd + 3
 template <typename T, int ATT_ACC>        // ATT_ACC: output entries a lane holds per row, head size <= 32 * ATT_ACC
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attention_simt_kernel(AttnArgs a, PagedKV c) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     extern __shared__ float smem[];
     const int hd = c.head_dim;
     const int ld = att_pitch(hd);                  // a row's floats in shared memory
@@ -385,7 +387,7 @@ static int launch_attention_simt(const void* q, void* out, int dtype, const int*
             if (e != cudaSuccess) return (int)e;                                                                         \
             allowed = smem;                                                                                              \
         }                                                                                                                \
-        attention_simt_kernel<T, ACC><<<grid, ATT_WARPS * 32, smem, s>>>(a, c);                                          \
+        launch_pdl(attention_simt_kernel<T, ACC>, grid, dim3(ATT_WARPS * 32), smem, s, a, c);                                          \
     } while (0)
     if (dtype == MLC_DTYPE_F32) {
         if (hd <= 256) MLC_SIMT_LAUNCH(float, 8);

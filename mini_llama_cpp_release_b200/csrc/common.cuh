@@ -41,7 +41,9 @@ typedef __nv_bfloat16 bf16;
 // running; it must call grid_dependency_wait() before it reads anything an earlier kernel wrote
 // (the wait returns once every earlier kernel has finished and its writes are visible), and it
 // calls grid_launch_dependents() to let the kernel after it start in the same way.  The launch
-// latency of a chain of short kernels then overlaps with their execution.
+// latency of a chain of short kernels then overlaps with their execution.  Small kernels of a decode step do both first of
+// all; B200, launched so instead of in the ordinary way: 48 tokens of 8 Betepel prompts 36.4 -> 32.2 ms, of 4 Mepolix prompts
+// 19.45 -> 19.16.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -192,6 +192,8 @@ __global__ void qkv_post_kernel(const float* __restrict__ qkv, const float* __re
                                 const int* __restrict__ positions, const int* __restrict__ tok_seq,
                                 const float2* __restrict__ rope, int rope_positions, int q_heads,
                                 int kv_heads_in_row, int hd, T* __restrict__ q_out, PagedKV cache) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int n = blockIdx.x;
     const int half = hd >> 1;
     const int row_width = (q_heads + 2 * kv_heads_in_row) * hd;
@@ -242,6 +244,8 @@ __global__ void qkv_post_kernel(const float* __restrict__ qkv, const float* __re
 template <typename TIn, typename TOut>
 __global__ void silu_mul_kernel(const TIn* __restrict__ gu, int inter, long long total, int interleaved,
                                 TOut* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const long long n = idx / inter;
@@ -256,6 +260,8 @@ __global__ void silu_mul_kernel(const TIn* __restrict__ gu, int inter, long long
 // Eight outputs per thread with 16-byte loads and stores (bfloat16 in and out, I a multiple of 8).
 __global__ void silu_mul_vec8_kernel(const bf16* __restrict__ gu, int inter, long long total_vec, int interleaved,
                                      bf16* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total_vec) return;
     const int per_row = inter >> 3;
@@ -576,6 +582,8 @@ __global__ void qk_norm_rope_cache_kernel(const float* __restrict__ proj, long l
                                           const float2* __restrict__ rope, int rope_positions, int rot_dims, int q_heads,
                                           int kv_heads_in_row, int dim, int vdim, int D, float v_scale, T* __restrict__ q_out,
                                           PagedKV cache, QkOptions opt) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int n = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     const float* row = proj + (long long)n * stride;
@@ -775,11 +783,11 @@ extern "C" int mlc_qk_norm_rope_cache(const float* proj, long long stride, int q
     const int heads = q_heads + (maps + 1) * kv_heads_in_row;
     const int threads = 32 * (heads < 8 ? heads : 8);
     if (dtype == MLC_DTYPE_F32)
-        qk_norm_rope_cache_kernel<float><<<n, threads, 0, s>>>(proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
+        launch_pdl(qk_norm_rope_cache_kernel<float>, dim3(n), dim3(threads), 0, s, proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
                                                                tok_seq, (const float2*)rope_table, rope_positions, rot_dims, q_heads,
                                                                kv_heads_in_row, dim, vdim, D, v_scale, (float*)q_out, c, opt);
     else if (dtype == MLC_DTYPE_BF16)
-        qk_norm_rope_cache_kernel<bf16><<<n, threads, 0, s>>>(proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
+        launch_pdl(qk_norm_rope_cache_kernel<bf16>, dim3(n), dim3(threads), 0, s, proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
                                                               tok_seq, (const float2*)rope_table, rope_positions, rot_dims, q_heads,
                                                               kv_heads_in_row, dim, vdim, D, v_scale, (bf16*)q_out, c, opt);
     else
@@ -817,11 +825,11 @@ extern "C" int mlc_qkv_post(const float* qkv, const float* bias, const int* posi
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = row_threads((q_heads + kv_heads_in_row) * hd / 2);
     if (dtype == MLC_DTYPE_F32)
-        qkv_post_kernel<float><<<n, threads, 0, s>>>(qkv, bias, positions, tok_seq, (const float2*)rope_table,
+        launch_pdl(qkv_post_kernel<float>, dim3(n), dim3(threads), 0, s, qkv, bias, positions, tok_seq, (const float2*)rope_table,
                                                      rope_positions, q_heads, kv_heads_in_row, hd,
                                                      (float*)q_out, c);
     else if (dtype == MLC_DTYPE_BF16)
-        qkv_post_kernel<bf16><<<n, threads, 0, s>>>(qkv, bias, positions, tok_seq, (const float2*)rope_table,
+        launch_pdl(qkv_post_kernel<bf16>, dim3(n), dim3(threads), 0, s, qkv, bias, positions, tok_seq, (const float2*)rope_table,
                                                     rope_positions, q_heads, kv_heads_in_row, hd, (bf16*)q_out,
                                                     c);
     else
@@ -840,19 +848,19 @@ extern "C" int mlc_silu_mul(const void* gate_up, int in_dtype, int n, int inter,
     if (in_dtype == MLC_DTYPE_BF16 && out_dtype == MLC_DTYPE_BF16 && (inter & 7) == 0 &&
         ((((uintptr_t)gate_up) | ((uintptr_t)out)) & 15) == 0) {
         const long long total_vec = total >> 3;
-        silu_mul_vec8_kernel<<<(unsigned)((total_vec + 255) / 256), 256, 0, s>>>((const bf16*)gate_up, inter, total_vec,
+        launch_pdl(silu_mul_vec8_kernel, dim3((unsigned)((total_vec + 255) / 256)), dim3(256), 0, s, (const bf16*)gate_up, inter, total_vec,
                                                                                  interleaved, (bf16*)out);
         MLC_LAUNCH_CHECK();
         return 0;
     }
     if (in_dtype == MLC_DTYPE_F32 && out_dtype == MLC_DTYPE_F32)
-        silu_mul_kernel<float, float><<<blocks, 256, 0, s>>>((const float*)gate_up, inter, total, interleaved, (float*)out);
+        launch_pdl(silu_mul_kernel<float, float>, dim3(blocks), dim3(256), 0, s, (const float*)gate_up, inter, total, interleaved, (float*)out);
     else if (in_dtype == MLC_DTYPE_F32 && out_dtype == MLC_DTYPE_BF16)
-        silu_mul_kernel<float, bf16><<<blocks, 256, 0, s>>>((const float*)gate_up, inter, total, interleaved, (bf16*)out);
+        launch_pdl(silu_mul_kernel<float, bf16>, dim3(blocks), dim3(256), 0, s, (const float*)gate_up, inter, total, interleaved, (bf16*)out);
     else if (in_dtype == MLC_DTYPE_BF16 && out_dtype == MLC_DTYPE_BF16)
-        silu_mul_kernel<bf16, bf16><<<blocks, 256, 0, s>>>((const bf16*)gate_up, inter, total, interleaved, (bf16*)out);
+        launch_pdl(silu_mul_kernel<bf16, bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)gate_up, inter, total, interleaved, (bf16*)out);
     else if (in_dtype == MLC_DTYPE_BF16 && out_dtype == MLC_DTYPE_F32)
-        silu_mul_kernel<bf16, float><<<blocks, 256, 0, s>>>((const bf16*)gate_up, inter, total, interleaved, (float*)out);
+        launch_pdl(silu_mul_kernel<bf16, float>, dim3(blocks), dim3(256), 0, s, (const bf16*)gate_up, inter, total, interleaved, (float*)out);
     else
         return MLC_ERR_BAD_DTYPE;
     MLC_LAUNCH_CHECK();

@@ -73,6 +73,8 @@ template <typename TX, typename TW, typename TY, int BM, int BN, int TM, int TN,
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restrict__ y, float* __restrict__ part,
                    int M, int N, int K) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     constexpr int XV = (BM * (LS_BK / 4) + THREADS - 1) / THREADS;       // 16-byte loads per thread and K step
     constexpr int WV = (BN * (LS_BK / 4) + THREADS - 1) / THREADS;
@@ -187,6 +189,8 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
 // y = the chunks' sums added in ascending order into a total that starts at zero.
 template <typename TY>
 __global__ void linear_simt_add_chunks_kernel(const float* __restrict__ part, TY* __restrict__ y, long long MN, int n_chunks) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= MN) return;
     float total = 0.0f;
@@ -452,13 +456,13 @@ static int launch_linear(const void* x, const void* w, void* y, float* scratch, 
         if (p.large || (M + 63) / 64 > 65535) {
             dim3 grid((N + 127) / 128, (M + 127) / 128);
             if (grid.y > 65535) return MLC_ERR_BAD_SIZE;
-            linear_simt_kernel<TX, TW, TY, 128, 128, 8, 8, false><<<grid, 256, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
+            launch_pdl(linear_simt_kernel<TX, TW, TY, 128, 128, 8, 8, false>, grid, dim3(256), 0, s, xp, wp, yp, nullptr, M, N, K);
         } else if (chunks) {
             dim3 grid((N + 63) / 64, (M + 63) / 64, n_chunks);
-            linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, true><<<grid, 64, 0, s>>>(xp, wp, yp, scratch, M, N, K);
+            launch_pdl(linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, true>, grid, dim3(64), 0, s, xp, wp, yp, scratch, M, N, K);
         } else {
             dim3 grid((N + 63) / 64, (M + 63) / 64);
-            linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, false><<<grid, 64, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
+            launch_pdl(linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, false>, grid, dim3(64), 0, s, xp, wp, yp, nullptr, M, N, K);
         }
     } else {
         if constexpr (sizeof(TX) == 4 && sizeof(TW) == 4) {
@@ -469,15 +473,15 @@ static int launch_linear(const void* x, const void* w, void* y, float* scratch, 
         chunks = tiles < 4 * n_sms && n_chunks > 1 && n_chunks <= 65535 && scratch != nullptr && scratch_floats >= n_chunks * MN;
         if (chunks) {
             dim3 grid(tiles, 1, n_chunks);
-            linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, true><<<grid, 128, 0, s>>>(xp, wp, yp, scratch, M, N, K);
+            launch_pdl(linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, true>, grid, dim3(128), 0, s, xp, wp, yp, scratch, M, N, K);
         } else {
             dim3 grid(tiles, 1);
-            linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, false><<<grid, 128, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
+            launch_pdl(linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, false>, grid, dim3(128), 0, s, xp, wp, yp, nullptr, M, N, K);
         }
     }
     MLC_LAUNCH_CHECK();
     if (chunks) {
-        linear_simt_add_chunks_kernel<TY><<<(unsigned)((MN + 255) / 256), 256, 0, s>>>(scratch, yp, MN, n_chunks);
+        launch_pdl(linear_simt_add_chunks_kernel<TY>, dim3((unsigned)((MN + 255) / 256)), dim3(256), 0, s, scratch, yp, MN, n_chunks);
         MLC_LAUNCH_CHECK();
     }
     return 0;

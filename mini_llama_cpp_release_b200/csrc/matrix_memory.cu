@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(1024)
 row_norm_gate_kernel(const float* __restrict__ o, int slices, long long slice_stride, const float* __restrict__ gate,
                      long long gate_stride, const float* __restrict__ gain, float eps, float out_scale, int inner,
                      T* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     __shared__ float scratch[32];
     const long long t = blockIdx.x;
     const float* src = o + t * inner;
@@ -121,6 +123,8 @@ struct ExpGateArgs {
 
 // Steps of one token per sequence: a thread per (sequence, head).
 __global__ void exp_gates_step_kernel(ExpGateArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= a.n_seqs * a.H) return;
     const int seq = idx / a.H, h = idx % a.H;
@@ -224,6 +228,8 @@ __global__ void __launch_bounds__(128)
 memory_finish_kernel(const float* __restrict__ o, int slices, long long slice_stride, const float* __restrict__ m,
                      const float* __restrict__ gate, long long gate_stride, const float* __restrict__ gain, float eps,
                      long long n_rows, int H, int vdim, T* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= n_rows) return;
     const int lane = threadIdx.x & 31;
@@ -273,7 +279,7 @@ static int launch_memory_finish(const float* o, int slices, long long slice_stri
     const unsigned blocks = (unsigned)((n_rows + 3) / 4);
     auto k = vdim <= 64 ? memory_finish_kernel<T, 2> : vdim <= 128 ? memory_finish_kernel<T, 4> : vdim <= 256 ? memory_finish_kernel<T, 8>
            : vdim <= 512 ? memory_finish_kernel<T, 16> : memory_finish_kernel<T, 32>;
-    k<<<blocks, 128, 0, s>>>(o, slices, slice_stride, m, gate, gate_stride, gain, eps, n_rows, H, vdim, out);
+    launch_pdl(k, dim3(blocks), dim3(128), 0, s, o, slices, slice_stride, m, gate, gate_stride, gain, eps, n_rows, H, vdim, out);
     MLC_LAUNCH_CHECK();
     return 0;
 }
@@ -289,7 +295,7 @@ static int launch_row_norm_gate(const float* o, int slices, long long slice_stri
     const int pieces = (items + threads - 1) / threads;
     auto k = vec ? (pieces <= 1 ? row_norm_gate_kernel<T, 4, 1> : pieces <= 2 ? row_norm_gate_kernel<T, 4, 2> : row_norm_gate_kernel<T, 4, 4>)
                  : (pieces <= 2 ? row_norm_gate_kernel<T, 1, 2> : row_norm_gate_kernel<T, 1, 16>);
-    k<<<n, threads, 0, s>>>(o, slices, slice_stride, gate, gate_stride, gain, eps, out_scale, inner, out);
+    launch_pdl(k, dim3(n), dim3(threads), 0, s, o, slices, slice_stride, gate, gate_stride, gain, eps, out_scale, inner, out);
     MLC_LAUNCH_CHECK();
     return 0;
 }
@@ -356,7 +362,7 @@ extern "C" int mlc_matrix_memory(const float* proj, long long proj_stride, int q
     float *decay = gates, *take = gates + per, *m = gates + 2 * per;
     const ExpGateArgs g{proj, proj_stride, i_col, f_col, i_bias, f_bias, cap, 1.0f / cap, state + (long long)H * (vdim + 1) * dim,
                         state_stride, slots, cu_seqlens, H, n_seqs, decay, take, m};
-    if (max_q_len <= 4) exp_gates_step_kernel<<<(n_seqs * H + 63) / 64, 64, 0, s>>>(g);
+    if (max_q_len <= 4) launch_pdl(exp_gates_step_kernel, dim3((n_seqs * H + 63) / 64), dim3(64), 0, s, g);
     else exp_gates_scan_kernel<<<dim3(H, n_seqs), EG_THREADS, 0, s>>>(g);
     MLC_LAUNCH_CHECK();
     GlaArgs a = {};

@@ -75,6 +75,8 @@ template <typename TX, int PL>
 __global__ void __launch_bounds__(128)
 moe_route_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, int n,
                  int E, int K, int top, int weighting, int* __restrict__ ids, float* __restrict__ weights) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ float part[4][16];
@@ -145,6 +147,8 @@ __global__ void __launch_bounds__(128)
 moe_route_scored_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ correction, int n,
                         int E, int K, int top, int G, int keep, int pair_groups, float scale, int* __restrict__ ids,
                         float* __restrict__ weights) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ float part[4][16];
@@ -272,6 +276,8 @@ __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ ids, const int* __restrict__ tokens, const int* __restrict__ table, float weight,
                 float* __restrict__ weights, int n_pairs, int top, int E, int tile, int max_rows, int* __restrict__ row_of,
                 int* __restrict__ src_tok, int* __restrict__ tile_expert) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     auto expert_of = [&](int p) { return table != nullptr ? table[(long long)tokens[p / top] * top + p % top] : ids[p]; };
     extern __shared__ int sh[];
     int* cnt = sh;                 // [32][E]
@@ -416,6 +422,8 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
 template <typename TI>
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ row_of, const float* __restrict__ weights,
                                    const TI* __restrict__ ident, int top, int d, float* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int t = blockIdx.x;
     for (int i = threadIdx.x; i < d; i += blockDim.x) {
         float acc = 0.0f;
@@ -473,6 +481,8 @@ __global__ void scaled_add_experts_kernel(float* __restrict__ x, const float* __
                                           const float* __restrict__ rows, const int* __restrict__ row_of,
                                           const float* __restrict__ weights, int top, const float* __restrict__ s2,
                                           long long total, int d) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
     if (idx >= total) return;
     const long long t = idx / d;
@@ -508,9 +518,9 @@ extern "C" int mlc_moe_route(const void* x, int x_dtype, const float* w, const f
     if (E <= 0 || E > 32 * ROUTE_MAX_PER_LANE || top <= 0 || top > 32 || top > E || (w != nullptr && K <= 0)) return MLC_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     if (w == nullptr || x_dtype == MLC_DTYPE_F32)
-        (E <= 32 ? moe_route_kernel<float, 1> : moe_route_kernel<float, ROUTE_MAX_PER_LANE>)<<<n, 128, 0, s>>>((const float*)x, w, bias, n, E, K, top, weighting, ids, weights);
+        launch_pdl(E <= 32 ? moe_route_kernel<float, 1> : moe_route_kernel<float, ROUTE_MAX_PER_LANE>, dim3(n), dim3(128), 0, s, (const float*)x, w, bias, n, E, K, top, weighting, ids, weights);
     else if (x_dtype == MLC_DTYPE_BF16)
-        (E <= 32 ? moe_route_kernel<bf16, 1> : moe_route_kernel<bf16, ROUTE_MAX_PER_LANE>)<<<n, 128, 0, s>>>((const bf16*)x, w, bias, n, E, K, top, weighting, ids, weights);
+        launch_pdl(E <= 32 ? moe_route_kernel<bf16, 1> : moe_route_kernel<bf16, ROUTE_MAX_PER_LANE>, dim3(n), dim3(128), 0, s, (const bf16*)x, w, bias, n, E, K, top, weighting, ids, weights);
     else
         return MLC_ERR_BAD_DTYPE;
     MLC_LAUNCH_CHECK();
@@ -527,7 +537,7 @@ extern "C" int mlc_moe_route_scored(const void* x, int x_dtype, const float* w, 
     if (G > 1 && (E % G != 0 || keep < 1)) return MLC_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
 #define MLC_ROUTE(TX, PL, SG) \
-    moe_route_scored_kernel<TX, PL, SG><<<n, 128, 0, s>>>((const TX*)x, w, correction, n, E, K, top, G, keep, pair_groups, scale, ids, weights)
+    launch_pdl(moe_route_scored_kernel<TX, PL, SG>, dim3(n), dim3(128), 0, s, (const TX*)x, w, correction, n, E, K, top, G, keep, pair_groups, scale, ids, weights)
 #define MLC_ROUTE_SIZES(TX, SG) do { if (E <= 32) MLC_ROUTE(TX, 1, SG); else MLC_ROUTE(TX, ROUTE_MAX_PER_LANE, SG); } while (0)
     if (x_dtype == MLC_DTYPE_F32) {
         if (sigmoid) MLC_ROUTE_SIZES(float, true); else MLC_ROUTE_SIZES(float, false);
@@ -549,7 +559,7 @@ static int launch_plan(const int* ids, const int* tokens, const int* table, floa
     // every expert's run, rounded up to whole tiles, must fit
     const long long most = (long long)n_pairs + (long long)(E < n_pairs ? E : n_pairs) * (tile - 1);     // only experts that were chosen have a run
     if ((long long)max_rows < most - most % tile) return MLC_ERR_BAD_SIZE;
-    moe_plan_kernel<<<1, 1024, 33 * E * sizeof(int), (cudaStream_t)stream>>>(ids, tokens, table, weight, weights, n_pairs, top, E, tile,
+    launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), 33 * E * sizeof(int), (cudaStream_t)stream, ids, tokens, table, weight, weights, n_pairs, top, E, tile,
                                                                             max_rows, row_of, src_tok, tile_expert);
     MLC_LAUNCH_CHECK();
     return 0;
@@ -615,9 +625,9 @@ extern "C" int mlc_moe_combine(const float* y, const int* row_of, const float* w
     if (n <= 0) return 0;
     if (top <= 0 || d <= 0) return MLC_ERR_BAD_SIZE;
     if (ident != nullptr && ident_dtype == MLC_DTYPE_BF16)
-        moe_combine_kernel<bf16><<<n, d >= 256 ? 256 : 64, 0, (cudaStream_t)stream>>>(y, row_of, weights, (const bf16*)ident, top, d, out);
+        launch_pdl(moe_combine_kernel<bf16>, dim3(n), dim3(d >= 256 ? 256 : 64), 0, (cudaStream_t)stream, y, row_of, weights, (const bf16*)ident, top, d, out);
     else
-        moe_combine_kernel<float><<<n, d >= 256 ? 256 : 64, 0, (cudaStream_t)stream>>>(y, row_of, weights, (const float*)ident, top, d, out);
+        launch_pdl(moe_combine_kernel<float>, dim3(n), dim3(d >= 256 ? 256 : 64), 0, (cudaStream_t)stream, y, row_of, weights, (const float*)ident, top, d, out);
     MLC_LAUNCH_CHECK();
     return 0;
 }
@@ -645,10 +655,10 @@ extern "C" int mlc_scaled_add_experts(float* x, const float* y1, int slices1, co
     if (d <= 0 || (y1 == nullptr ? slices1 != 0 : slices1 < 1) || top < 1) return MLC_ERR_BAD_SIZE;
     const long long total = n * d;
     if ((d & 3) == 0)
-        scaled_add_experts_kernel<4><<<(unsigned)((total / 4 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        launch_pdl(scaled_add_experts_kernel<4>, dim3((unsigned)((total / 4 + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, 
             x, y1, slices1, s1, rows, row_of, weights, top, s2, total, d);
     else
-        scaled_add_experts_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        launch_pdl(scaled_add_experts_kernel<1>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, 
             x, y1, slices1, s1, rows, row_of, weights, top, s2, total, d);
     MLC_LAUNCH_CHECK();
     return 0;

@@ -143,6 +143,8 @@ __global__ void conv_state_kernel(ConvArgs a) {
 
 // Every sequence brings one token (token b belongs to sequence b): output and state in one pass.
 __global__ void conv_step_kernel(ConvArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)a.n_seqs * a.C) return;
     const int token = (int)(idx / a.C), c = (int)(idx % a.C);
@@ -195,6 +197,8 @@ struct DeltaArgs {
 };
 
 __global__ void delta_prepare_kernel(DeltaArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (w >= (long long)a.n_tokens * a.H) return;
     const int lane = threadIdx.x & 31;
@@ -247,6 +251,8 @@ struct DeltaSmem {
 template <int NI>
 __global__ void __launch_bounds__(128)
 delta_rule_kernel(DeltaArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     static_assert(NI % 4 == 0, "rows per lane come in fours");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DeltaSmem<NI>* bufs = reinterpret_cast<DeltaSmem<NI>*>(smem_raw);
@@ -372,7 +378,7 @@ static cudaError_t launch_delta_rule(const DeltaArgs& a, dim3 grid, cudaStream_t
         if (e != cudaSuccess) return e;
         raised = true;
     }
-    delta_rule_kernel<NI><<<grid, 128, smem, s>>>(a);
+    launch_pdl(delta_rule_kernel<NI>, grid, dim3(128), smem, s, a);
     return cudaGetLastError();
 }
 
@@ -706,6 +712,8 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, int n_slices, 
                                      const float* __restrict__ gate, long long gate_stride,
                                      const float* __restrict__ w, float eps, long long n_rows, int H, int vdim,
                                      T* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= n_rows) return;
     const int lane = threadIdx.x & 31;
@@ -962,6 +970,8 @@ gates_scan_step_kernel(const float* __restrict__ u, const float* __restrict__ wr
                        const float* __restrict__ y, long long y_stride, const float* __restrict__ y_bias, float* state,
                        long long state_stride, const int* __restrict__ slots, int n_seqs, int W, int bw, float out_scale,
                        T* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     extern __shared__ float gs_smem[];
     float* us = gs_smem;                                  // [GS_SEQS][bw]
     float* part = us + GS_SEQS * bw;                      // [8 warps][GS_SEQS][2][32]
@@ -1037,7 +1047,7 @@ extern "C" int mlc_causal_conv(const float* x, long long x_stride, const float* 
     ConvArgs a{x, x_stride, w, bias, in_bias, state, state_stride, slots, cu_seqlens, tok_seq, out, out_stride, C, taps, act, n_tokens, n_seqs};
     cudaStream_t s = (cudaStream_t)stream;
     if (max_q_len == 1 && n_tokens == n_seqs) {
-        conv_step_kernel<<<(unsigned)(((long long)n_seqs * C + 255) / 256), 256, 0, s>>>(a);
+        launch_pdl(conv_step_kernel, dim3((unsigned)(((long long)n_seqs * C + 255) / 256)), dim3(256), 0, s, a);
         MLC_LAUNCH_CHECK();
         return 0;
     }
@@ -1080,7 +1090,7 @@ extern "C" int mlc_gated_delta_rule(const float* qkv, long long qkv_stride, int 
         else e = launch_delta_rule_group<16>(a, grid, s);
         return e == cudaSuccess ? 0 : (int)e;
     }
-    delta_prepare_kernel<<<(unsigned)(((long long)n_tokens * H + 7) / 8), 256, 0, s>>>(a);
+    launch_pdl(delta_prepare_kernel, dim3((unsigned)(((long long)n_tokens * H + 7) / 8)), dim3(256), 0, s, a);
     MLC_LAUNCH_CHECK();
     if (ni <= 4) e = launch_delta_rule<4>(a, grid, s);
     else if (ni <= 8) e = launch_delta_rule<8>(a, grid, s);
@@ -1101,9 +1111,9 @@ extern "C" int mlc_gated_rmsnorm(const float* o, int n_slices, const float* gate
     const unsigned blocks = (unsigned)((n_rows + 3) / 4);
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == MLC_DTYPE_F32)
-        gated_rmsnorm_kernel<float><<<blocks, 128, 0, s>>>(o, n_slices, slice_stride, gate, gate_stride, w, eps, n_rows, H, vdim, (float*)out);
+        launch_pdl(gated_rmsnorm_kernel<float>, dim3(blocks), dim3(128), 0, s, o, n_slices, slice_stride, gate, gate_stride, w, eps, n_rows, H, vdim, (float*)out);
     else if (out_dtype == MLC_DTYPE_BF16)
-        gated_rmsnorm_kernel<bf16><<<blocks, 128, 0, s>>>(o, n_slices, slice_stride, gate, gate_stride, w, eps, n_rows, H, vdim, (bf16*)out);
+        launch_pdl(gated_rmsnorm_kernel<bf16>, dim3(blocks), dim3(128), 0, s, o, n_slices, slice_stride, gate, gate_stride, w, eps, n_rows, H, vdim, (bf16*)out);
     else
         return MLC_ERR_BAD_DTYPE;
     MLC_LAUNCH_CHECK();
@@ -1166,10 +1176,10 @@ extern "C" int mlc_gates_scan_step(const float* u, const float* wr_t, const floa
     if (grid.y > 65535) return MLC_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     if (out_dtype == MLC_DTYPE_F32)
-        gates_scan_step_kernel<float><<<grid, 256, smem, s>>>(u, wr_t, wi_t, br, bi, lam, c, y, y_stride, y_bias, state, state_stride,
+        launch_pdl(gates_scan_step_kernel<float>, grid, dim3(256), smem, s, u, wr_t, wi_t, br, bi, lam, c, y, y_stride, y_bias, state, state_stride,
                                                               slots, n_seqs, W, bw, out_scale, (float*)out);
     else if (out_dtype == MLC_DTYPE_BF16)
-        gates_scan_step_kernel<bf16><<<grid, 256, smem, s>>>(u, wr_t, wi_t, br, bi, lam, c, y, y_stride, y_bias, state, state_stride,
+        launch_pdl(gates_scan_step_kernel<bf16>, grid, dim3(256), smem, s, u, wr_t, wi_t, br, bi, lam, c, y, y_stride, y_bias, state, state_stride,
                                                              slots, n_seqs, W, bw, out_scale, (bf16*)out);
     else
         return MLC_ERR_BAD_DTYPE;

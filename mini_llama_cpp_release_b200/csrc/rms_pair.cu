@@ -241,6 +241,8 @@ template <typename T, int VEC, int PIECES>
 __global__ void __launch_bounds__(128)
 diff_combine_kernel(const T* __restrict__ o, const float* __restrict__ gate, long long gate_stride, float lambda, float eps, float mult,
                     long long n_rows, int H, int vdim, int D, T* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= n_rows) return;
     const int lane = threadIdx.x & 31;
@@ -284,7 +286,7 @@ static int launch_diff_combine(const T* o, const float* gate, long long gate_str
     const bool vec = vdim >= 128 && (vdim & 3) == 0 && (D & 3) == 0 && ((((uintptr_t)o) | ((uintptr_t)out)) & 15) == 0;
     auto k = vec ? (vdim <= 128 ? diff_combine_kernel<T, 4, 1> : vdim <= 256 ? diff_combine_kernel<T, 4, 2> : diff_combine_kernel<T, 4, 4>)
                  : (vdim <= 64 ? diff_combine_kernel<T, 1, 2> : vdim <= 128 ? diff_combine_kernel<T, 1, 4> : diff_combine_kernel<T, 1, 16>);
-    k<<<(unsigned)((n_rows + 3) / 4), 128, 0, s>>>(o, gate, gate_stride, lambda, eps, mult, n_rows, H, vdim, D, out);
+    launch_pdl(k, dim3((unsigned)((n_rows + 3) / 4)), dim3(128), 0, s, o, gate, gate_stride, lambda, eps, mult, n_rows, H, vdim, D, out);
     MLC_LAUNCH_CHECK();
     return 0;
 }

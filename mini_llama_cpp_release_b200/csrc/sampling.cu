@@ -67,6 +67,8 @@ __device__ __forceinline__ MaxIdx block_argmax(MaxIdx v, MaxIdx* scratch) {
 }
 
 __global__ void argmax_kernel(const float* __restrict__ logits, int vocab, int* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     __shared__ MaxIdx scratch[32];
     const float* row = logits + (long long)blockIdx.x * vocab;
     MaxIdx best{-INFINITY, 0x7fffffff};
@@ -165,6 +167,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_temperature_kernel(const float* __restrict__ logits, int vocab, float temperature,
                           unsigned long long seed, const unsigned long long* __restrict__ seed_ptr, const int* __restrict__ seq_ids,
                           const int* __restrict__ positions, int* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     __shared__ float fscratch[32];
     __shared__ int first_thread;
     const float* row = logits + (long long)blockIdx.x * vocab;
@@ -267,6 +271,8 @@ __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_top_k_kernel(const float* __restrict__ logits, int vocab, float temperature, int top_k,
                     unsigned long long seed, const unsigned long long* __restrict__ seed_ptr, const int* __restrict__ seq_ids,
                     const int* __restrict__ positions, int* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     __shared__ unsigned int hist[256];
     __shared__ float cand_v[TOPK_MAX];
     __shared__ int cand_i[TOPK_MAX];
@@ -428,7 +434,7 @@ using namespace mlc;
 extern "C" int mlc_argmax(const float* logits, int rows, int vocab, int* out, void* stream) {
     if (rows <= 0) return 0;
     if (vocab <= 0) return MLC_ERR_BAD_SIZE;
-    argmax_kernel<<<rows, SAMPLE_THREADS, 0, (cudaStream_t)stream>>>(logits, vocab, out);
+    launch_pdl(argmax_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, (cudaStream_t)stream, logits, vocab, out);
     MLC_LAUNCH_CHECK();
     return 0;
 }
@@ -454,12 +460,12 @@ extern "C" int mlc_sample(const float* logits, int rows, int vocab, float temper
     if (vocab <= 0 || !(temperature > 0.0f) || top_k < 0 || top_k == 1) return MLC_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     if (top_k == 0) {
-        sample_temperature_kernel<<<rows, SAMPLE_THREADS, 0, s>>>(logits, vocab, temperature, seed, seed_ptr, seq_ids,
+        launch_pdl(sample_temperature_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, s, logits, vocab, temperature, seed, seed_ptr, seq_ids,
                                                                   positions, out);
     } else {
         const int k = top_k < vocab ? top_k : vocab;
         if (k > TOPK_MAX) return MLC_ERR_UNSUPPORTED;
-        sample_top_k_kernel<<<rows, SAMPLE_THREADS, 0, s>>>(logits, vocab, temperature, top_k, seed, seed_ptr, seq_ids,
+        launch_pdl(sample_top_k_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, s, logits, vocab, temperature, top_k, seed, seed_ptr, seq_ids,
                                                             positions, out);
     }
     MLC_LAUNCH_CHECK();

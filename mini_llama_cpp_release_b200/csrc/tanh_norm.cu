@@ -141,6 +141,8 @@ __device__ __forceinline__ float glu_one(float g, float u, int kind, float limit
 template <typename TIn, typename TOut>
 __global__ void glu_kernel(const TIn* __restrict__ gu, int inter, long long total, int interleaved, int kind, float limit,
                            float alpha, TOut* __restrict__ out) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const long long n = idx / inter;
@@ -156,6 +158,8 @@ __global__ void glu_kernel(const TIn* __restrict__ gu, int inter, long long tota
 template <typename T>
 __global__ void sigmoid_gate_kernel(T* __restrict__ o, const float* __restrict__ gate, long long gate_stride, int heads, int vdim,
                                     int D, long long total) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int width = heads * vdim;
@@ -214,13 +218,13 @@ extern "C" int mlc_glu(const void* gate_up, int in_dtype, int n, int inter, int 
     const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (in_dtype == MLC_DTYPE_F32 && out_dtype == MLC_DTYPE_F32)
-        glu_kernel<float, float><<<blocks, 256, 0, s>>>((const float*)gate_up, inter, total, interleaved, kind, limit, alpha, (float*)out);
+        launch_pdl(glu_kernel<float, float>, dim3(blocks), dim3(256), 0, s, (const float*)gate_up, inter, total, interleaved, kind, limit, alpha, (float*)out);
     else if (in_dtype == MLC_DTYPE_F32 && out_dtype == MLC_DTYPE_BF16)
-        glu_kernel<float, bf16><<<blocks, 256, 0, s>>>((const float*)gate_up, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
+        launch_pdl(glu_kernel<float, bf16>, dim3(blocks), dim3(256), 0, s, (const float*)gate_up, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
     else if (in_dtype == MLC_DTYPE_BF16 && out_dtype == MLC_DTYPE_BF16)
-        glu_kernel<bf16, bf16><<<blocks, 256, 0, s>>>((const bf16*)gate_up, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
+        launch_pdl(glu_kernel<bf16, bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)gate_up, inter, total, interleaved, kind, limit, alpha, (bf16*)out);
     else if (in_dtype == MLC_DTYPE_BF16 && out_dtype == MLC_DTYPE_F32)
-        glu_kernel<bf16, float><<<blocks, 256, 0, s>>>((const bf16*)gate_up, inter, total, interleaved, kind, limit, alpha, (float*)out);
+        launch_pdl(glu_kernel<bf16, float>, dim3(blocks), dim3(256), 0, s, (const bf16*)gate_up, inter, total, interleaved, kind, limit, alpha, (float*)out);
     else
         return MLC_ERR_BAD_DTYPE;
     MLC_LAUNCH_CHECK();
@@ -235,9 +239,9 @@ extern "C" int mlc_sigmoid_gate(void* o, int dtype, const float* gate, long long
     const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == MLC_DTYPE_F32)
-        sigmoid_gate_kernel<float><<<blocks, 256, 0, s>>>((float*)o, gate, gate_stride, heads, vdim, D, total);
+        launch_pdl(sigmoid_gate_kernel<float>, dim3(blocks), dim3(256), 0, s, (float*)o, gate, gate_stride, heads, vdim, D, total);
     else if (dtype == MLC_DTYPE_BF16)
-        sigmoid_gate_kernel<bf16><<<blocks, 256, 0, s>>>((bf16*)o, gate, gate_stride, heads, vdim, D, total);
+        launch_pdl(sigmoid_gate_kernel<bf16>, dim3(blocks), dim3(256), 0, s, (bf16*)o, gate, gate_stride, heads, vdim, D, total);
     else
         return MLC_ERR_BAD_DTYPE;
     MLC_LAUNCH_CHECK();
