@@ -214,10 +214,12 @@ class GQAttention(Part):
                                softcap=softcap)
 
 
-def choose_splits(step, q_heads: int, kv_heads: int, n_sms: int, tokens_per_block: int, keys_per_split: int = 256,
+def choose_splits(step, q_heads: int, kv_heads: int, n_sms: int, tokens_per_block: int, keys_per_split: int = 32,
                   max_splits: int = 32) -> int:
     """How many blocks share one row's key range: enough to fill the GPU when the step
-    has few rows and long sequences (decoding), one when the rows alone fill it."""
+    has few rows (decoding), one when the rows alone fill it.  A split of a single tile of 32 keys is worth its share of the
+    merging kernel.  B200, a request of 3 prompts of up to 100 tokens and 16 tokens each in float32: 30.7 ms, with splits of
+    256 keys (none, here) 34.8."""
     q_tiles = (step.max_q_len + tokens_per_block - 1) // tokens_per_block
     blocks = q_tiles * kv_heads * max(1, (q_heads // kv_heads + 15) // 16) * step.n_seqs
     if blocks >= 2 * n_sms:
