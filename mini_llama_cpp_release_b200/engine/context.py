@@ -165,13 +165,25 @@ class Context:
             page_tables=page_tables, slots_long=slots_dev.long() if self.cache.has_state else None,
         )
 
-    # A step of many tokens is some two hundred launches issued from Python; when its kernels are fast the host
+    # A step is some two hundred launches issued from Python; when its kernels are fast the host
     # becomes the limit.  A shape of step that comes again (the same numbers of tokens and sequences, the same
     # longest lengths: fixed-size prompts, a benchmark, chunks of a fixed size) is therefore captured into a CUDA
-    # graph the second time it is seen and replayed from then on; everything that may differ between two such
+    # graph the second time it is seen (below 64 tokens the eighth time: lengths of short prompts are many and each comes
+    # again soon) and replayed from then on; everything that may differ between two such
     # steps (tokens, positions, lengths, pages) lies in the description buffer the graph reads.
-    STEP_GRAPHS = 4                     # captured shapes kept
-    STEP_GRAPH_MIN_TOKENS = 64          # smaller steps are cheap to issue
+    # A capture costs a step several times over (a run to warm up, the collector, two synchronisations), so it has to be worth it:
+    #   - a step of more tokens than STEP_GRAPH_MAX_TOKENS is not captured: its kernels take longer than issuing them does;
+    #   - a captured shape gives way to another only when it was not used for STEP_GRAPH_IDLE steps: more shapes in turn than
+    #     are kept would otherwise be captured at every single step.
+    # Sixteen ragged prompts of up to 2,048 tokens (1.5B sizes), whose pieces take turns in shape, B200: 159 ms a request with
+    # captures at nearly every step, 94 without.
+    STEP_GRAPHS = 8                     # captured shapes kept
+    STEP_GRAPH_MAX_TOKENS = 4096
+    STEP_GRAPH_IDLE = 64
+
+    @staticmethod
+    def _sights_to_capture(n_tokens: int) -> int:
+        return 2 if n_tokens >= 64 else 8
 
     def forward_batch(self, batch: MiniBatch) -> torch.Tensor:
         """Run the batch's tokens; returns float32 logits [number of wanted places, vocab], in
@@ -207,7 +219,7 @@ class Context:
         dev = self.model.runtime.device
         with torch.cuda.device(dev):
             n_new = sum(len(c.tokens) for c in batch.chunks)
-            if self.use_graphs and n_new >= self.STEP_GRAPH_MIN_TOKENS:
+            if self.use_graphs and n_new <= self.STEP_GRAPH_MAX_TOKENS:
                 logits = self._forward_maybe_replayed(batch)
             else:
                 step = self.describe(batch)
@@ -226,18 +238,21 @@ class Context:
         layout = self._describe_host(batch)
         key = self._step_key(layout)
         entry = graphs.get(key)
+        self._graph_clock = now = getattr(self, "_graph_clock", 0) + 1
         if entry is not None:
+            entry["used"] = now
             self._upload(layout, into=entry["dev"])
             entry["graph"].replay()
             graphs[key] = graphs.pop(key)                                     # most recently used last
             return entry["logits"].clone()
-        seen[key] = seen.get(key, 0) + 1
+        seen[key] = seen.pop(key, 0) + 1
         if len(seen) > 64:
             seen.pop(next(iter(seen)))
         own = self._upload(layout)
-        if seen[key] < 2:
+        room = len(graphs) < self.STEP_GRAPHS or now - next(iter(graphs.values()))["used"] > self.STEP_GRAPH_IDLE
+        if seen[key] < self._sights_to_capture(layout["n_tokens"]) or not room:
             return self.model.forward(self._step_over(own, layout), self.cache)
-        # second time: run it once more eagerly on a side stream (what capture needs), then capture and replay
+        # worth a capture: run it once more eagerly on a side stream (what capture needs), then capture and replay
         stream = torch.cuda.Stream(device=dev)
         stream.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(stream):
@@ -253,7 +268,7 @@ class Context:
         torch.cuda.synchronize(dev)
         while len(graphs) >= self.STEP_GRAPHS:
             graphs.pop(next(iter(graphs)))
-        graphs[key] = dict(graph=graph, dev=own, logits=logits)
+        graphs[key] = dict(graph=graph, dev=own, logits=logits, used=now)
         graph.replay()
         return logits.clone()
 
