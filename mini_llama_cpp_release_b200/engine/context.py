@@ -172,13 +172,14 @@ class Context:
     # again soon) and replayed from then on; everything that may differ between two such
     # steps (tokens, positions, lengths, pages) lies in the description buffer the graph reads.
     # A capture costs a step several times over (a run to warm up, the collector, two synchronisations), so it has to be worth it:
-    #   - a step of more tokens than STEP_GRAPH_MAX_TOKENS is not captured: its kernels take longer than issuing them does;
+    #   - a step of more tokens than STEP_GRAPH_MAX_TOKENS is not captured: its kernels take longer than issuing
+    #     them does (8,191 tokens at the 0.5B sizes still gain 1 %: 12.02 ms replayed, 12.10 issued);
     #   - a captured shape gives way to another only when it was not used for STEP_GRAPH_IDLE steps: more shapes in turn than
     #     are kept would otherwise be captured at every single step.
     # Sixteen ragged prompts of up to 2,048 tokens (1.5B sizes), whose pieces take turns in shape, B200: 159 ms a request with
     # captures at nearly every step, 94 without.
     STEP_GRAPHS = 8                     # captured shapes kept
-    STEP_GRAPH_MAX_TOKENS = 4096
+    STEP_GRAPH_MAX_TOKENS = 8192
     STEP_GRAPH_IDLE = 64
 
     @staticmethod
