@@ -14,7 +14,8 @@
 // What bounds it: the multiply-adds (per chunk and head 2 · 64 · dim · vdim for the state and the queries' product with it,
 // 64 · 64 · (dim · column tiles + vdim) inside the chunk), on tiles of 64 tokens x 64 columns or 128 rows x 64 columns, 8 x 4 or
 // 8 x 8 outputs per thread.  The walk is a chain 64 times as long on a fraction of the GPU.  B200, three prompts of 1,500, 638 and
-// 902 tokens, 6 heads of 128 x 257: 342 us (states 79, scan 23, outputs 240), the walk 1,665 us.
+// 902 tokens, 6 heads of 128 x 257: 299 us (states 79, scan 23, outputs 197; 240 with keys, values and products side by side in shared
+// memory, two blocks an SM), the walk 1,665 us.
 #include "common.cuh"
 #include "linear_attention.cuh"
 
@@ -191,15 +192,19 @@ __device__ __forceinline__ void gc_transpose(float* dst, int n, int width, F val
 }
 
 // grid: (column tiles, heads, chunks of the longest sequence x sequences).  A thread: 8 tokens (two fours) x 4 neighbours.
+// One region of shared memory holds first S before the chunk, then the keys, then the weighted products of queries and keys
+// and the values: three blocks of dim 128 share an SM, and one's loads hide behind another's products.
+__host__ __device__ constexpr int gc_region_floats(int dim) { return (dim > 2 * GC_TOKENS ? dim : 2 * GC_TOKENS) * GC_P; }
+
 __global__ void __launch_bounds__(GC_THREADS)
 gla_chunk_outputs_kernel(GcArgs g, int max_chunks) {
     extern __shared__ __align__(16) float gc_smem[];
     const GlaArgs& a = g.a;
-    float* const qT = gc_smem;                         // [dim][GC_P]
-    float* const kT = qT + a.dim * GC_P;               // [dim][GC_P] keys, then S [dim][columns]
-    float* const PT = kT + a.dim * GC_P;               // [token j][GC_P tokens i]
-    float* const vs = PT + GC_TOKENS * GC_P;           // [token][GC_P columns]
-    float* const as = vs + GC_TOKENS * GC_P;           // [64] decays
+    float* const region = gc_smem;                     // S [dim][columns], keys [dim][tokens], then the two below
+    float* const PT = region;                          // [token j][GC_P tokens i]
+    float* const vs = region + GC_TOKENS * GC_P;       // [token][GC_P columns]
+    float* const qT = region + gc_region_floats(a.dim);        // [dim][GC_P]
+    float* const as = qT + a.dim * GC_P;               // [64] decays
     float* const Ds = as + GC_TOKENS;                  // [64] decays from the chunk's first token to token i
     const int head = blockIdx.y, seq = blockIdx.z / max_chunks, c = blockIdx.z % max_chunks;
     const int t0 = a.cu_seqlens[seq], t1 = a.cu_seqlens[seq + 1];
@@ -210,25 +215,15 @@ gla_chunk_outputs_kernel(GcArgs g, int max_chunks) {
     if (tid < GC_TOKENS) as[tid] = tid < n ? gc_decay(a, c0 + tid, head) : 1.0f;
     const float* qp = a.qk + a.q_col + (head / a.qk_share) * a.dim + (long long)c0 * a.qk_stride;
     const float* kp = a.qk + a.k_col + (head / a.qk_share) * a.dim + (long long)c0 * a.qk_stride;
+    const float* sp = g.states + ((long long)(gc_first(t0, seq) + c) * a.H + head) * a.vdim * a.dim + (long long)col0 * a.dim;
     gc_transpose(qT, n, a.dim, [&](int t, int d) { return qp[(long long)t * a.qk_stride + d] * a.q_scale; });
-    gc_transpose(kT, n, a.dim, [&](int t, int d) { return kp[(long long)t * a.qk_stride + d]; });
-    gc_stage<GC_TOKENS * GC_COLS>([&](int idx) { return idx / GC_COLS < n ? gc_value(a, c0 + idx / GC_COLS, head, col0 + idx % GC_COLS) : 0.0f; },
-                                  [&](int idx, float v) { vs[idx / GC_COLS * GC_P + idx % GC_COLS] = v; });
+    gc_transpose(region, cols, a.dim, [&](int t, int d) { return sp[(long long)t * a.dim + d]; });
     __syncthreads();
-    // the decays W_ij, j down the rows of PT (zero above the diagonal); thread j < 64 walks i
     if (tid < GC_TOKENS) {
         float w = 1.0f;
-#pragma unroll 8
-        for (int i = 0; i < GC_TOKENS; ++i) {
-            w = i > tid ? w * as[i] : w;
-            PT[tid * GC_P + i] = i >= tid ? w : 0.0f;
-        }
-    } else {
-        const int i = tid - GC_TOKENS;
-        float w = 1.0f;
 #pragma unroll 16
-        for (int l = 0; l < GC_TOKENS; ++l) w *= l <= i ? as[l] : 1.0f;
-        Ds[i] = w;
+        for (int l = 0; l < GC_TOKENS; ++l) w *= l <= tid ? as[l] : 1.0f;
+        Ds[tid] = w;
     }
     auto product = [&](float (&acc)[8][4], const float* A, const float* B, int depth) {      // acc[i][j] += sum_d A[d][i] B[d][j]
 #pragma unroll 4
@@ -246,31 +241,52 @@ gla_chunk_outputs_kernel(GcArgs g, int max_chunks) {
         }
     };
     auto token_of = [&](int i) { return ty * 4 + 32 * (i >> 2) + (i & 3); };
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-    product(acc, qT, kT, a.dim);                       // q_i · k_j
-    __syncthreads();                                   // the keys have been read, W is there
-    const float* sp = g.states + ((long long)(gc_first(t0, seq) + c) * a.H + head) * a.vdim * a.dim + (long long)col0 * a.dim;
-    gc_transpose(kT, cols, a.dim, [&](int t, int d) { return sp[(long long)t * a.dim + d]; });      // S before the chunk, [dim][columns]
+    float out[8][4], qk[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float* at = PT + (tx * 4 + j) * GC_P + token_of(i);
-            // a token that sees no key of the chunk's later tokens gets a zero whatever their product is
-            *at = *at != 0.0f ? *at * acc[i][j] : 0.0f;
-            acc[i][j] = 0.0f;
-        }
-    __syncthreads();
-    product(acc, qT, kT, a.dim);                       // S_beforeᵀ q_i
+        for (int j = 0; j < 4; ++j) out[i][j] = qk[i][j] = 0.0f;
+    product(out, qT, region, a.dim);                   // S_beforeᵀ q_i
+    __syncthreads();                                   // S has been read, the decays are there
+    gc_transpose(region, n, a.dim, [&](int t, int d) { return kp[(long long)t * a.qk_stride + d]; });
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float D = Ds[token_of(i)];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] *= D;
+        for (int j = 0; j < 4; ++j) out[i][j] *= D;
     }
-    product(acc, PT, vs, n);
+    __syncthreads();
+    product(qk, qT, region, a.dim);                    // q_i · k_j
+    // times the decays W_ij: per column the product from the column's next token to the thread's first, then on token by token;
+    // a token that does not see the other gets a zero whatever their product is
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int i0 = token_of(4 * half);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int col = tx * 4 + j;
+            float w = 1.0f;
+#pragma unroll 4
+            for (int l = col + 1; l < i0; ++l) w *= as[l];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (i0 + i > col) w *= as[i0 + i];
+                const bool sees = i0 + i >= col && w != 0.0f;
+                qk[4 * half + i][j] = sees ? w * qk[4 * half + i][j] : 0.0f;
+            }
+        }
+    }
+    __syncthreads();                                   // the keys have been read
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(PT + (tx * 4 + j) * GC_P + token_of(4 * half)) =
+                make_float4(qk[4 * half][j], qk[4 * half + 1][j], qk[4 * half + 2][j], qk[4 * half + 3][j]);
+    gc_stage<GC_TOKENS * GC_COLS>([&](int idx) { return idx / GC_COLS < n ? gc_value(a, c0 + idx / GC_COLS, head, col0 + idx % GC_COLS) : 0.0f; },
+                                  [&](int idx, float v) { vs[idx / GC_COLS * GC_P + idx % GC_COLS] = v; });
+    __syncthreads();
+    product(out, PT, vs, n);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int t = token_of(i);
@@ -278,7 +294,7 @@ gla_chunk_outputs_kernel(GcArgs g, int max_chunks) {
         float* o = a.out + (long long)(c0 + t) * a.H * a.vdim + (long long)head * a.vdim + col0 + tx * 4;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (tx * 4 + j < cols) o[j] = acc[i][j];
+            if (tx * 4 + j < cols) o[j] = out[i][j];
     }
 }
 
@@ -300,10 +316,10 @@ int gla_chunks(GlaArgs a, int n_seqs, int n_tokens, int max_q_len, float* scratc
     MLC_LAUNCH_CHECK();
     gla_chunk_scan_kernel<<<dim3((unsigned)((per_seq + 255) / 256), n_seqs), 256, 0, s>>>(g, per_seq);
     MLC_LAUNCH_CHECK();
-    const size_t smem = ((size_t)(2 * a.dim + 2 * GC_TOKENS) * GC_P + 2 * GC_TOKENS) * sizeof(float);
+    const size_t smem = ((size_t)gc_region_floats(a.dim) + a.dim * GC_P + 2 * GC_TOKENS) * sizeof(float);
     static size_t allowed = 48 * 1024;
     if (smem > allowed) {
-        constexpr size_t most = ((size_t)(2 * 256 + 2 * GC_TOKENS) * GC_P + 2 * GC_TOKENS) * sizeof(float);
+        constexpr size_t most = ((size_t)gc_region_floats(256) + 256 * GC_P + 2 * GC_TOKENS) * sizeof(float);
         static_assert(most <= 227 * 1024, "shared memory of a block");
         cudaError_t e = cudaFuncSetAttribute(gla_chunk_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e != cudaSuccess) return (int)e;
