@@ -7,7 +7,7 @@
 // gathered on the way (row r of a run is row src_tok[r] of x), which saves the kernel that would lay them out.
 //
 // What bounds it: the chosen experts' weights.  B200, 8 tokens of which each takes one of 8 experts of 1,536 x 4,480 (5.3 chosen
-// on average), in brackets tiles of 128 tokens: gate/up 33 us = 4.4 TB/s (33 and 3 for the gather), down 22 us = 3.3 TB/s (57:
+// on average), in brackets tiles of 128 tokens: gate/up 30 us = 4.8 TB/s (33 and 3 for the gather), down 22 us = 3.3 TB/s (57:
 // its 64 tiles left most SMs idle).
 #include "gemm_few.cuh"
 
@@ -26,8 +26,10 @@ struct GroupedFewArgs {
     float glu_limit, glu_alpha;
 };
 
+// Two units a warp and two tiles at a time: up to 12 warps' rings leave room for a second block on an SM, whose loads are
+// under way while the first block's sums meet; the registers are held down to allow it.
 template <int NT, int UW, int RT, bool SILU>
-__global__ void __launch_bounds__(32 * FEW_MAX_WARPS, 1)
+__global__ void __launch_bounds__(UW == 2 && NT == 1 ? 384 : 32 * FEW_MAX_WARPS, UW == 2 && NT == 1 ? 2 : 1)
 gemm_few_grouped_kernel(GroupedFewArgs g) {
     constexpr int TOKENS = 8 * NT;
     constexpr int TILE_U4 = UW * 4 * 32;
@@ -229,7 +231,10 @@ extern "C" int mlc_gemm_few_grouped(const void* x, const int* src_tok, const voi
     if (glu_kind < 0 || glu_kind > 2 || (glu_kind == 2 && !(glu_limit > 0.0f))) return MLC_ERR_UNSUPPORTED;
     GroupedFewArgs g{(const bf16*)x, src_tok, (const bf16*)w, tile_group, out, out_dtype, groups, group_rows, n_out, K,
                      (n_out + FEW_ROWS - 1) / FEW_ROWS, glu_kind, glu_limit, glu_alpha};
-    const int units = K / FEW_UNIT, uw = (units + FEW_MAX_WARPS - 1) / FEW_MAX_WARPS, warps = (units + uw - 1) / uw;
+    const int units = K / FEW_UNIT;
+    int uw = (units + FEW_MAX_WARPS - 1) / FEW_MAX_WARPS;
+    if (uw == 2 && group_rows <= 8 && units > 24) uw = 3;            // (that instance has 12 warps at most)
+    const int warps = (units + uw - 1) / uw;
     cudaStream_t s = (cudaStream_t)stream;
     if (group_rows <= 8) return silu ? launch_grouped_shape<1, true>(g, warps, uw, n_sms, s) : launch_grouped_shape<1, false>(g, warps, uw, n_sms, s);
     return silu ? launch_grouped_shape<2, true>(g, warps, uw, n_sms, s) : launch_grouped_shape<2, false>(g, warps, uw, n_sms, s);

