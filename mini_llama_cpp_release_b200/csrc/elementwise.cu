@@ -614,7 +614,7 @@ __global__ void qk_norm_rope_cache_kernel(const float* __restrict__ proj, long l
             f_k = 1.0f / sqrtf(block_sum(ss, scratch) / (float)(k_units * dim) + eps);
         }
     }
-    for (int head = warp; head < n_heads; head += n_warps) {
+    for (int head = blockIdx.y * n_warps + warp; head < n_heads; head += gridDim.y * n_warps) {
         if (head < q_heads + k_units) {
             const bool is_q = head < q_heads;
             const int h = is_q ? head : head - q_heads;
@@ -782,12 +782,15 @@ extern "C" int mlc_qk_norm_rope_cache(const float* proj, long long stride, int q
     cudaStream_t s = (cudaStream_t)stream;
     const int heads = q_heads + (maps + 1) * kv_heads_in_row;
     const int threads = 32 * (heads < 8 ? heads : 8);
+    // a few tokens: a warp per head, so that no warp takes heads one after the other (4 tokens, 18 heads, three a warp, B200:
+    // 6.8 us; the gain is told at gates_scan_step_kernel, with which it was measured)
+    const dim3 grid(n, n < 64 ? (heads + 7) / 8 : 1);
     if (dtype == MLC_DTYPE_F32)
-        launch_pdl(qk_norm_rope_cache_kernel<float>, dim3(n), dim3(threads), 0, s, proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
+        launch_pdl(qk_norm_rope_cache_kernel<float>, grid, dim3(threads), 0, s, proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
                                                                tok_seq, (const float2*)rope_table, rope_positions, rot_dims, q_heads,
                                                                kv_heads_in_row, dim, vdim, D, v_scale, (float*)q_out, c, opt);
     else if (dtype == MLC_DTYPE_BF16)
-        launch_pdl(qk_norm_rope_cache_kernel<bf16>, dim3(n), dim3(threads), 0, s, proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
+        launch_pdl(qk_norm_rope_cache_kernel<bf16>, grid, dim3(threads), 0, s, proj, stride, q_col, k_col, v_col, q_gain, k_gain, eps, positions,
                                                               tok_seq, (const float2*)rope_table, rope_positions, rot_dims, q_heads,
                                                               kv_heads_in_row, dim, vdim, D, v_scale, (bf16*)q_out, c, opt);
     else
