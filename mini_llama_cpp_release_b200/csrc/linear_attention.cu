@@ -207,15 +207,15 @@ gla_walk_kernel(GlaArgs a) {
 
 
 // Steps of one token per sequence: a warp per (sequence, head, eight columns), a column's rows spread over its lanes, so that
-// the state streams through in whole lines and nothing but a warp's sum stands between its arrival and the output.  The
-// state was written by the step before, so its loads do not wait for the kernel before this one.  Bound by the state's bytes:
-// B200, 8 sequences, 6 heads of 128 x 257 (12.6 MB in and out), 5.5 us, the walk 32 us.
+// the state streams through in whole lines and nothing but a warp's sum stands between its arrival and the output.  Bound by
+// the state's bytes: B200, 8 sequences, 6 heads of 128 x 257 (12.6 MB in and out), 5.5 us, the walk 32 us.
 constexpr int GLS_COLS = 8;
 
 template <int RPL, bool SILU>          // rows of a column per lane: dim <= 32 * RPL
 __global__ void __launch_bounds__(128)
 gla_step_kernel(GlaArgs a) {
     grid_launch_dependents();
+    grid_dependency_wait();                            // for the state too: the step before may be the kernel before
     const int lane = threadIdx.x & 31;
     const int col0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * GLS_COLS, head = blockIdx.y, seq = blockIdx.z;
     const int dim = a.dim, vdim = a.vdim;
@@ -229,7 +229,6 @@ gla_step_kernel(GlaArgs a) {
             const int row = lane + 32 * i;
             S[c][i] = (col0 + c < vdim && row < dim) ? S_base[(long long)(col0 + c) * dim + row] : 0.0f;
         }
-    grid_dependency_wait();
     for (int t = a.cu_seqlens[seq], t1 = a.cu_seqlens[seq + 1]; t < t1; ++t) {
         const float* qk = a.qk + (long long)t * a.qk_stride + (head / a.qk_share) * dim;
         const float one = a.const_decay != nullptr ? a.const_decay[head] : a.head_decay != nullptr ? a.head_decay[(long long)t * a.H + head] : 1.0f;

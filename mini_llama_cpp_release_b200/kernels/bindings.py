@@ -1662,7 +1662,9 @@ def gemm_few_grouped_takes(n_pairs: int, n_out: int, k: int) -> bool:
 def gemm_few_grouped(x: torch.Tensor, src_tok: Optional[torch.Tensor], w: torch.Tensor, tile_group: torch.Tensor, group_rows: int,
                      out: torch.Tensor, epilogue: int, n_sms: int, glu=None) -> None:
     """out[row] = w[tile_group[row // group_rows]] x[src_tok[row]] (x[row] without src_tok) for the runs of a `moe_plan` with
-    tiles of `group_rows` <= 16 rows; w bfloat16 [E, N, K], epilogue EPI_STORE or EPI_SILU_MUL."""
+    tiles of `group_rows` <= 16 rows; w bfloat16 [E, N, K], epilogue EPI_STORE or EPI_SILU_MUL.  Without src_tok the plan is read
+    ahead of the wait for the kernel before: another kernel has to stand between the plan's and this one (a product with
+    src_tok, as a rule)."""
     require_cuda(x, src_tok, w, tile_group, out)
     E, n_out, K = w.shape
     groups = tile_group.numel()
