@@ -227,6 +227,87 @@ __global__ void delta_prepare_kernel(DeltaArgs a) {
     }
 }
 
+// Steps of one token per sequence: both kernels in one.  A block owns 32 columns of a (sequence, head), a lane one of them, a
+// warp a quarter of the rows, so that a row's columns arrive as one line.  The five numbers are formed by every block for
+// itself, from rows it reads anyway.  Bound by the chain: one trip for the state, q, k and the gates, two exchanges over the
+// warps.  B200, 48 tokens of 4
+// Mepolix prompts: 17.9 ms with the two kernels, 17.5 with one.
+template <int NR>                       // rows of S per warp: dim <= 4 * NR
+__global__ void __launch_bounds__(128)
+delta_step_kernel(DeltaArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();                            // for the state too: the step before may be the kernel before
+    __shared__ float ks[4 * NR], qs[4 * NR], sums[4][3], dots[4][2][32];
+    const int seq = blockIdx.z, head = blockIdx.y;
+    const int kv_head = head / (a.H / a.G);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col = blockIdx.x * DR_COLS + lane;
+    const bool ok = col < a.vdim;
+    float* S_glob = a.state + (long long)a.slots[seq] * a.state_stride + (long long)head * a.dim * a.vdim + col;
+    const float rate = expf(a.A_log[head]), bias = a.dt_bias[head];
+    float S[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = warp * NR + i;
+        S[i] = ok && r < a.dim ? S_glob[(long long)r * a.vdim] : 0.0f;
+    }
+    for (int token = a.cu_seqlens[seq], end = a.cu_seqlens[seq + 1]; token < end; ++token) {
+        const float* row = a.qkv + (long long)token * a.qkv_stride;
+        const float* gr = a.gates + (long long)token * a.gates_stride;
+        const float v = ok ? row[a.v_col + head * a.vdim + col] : 0.0f;
+        const float z = gr[a.a_col + head], zb = gr[a.b_col + head];
+        float sk = 0.0f, sq = 0.0f, skq = 0.0f;
+        for (int i = tid; i < 4 * NR; i += 128) {
+            const float kv = i < a.dim ? row[a.k_col + kv_head * a.dim + i] : 0.0f, qv = i < a.dim ? row[a.q_col + kv_head * a.dim + i] : 0.0f;
+            ks[i] = kv;
+            qs[i] = qv;
+            sk = fmaf(kv, kv, sk);
+            sq = fmaf(qv, qv, sq);
+            skq = fmaf(kv, qv, skq);
+        }
+        sk = warp_sum(sk);
+        sq = warp_sum(sq);
+        skq = warp_sum(skq);
+        if (lane == 0) {
+            sums[warp][0] = sk;
+            sums[warp][1] = sq;
+            sums[warp][2] = skq;
+        }
+        const float g = expf(-rate * softplus_f(z + bias)), beta = sigmoid_f(zb);
+        __syncthreads();
+        const float fk = 1.0f / sqrtf(sums[0][0] + sums[1][0] + sums[2][0] + sums[3][0] + 1e-6f);
+        const float fq = a.q_scale / sqrtf(sums[0][1] + sums[1][1] + sums[2][1] + sums[3][1] + 1e-6f);
+        const float kq = (sums[0][2] + sums[1][2] + sums[2][2] + sums[3][2]) * fk * fq;
+        float dk = 0.0f, dq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            dk = fmaf(S[i], ks[warp * NR + i], dk);
+            dq = fmaf(S[i], qs[warp * NR + i], dq);
+        }
+        dots[warp][0][lane] = dk;
+        dots[warp][1][lane] = dq;
+        __syncthreads();
+        dk = fk * (dots[0][0][lane] + dots[1][0][lane] + dots[2][0][lane] + dots[3][0][lane]);
+        dq = fq * (dots[0][1][lane] + dots[1][1][lane] + dots[2][1][lane] + dots[3][1][lane]);
+        const float u = beta * (v - g * dk);
+        if (warp == 0 && ok) a.out[(long long)token * a.H * a.vdim + head * a.vdim + col] = fmaf(g, dq, kq * u);
+        const float fu = fk * u;
+#pragma unroll
+        for (int i = 0; i < NR; ++i) S[i] = fmaf(g, S[i], ks[warp * NR + i] * fu);
+        __syncthreads();                               // the rows in shared memory have been read
+    }
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = warp * NR + i;
+        if (ok && r < a.dim) S_glob[(long long)r * a.vdim] = S[i];
+    }
+}
+
+static cudaError_t launch_delta_step(const DeltaArgs& a, dim3 grid, cudaStream_t s) {
+    auto k = a.dim <= 32 ? delta_step_kernel<8> : a.dim <= 64 ? delta_step_kernel<16> : a.dim <= 128 ? delta_step_kernel<32> : delta_step_kernel<64>;
+    return launch_pdl(k, grid, dim3(128), 0, s, a);
+}
+
 __device__ __forceinline__ void cp_async_f32x4(float* smem, const float* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
@@ -1106,6 +1187,10 @@ extern "C" int mlc_gated_delta_rule(const float* qkv, long long qkv_stride, int 
         else if (ni <= 8) e = launch_delta_rule_group<8>(a, grid, s);
         else if (ni <= 12) e = launch_delta_rule_group<12>(a, grid, s);
         else e = launch_delta_rule_group<16>(a, grid, s);
+        return e == cudaSuccess ? 0 : (int)e;
+    }
+    if (max_q_len == 1) {
+        e = launch_delta_step(a, grid, s);
         return e == cudaSuccess ? 0 : (int)e;
     }
     launch_pdl(delta_prepare_kernel, dim3((unsigned)(((long long)n_tokens * H + 7) / 8)), dim3(256), 0, s, a);
