@@ -286,7 +286,46 @@ gla_chunk_outputs_kernel(GcArgs g, int max_chunks) {
     gc_stage<GC_TOKENS * GC_COLS>([&](int idx) { return idx / GC_COLS < n ? gc_value(a, c0 + idx / GC_COLS, head, col0 + idx % GC_COLS) : 0.0f; },
                                   [&](int idx, float v) { vs[idx / GC_COLS * GC_P + idx % GC_COLS] = v; });
     __syncthreads();
-    product(out, PT, vs, n);
+    // The weighted products times the values, each token over the tokens up to itself: half the work, and a value that is not a
+    // number reaches no token before its own.
+    auto add = [&](int first, const float4& x, const float4& y) {
+        const float xi[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            out[first + i][0] = fmaf(xi[i], y.x, out[first + i][0]);
+            out[first + i][1] = fmaf(xi[i], y.y, out[first + i][1]);
+            out[first + i][2] = fmaf(xi[i], y.z, out[first + i][2]);
+            out[first + i][3] = fmaf(xi[i], y.w, out[first + i][3]);
+        }
+    };
+    const float* const pt = PT + ty * 4;
+    const float* const vt = vs + tx * 4;
+    const int full0 = min(n, ty * 4), full1 = min(n, ty * 4 + 32);
+#pragma unroll 4
+    for (int j = 0; j < full0; ++j) {
+        const float4 y = *reinterpret_cast<const float4*>(vt + j * GC_P);
+        add(0, *reinterpret_cast<const float4*>(pt + j * GC_P), y);
+        add(4, *reinterpret_cast<const float4*>(pt + j * GC_P + 32), y);
+    }
+#pragma unroll 4
+    for (int j = full0; j < full1; ++j)
+        add(4, *reinterpret_cast<const float4*>(pt + j * GC_P + 32), *reinterpret_cast<const float4*>(vt + j * GC_P));
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {                  // the four tokens among themselves
+            const int j = ty * 4 + 32 * half + u;
+            const float4 y = *reinterpret_cast<const float4*>(vt + j * GC_P);
+#pragma unroll
+            for (int i = u; i < 4; ++i) {
+                const float x = PT[j * GC_P + ty * 4 + 32 * half + i];
+                float (&o)[4] = out[4 * half + i];
+                o[0] = fmaf(x, y.x, o[0]);
+                o[1] = fmaf(x, y.y, o[1]);
+                o[2] = fmaf(x, y.z, o[2]);
+                o[3] = fmaf(x, y.w, o[3]);
+            }
+        }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int t = token_of(i);

@@ -94,3 +94,19 @@ def test_state_space_groups(lens):
     a, b, sa, sb = _both(lens, inner + H + n_conv, inner * N, inner, run)
     _close(a, b, TOL)
     _close(sa, sb, TOL)
+
+
+def test_a_value_that_is_not_a_number_reaches_no_earlier_token():
+    H, dim, vdim, n, bad = 2, 32, 40, 100, 70
+    x = torch.randn(n, 2 * H * dim + 2 * H * vdim, generator=torch.Generator().manual_seed(1)).to(DEV)
+    decay, gain = torch.tensor([0.9, 0.99], device=DEV), torch.ones(H * vdim, device=DEV)
+    outs = []
+    for spoil in (False, True):
+        rows = x.clone()
+        if spoil:
+            rows[bad, 2 * H * dim:2 * H * dim + H * vdim] = float("inf")
+        out = torch.empty(n, H * vdim, device=DEV)
+        kernels.decay_attention(rows, 0, 2 * H * dim + H * vdim, decay, gain, 1e-5, 1.0, torch.zeros(6, H * dim * vdim, device=DEV),
+                                _step([n]), H, dim, vdim, out)
+        outs.append(out)
+    assert torch.equal(outs[0][:bad], outs[1][:bad]) and not torch.isfinite(outs[1][bad:]).any()
