@@ -428,7 +428,8 @@ static int launch_few_rows(const float* x, const float* w, TY* y, int M, int N, 
 }
 
 // The tile of a product of more than 16 rows: 128 x 128 where those fill the GPU four times over (a block has an SM almost
-// for itself, so a short last wave costs a whole tile), else 64 x 64; and whether its blocks take single chunks of K.
+// for itself, so a short last wave costs a whole tile), else 64 x 64; and whether its blocks take single chunks of K: below six
+// tiles an SM (a request with prompts of 230 tokens, 608 tiles in the widest product: 30.4 ms, 30.7 with the line at three).
 struct TilePlan { bool large; bool chunks; long long scratch; };
 constexpr long long LS_MAX_SCRATCH = 32LL << 20;          // floats: 128 MB
 static TilePlan tile_plan(int M, int N, int K, int n_sms) {
@@ -436,7 +437,7 @@ static TilePlan tile_plan(int M, int N, int K, int n_sms) {
     const int n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
     const long long need = (long long)n_chunks * M * N;
     TilePlan p{t128 >= 4LL * n_sms, false, 0};
-    p.chunks = !p.large && t64 < 3LL * n_sms && n_chunks > 1 && n_chunks <= 65535 && need <= LS_MAX_SCRATCH;
+    p.chunks = !p.large && t64 < 6LL * n_sms && n_chunks > 1 && n_chunks <= 65535 && need <= LS_MAX_SCRATCH;
     if (p.chunks) p.scratch = need;
     return p;
 }
