@@ -22,7 +22,7 @@ from ..config.registry import register_part, build_part
 from ..config.specs import PartSpec
 from .base import CacheNeed, MixerMemory, Part, TensorSpec
 from .linear import Linear
-from .norm import normed_rows
+from .norm import normed_rows, runs_plain
 
 
 @register_part("mixer", "gqa_attention")
@@ -108,9 +108,9 @@ class GQAttention(Part):
         return kernels.gemm_few_plan(n, rows, self.hidden, kernels.bindings.EPI_QKV, self.runtime.n_sms) if self.fused else None
 
     def takes_normed_stream(self, n: int) -> bool:
-        """Whether `forward` may be given a `NormedStream` of n rows: whichever rows of the projection it will use.  (A class
-        with a forward of its own is given finished rows.)"""
-        return type(self).forward is GQAttention.forward and all(self._few_plan(n, r) is not None for r in (self.H * self.hd, (self.H + 2 * self.KV) * self.hd))
+        """Whether `forward` may be given a `NormedStream` of n rows: whichever rows of the projection it will use.  (Another
+        `forward` is given finished rows.)"""
+        return runs_plain(self.forward, GQAttention._plain_forward) and all(self._few_plan(n, r) is not None for r in (self.H * self.hd, (self.H + 2 * self.KV) * self.hd))
 
     # ---- the step
     accumulates = True        # forward(..., residual=x) may add the branch into the float32 stream and return None
@@ -167,6 +167,8 @@ class GQAttention(Part):
         o = rt.empty(n, self.H * self.hd)
         self.attend(q, o, step, memory.kv)
         return self._out(o, residual)
+
+    _plain_forward = forward
 
     def _out(self, o: torch.Tensor, residual: Optional[torch.Tensor]):
         """The output product: added into the stream `residual` if that is given and its product can (returns None)."""

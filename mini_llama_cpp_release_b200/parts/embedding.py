@@ -12,7 +12,7 @@ from ..config.registry import build_part, register_part
 from ..config.specs import PartSpec
 from .base import Part, TensorSpec
 from .linear import Linear
-from .norm import RMSNorm, normed_rows
+from .norm import RMSNorm, normed_rows, runs_plain
 
 
 @register_part("embedding", "token_embedding")
@@ -80,8 +80,9 @@ class LinearHead(Part):
         return self.proj.nbytes()
 
     def takes_normed_stream(self, n: int) -> bool:
-        """Whether `forward` may be given a `NormedStream` of n rows.  (A class with a forward of its own is given finished rows.)"""
-        return type(self).forward is LinearHead.forward and self.proj.few_plan(n) is not None
+        """Whether `forward` may be given a `NormedStream` of n rows.  (Another `forward`, and another product than `Linear` in
+        `proj`, are given finished rows.)"""
+        return runs_plain(self.forward, LinearHead._plain_forward) and type(self.proj) is Linear and self.proj.few_plan(n) is not None
 
     def forward(self, h) -> torch.Tensor:
         h, gain, eps = normed_rows(h)
@@ -89,3 +90,5 @@ class LinearHead(Part):
         if self.softcap is not None:
             kernels.softcap(logits, self.softcap)
         return logits
+
+    _plain_forward = forward

@@ -13,7 +13,7 @@ from ..config.registry import build_part, register_part
 from ..config.specs import PartSpec
 from .base import Part, TensorSpec
 from .linear import Linear
-from .norm import normed_rows
+from .norm import normed_rows, runs_plain
 
 
 
@@ -65,8 +65,8 @@ class SwiGLU(Part):
         return kernels.gemm_few_plan(n, 2 * self.inter, self.hidden, kernels.bindings.EPI_SILU_MUL, self.runtime.n_sms) if self.fused else None
 
     def takes_normed_stream(self, n: int) -> bool:
-        """Whether `forward` may be given a `NormedStream` of n rows.  (A class with a forward of its own is given finished rows.)"""
-        return type(self).forward is SwiGLU.forward and self._few_plan(n) is not None
+        """Whether `forward` may be given a `NormedStream` of n rows.  (Another `forward` is given finished rows.)"""
+        return runs_plain(self.forward, SwiGLU._plain_forward) and self._few_plan(n) is not None
 
     def forward(self, h, step=None, residual=None):
         rt = self.runtime
@@ -86,6 +86,8 @@ class SwiGLU(Part):
             self.down.add_into(a, residual)
             return None
         return self.down(a, torch.float32, partial_ok=True)
+
+    _plain_forward = forward
 
 
 @register_part("feed_forward", "mixture")

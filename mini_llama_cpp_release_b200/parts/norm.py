@@ -30,6 +30,12 @@ def normed_rows(h):
     return (h.x, h.gain, h.eps) if isinstance(h, NormedStream) else (h, None, 0.0)
 
 
+def runs_plain(method, plain) -> bool:
+    """Whether the bound `method` is the function `plain` itself: not one that a subclass, the object or a later assignment to
+    the class put in its place."""
+    return getattr(method, "__func__", None) is plain
+
+
 @register_part("norm", "rmsnorm")
 class RMSNorm(Part):
     graph_safe = True
@@ -62,11 +68,15 @@ class RMSNorm(Part):
         kernels.add_rmsnorm(x, delta, self.gain, self.eps, out)
         return out
 
+    _plain_forward = forward
+
     def into(self, reader, x: torch.Tensor):
         """The norm of x for `reader`, the part that multiplies it: left to the reader's product where it says that it
-        can form the norm itself (`takes_normed_stream`)."""
+        can form the norm itself (`takes_normed_stream`), and only the norm above: a norm whose `forward` is another one is asked for
+        its output."""
         takes = getattr(reader, "takes_normed_stream", None)
-        if takes is not None and self.runtime.dtype == torch.bfloat16 and takes(x.shape[0]):
+        if (takes is not None and self.runtime.dtype == torch.bfloat16 and runs_plain(self.forward, RMSNorm._plain_forward)
+                and takes(x.shape[0])):
             return NormedStream(x, self.gain, self.eps)
         return self.forward(x)
 
