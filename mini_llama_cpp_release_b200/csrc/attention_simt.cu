@@ -56,7 +56,7 @@ __host__ __device__ __forceinline__ int att_pitch(int hd) { return 4 * (((hd + 3
 // registers once for all four rows of its warp.  B200, float32, 3 sequences of about 100 keys, 14 heads of 64 on 2: 82 us a
 // launch with entry-by-entry loads and a row at a time, now 22.
 template <typename T, int ATT_ACC>        // ATT_ACC: output entries a lane holds per row, head size <= 32 * ATT_ACC
-__global__ void __launch_bounds__(ATT_WARPS * 32)
+__global__ void __launch_bounds__(ATT_WARPS * 32, sizeof(T) == 2 && ATT_ACC <= 8 ? 4 : 3)
 attention_simt_kernel(AttnArgs a, PagedKV c) {
     grid_launch_dependents();
     grid_dependency_wait();
@@ -219,7 +219,7 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
 #pragma unroll
             for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) dot[i] = fmaf(qq[i].w, kk.w, dot[i]);
         }
-        bool any = false;
+        bool any = false, apart = false;               // apart: a row sees nothing of a tile that another row of the warp sees
         float corr[ATT_ROWS_PER_WARP];
 #pragma unroll
         for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) {
@@ -239,11 +239,35 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
                 l[i] = l[i] * corr[i] + warp_sum(p);
                 m[i] = m_new;
                 any = true;
+            } else if (row_ok[i]) {
+                corr[i] = -1.0f;                      // (no factor of a sum is negative)
+                apart = true;
             }
             Ps[warp][lane][i] = p;
         }
         __syncwarp();
         if (!any) continue;
+        if (apart) {
+            // Row by row, so that a row that sees nothing of the tile takes nothing from it, not even a zero times an
+            // infinite value of a later token.  Such tiles are the few at the edges of the rows' masks.  (A predicate per row in
+            // the loop below instead costs prompts a fifth.)
+#pragma unroll
+            for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) {
+                if (corr[i] < 0.0f || !row_ok[i]) continue;
+#pragma unroll
+                for (int k = 0; k < ATT_ACC; ++k) acc[i][k] *= corr[i];
+#pragma unroll 1
+                for (int j = 0; j < ATT_TILE; ++j) {
+                    const float pj = Ps[warp][j][i];
+#pragma unroll
+                    for (int k = 0; k < ATT_ACC; ++k) {
+                        const int d = lane + 32 * k;
+                        if (d < hd) acc[i][k] = fmaf(pj, Vs[j * ld + d], acc[i][k]);
+                    }
+                }
+            }
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < ATT_ROWS_PER_WARP; ++i)
 #pragma unroll
