@@ -55,8 +55,11 @@ __host__ __device__ __forceinline__ int att_pitch(int hd) { return 4 * (((hd + 3
 // loads are 16 bytes, the next tile's are in flight while a tile is used, and a key's (a value's) entries pass a lane's
 // registers once for all four rows of its warp.  B200, float32, 3 sequences of about 100 keys, 14 heads of 64 on 2: 82 us a
 // launch with entry-by-entry loads and a row at a time, now 22.
+// Up to 128 entries a head the accumulators are half as many and an SM holds four blocks, not three.  64 sequences of 200 keys,
+// 8 heads of 80 on 8, where only the first of a block's warps has a row: 72 us as it was at first, 83 when all warps multiplied and
+// an SM held three, now 66; 2,048 tokens, 16 heads of 128 on 4: 3,866, 1,665, now 1,372.
 template <typename T, int ATT_ACC>        // ATT_ACC: output entries a lane holds per row, head size <= 32 * ATT_ACC
-__global__ void __launch_bounds__(ATT_WARPS * 32, sizeof(T) == 2 && ATT_ACC <= 8 ? 4 : 3)
+__global__ void __launch_bounds__(ATT_WARPS * 32, ATT_ACC <= 4 || (sizeof(T) == 2 && ATT_ACC <= 8) ? 4 : 3)
 attention_simt_kernel(AttnArgs a, PagedKV c) {
     grid_launch_dependents();
     grid_dependency_wait();
@@ -124,6 +127,10 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
 #pragma unroll
         for (int k = 0; k < ATT_ACC; ++k) acc[i][k] = 0.0f;
     }
+
+    bool any_row = false;                          // the same for the whole warp
+#pragma unroll
+    for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) any_row |= row_ok[i];
 
     const T* kp = (const T*)c.k_pool;
     const T* vp = (const T*)c.v_pool;
@@ -195,6 +202,8 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
             }
         }
         __syncthreads();
+        // A single token of few heads a kv head: most warps have no row.
+        if (!any_row) continue;
 
         // scores of the warp's four rows against the lane's key, each summed in ascending order of the entries
         const int kpos = tile * ATT_TILE + lane;
@@ -250,7 +259,7 @@ attention_simt_kernel(AttnArgs a, PagedKV c) {
         if (apart) {
             // Row by row, so that a row that sees nothing of the tile takes nothing from it, not even a zero times an
             // infinite value of a later token.  Such tiles are the few at the edges of the rows' masks.  (A predicate per row in
-            // the loop below instead costs prompts a fifth.)
+            // the loop below instead: 2,048 tokens, float32, 16 heads of 128 on 4, 2,081 us, 1,372 so.)
 #pragma unroll
             for (int i = 0; i < ATT_ROWS_PER_WARP; ++i) {
                 if (corr[i] < 0.0f || !row_ok[i]) continue;
@@ -414,7 +423,8 @@ static int launch_attention_simt(const void* q, void* out, int dtype, const int*
         launch_pdl(attention_simt_kernel<T, ACC>, grid, dim3(ATT_WARPS * 32), smem, s, a, c);                                          \
     } while (0)
     if (dtype == MLC_DTYPE_F32) {
-        if (hd <= 256) MLC_SIMT_LAUNCH(float, 8);
+        if (hd <= 128) MLC_SIMT_LAUNCH(float, 4);
+        else if (hd <= 256) MLC_SIMT_LAUNCH(float, 8);
         else MLC_SIMT_LAUNCH(float, 16);
     } else {
         if (hd <= 256) MLC_SIMT_LAUNCH(bf16, 8);
