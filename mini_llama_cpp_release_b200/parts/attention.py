@@ -206,7 +206,8 @@ class GQAttention(Part):
                                   self.scale, window, row_tiles, n_splits, part_ml, part_o, sinks=sinks, keep_first=keep,
                                   chunk=chunk, softcap=softcap)
             return
-        n_splits = choose_splits(step, self.H, self.KV, rt.n_sms, tokens_per_block=max(1, 16 // min(16, self.H // self.KV)))
+        n_splits = choose_splits(step, self.H, self.KV, rt.n_sms, tokens_per_block=max(1, 16 // min(16, self.H // self.KV)),
+                                 by_length=rt.dtype == torch.float32)
         part_ml = part_o = None
         if n_splits > 1:
             part_ml = rt.empty(q.shape[0] * self.H * n_splits * 2, dtype=torch.float32)
@@ -216,19 +217,25 @@ class GQAttention(Part):
                                softcap=softcap)
 
 
-def choose_splits(step, q_heads: int, kv_heads: int, n_sms: int, tokens_per_block: int, keys_per_split: int = 32,
+def choose_splits(step, q_heads: int, kv_heads: int, n_sms: int, tokens_per_block: int, by_length: bool = True,
                   max_splits: int = 32) -> int:
-    """How many blocks share one row's key range: enough to fill the GPU when the step
-    has few rows (decoding), one when the rows alone fill it.  A split of a single tile of 32 keys is worth its share of the
-    merging kernel.  B200, a request of 3 prompts of up to 100 tokens and 16 tokens each in float32: 30.7 ms, with splits of
-    256 keys (none, here) 34.8."""
+    """How many blocks share one row's key range.
+
+    Single tokens with `by_length` (a float32 engine): a block per tile of 32 keys, up to `max_splits` blocks that then take equal
+    numbers of tiles.  The count follows from the lengths alone, and a sequence's tiles a block come out the same whatever the
+    longest of the batch is, so a token's sum does not depend on what else is in the batch.  It costs large batches a little:
+    14 heads of 64 on 2, 1,000 keys, B200: one sequence 20.8 us (16 splits 20.0), 64 sequences 81 (3 splits 72, one 174).
+
+    Otherwise as many blocks as fill the GPU when the rows are few, a tile each at least; with `by_length` one below 512 keys
+    (16 tokens behind 1,000 keys, 4 sequences, 14 heads of 64 on 2: 57 us, with splits of 256 keys 84)."""
+    if by_length and step.max_q_len == 1:
+        return max(1, min((step.max_kv_len + 31) // 32, max_splits))
     q_tiles = (step.max_q_len + tokens_per_block - 1) // tokens_per_block
     blocks = q_tiles * kv_heads * max(1, (q_heads // kv_heads + 15) // 16) * step.n_seqs
-    if blocks >= 2 * n_sms:
+    if blocks >= 2 * n_sms or (by_length and step.max_kv_len < 512):
         return 1
     by_fill = (2 * n_sms + blocks - 1) // blocks
-    by_len = max(1, step.max_kv_len // keys_per_split)
-    return max(1, min(by_fill, by_len, max_splits))
+    return max(1, min(by_fill, step.max_kv_len // 32, max_splits))
 
 
 def fused_rows(weights, runtime) -> Linear:
