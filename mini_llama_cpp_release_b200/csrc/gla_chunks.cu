@@ -338,7 +338,8 @@ gla_chunk_outputs_kernel(GcArgs g, int max_chunks) {
 }
 
 long long gla_chunk_floats(int n_seqs, int n_tokens, int max_q_len, int H, int dim, int vdim) {
-    // A run of 32 tokens takes the walk about as long as three launches take.
+    // A run of 32 tokens takes the walk about as long as three launches take (from there on gla_chunks_pay in
+    // kernels/bindings.py says which of the two is the sooner).
     if (max_q_len <= 32 || n_seqs <= 0 || H <= 0 || H > 65535 || dim <= 0 || dim > 256 || vdim <= 0) return 0;
     const long long max_chunks = (max_q_len + GC_TOKENS - 1) / GC_TOKENS;
     if (max_chunks * n_seqs > 65535) return 0;

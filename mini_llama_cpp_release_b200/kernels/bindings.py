@@ -802,18 +802,36 @@ def gla_slices(n_seqs: int, heads: int, dim: int, vdim: int, device: torch.devic
     return (dim + 8 * rows - 1) // (8 * rows)
 
 
+def gla_chunks_pay(n_seqs: int, n_tokens: int, max_q_len: int, heads: int, dim: int, vdim: int, walk_rows: int) -> bool:
+    """Whether a step through a memory with one decay per token and head is sooner done in chunks of 64 tokens
+    (csrc/gla_chunks.cu) than by the walk, by fitted times of both on a B200 (us).
+
+    The walk reads and writes the state and is a chain over the longest run of tokens, the longer a link the more rows of the
+    state a thread holds, or, where its blocks fill the GPU, its multiply-adds.  The chunks are three kernels, and a chunk costs
+    the same whether it holds 64 tokens or one.  Fitted to 1,256 steps of 8 shapes (heads x dim x vdim from 1 x 16 x 16 to 32 x 128 x
+    128 and 4 x 256 x 256) of 1 to 64 runs of 33 to 2,048 tokens, some beside up to 255 single tokens: what the rule takes
+    is 1 % slower than the better form on average, and 1.3 times as slow as the walk at worst.  6 heads of 128 x 256, walk and
+    chunks: one run of 64 tokens 26, 60 us; of 256 73, 65; of 2,048 551, 184; 16 runs of 64 303, 116; one of 256 beside 127
+    single tokens 469, 642."""
+    state = heads * dim * vdim
+    walk = 8.0 + (1.2 if dim > 128 else 1.0) * (1.3e-5 * n_seqs * state + max((0.02 + 0.075 * walk_rows) * max_q_len, 1.2e-6 * n_tokens * state))
+    chunks = min(n_seqs * ((max_q_len + 63) // 64), n_tokens / 64 + n_seqs)          # at most: the device alone knows the lengths
+    return 41.0 + 0.095 * dim + 2.65e-5 * chunks * heads * dim * 64 * ((vdim + 63) // 64) < walk
+
+
 def _head_decay_plan(step, n: int, heads: int, dim: int, vdim: int, device: torch.device) -> Tuple[int, int, Optional[torch.Tensor]]:
     """For a walk over one decay per token and head: rows of the state per thread, slices of partial outputs, and scratch
     memory if the step takes the prompt's form (csrc/gla_chunks.cu).  That form and the step of single tokens want the whole
     head in one slice."""
     lib = core()
-    need = lib.mlc_gla_chunk_floats(step.n_seqs, n, step.max_q_len, heads, dim, vdim)
+    rows = lib.mlc_gla_rows(step.n_seqs, heads, dim, vdim, _sm_count(device))
+    need = 0
+    if n > step.n_seqs and gla_chunks_pay(step.n_seqs, n, step.max_q_len, heads, dim, vdim, rows):
+        need = lib.mlc_gla_chunk_floats(step.n_seqs, n, step.max_q_len, heads, dim, vdim)
     if need > 0 or n == step.n_seqs:
         rows = 4
         while 8 * rows < dim:
             rows *= 2
-    else:
-        rows = lib.mlc_gla_rows(step.n_seqs, heads, dim, vdim, _sm_count(device))
     chunks = torch.empty(need, dtype=torch.float32, device=device) if need > 0 else None
     return rows, (dim + 8 * rows - 1) // (8 * rows), chunks
 
