@@ -324,6 +324,16 @@ def gather_rows(x: torch.Tensor, delta: Optional[torch.Tensor], rows: torch.Tens
                                   out_x.data_ptr(), _ptr(out_delta), _stream()), "gather")
 
 
+def spare_floats(n: int, device: torch.device) -> Optional[torch.Tensor]:
+    """Scratch memory of n floats for a form that another can stand in for: None where there is no room for it (or n is 0)."""
+    if n <= 0:
+        return None
+    try:
+        return torch.empty(n, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def linear_simt(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, n_sms: int = 0) -> None:
     """y = x @ w.T with float32 multiply-adds on the CUDA cores, every output the same sum in the same order
     whatever the number of rows (csrc/linear_simt.cu).  A product of few rows and few columns shares its K range out
@@ -336,7 +346,7 @@ def linear_simt(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, n_sms: int = 
         n_sms = _sm_count(x.device)
     lib = core()
     need = lib.mlc_linear_simt_scratch_floats(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype), m, n, k, n_sms)
-    scratch = torch.empty(need, dtype=torch.float32, device=x.device) if need > 0 else None
+    scratch = spare_floats(need, x.device)      # (without it the same sums, in fewer blocks)
     if scratch is not None:
         count_launches(1)                       # the kernel that adds the chunks
     _check(lib.mlc_linear_simt(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype), y.data_ptr(),
@@ -828,11 +838,11 @@ def _head_decay_plan(step, n: int, heads: int, dim: int, vdim: int, device: torc
     need = 0
     if n > step.n_seqs and gla_chunks_pay(step.n_seqs, n, step.max_q_len, heads, dim, vdim, rows):
         need = lib.mlc_gla_chunk_floats(step.n_seqs, n, step.max_q_len, heads, dim, vdim)
-    if need > 0 or n == step.n_seqs:
+    chunks = spare_floats(need, device)          # up to 2 GB; where there is no room for it the walk does as well
+    if chunks is not None or n == step.n_seqs:
         rows = 4
         while 8 * rows < dim:
             rows *= 2
-    chunks = torch.empty(need, dtype=torch.float32, device=device) if need > 0 else None
     return rows, (dim + 8 * rows - 1) // (8 * rows), chunks
 
 
