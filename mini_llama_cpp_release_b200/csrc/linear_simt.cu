@@ -14,7 +14,7 @@
 // or on which kernel took the step.
 //
 // Three shapes of work:
-//   many rows (prompts)   tiles of 128 x 128 or 64 x 64 outputs, 8 x 8 per thread; operands come in
+//   many rows (prompts)   tiles of 128 x 128 or 64 x 64 outputs, 8 x 8 or 4 x 4 per thread; operands come in
 //                         16-byte loads into registers one K step ahead and go through a
 //                         double-buffered shared-memory tile;
 //   few rows (decoding)   of a float32 matrix whose rows are 16-byte aligned: a stream of weights with almost no
@@ -22,7 +22,10 @@
 //   few rows, other types or alignments   tiles of 16 rows x 64 columns.
 // Where the tiles alone would leave SMs idle, each block of the tiled kernel takes one chunk of K for its tile and
 // leaves the chunk's sums in scratch memory, and a second kernel adds the chunks in order.
-// 230 rows of x, B200, in brackets 128 x 128 tiles without chunks: 9,728 x 896 160 us (266), 896 x 4,864 89 us (350).
+// 256 rows of x, B200, in brackets 128 x 128 tiles without chunks: 9,728 x 896 149 us (266), 896 x 4,864 84 us (715).
+// The tiled kernels start in the ordinary way.  Blocks that were launched while the kernel before ran came to lie several on the SMs
+// that were free first: 64 x 64 tiles of 700 x 1,536 x 8,960 1,356 us so and 815 in the ordinary way, 16 x 64 tiles of 1 x
+// 9,728 x 898 53 and 30.
 #include "tcgen05.cuh"      // mbarriers with bounded waits, TMA tile loads, tensor maps, shared-memory addresses of a cluster's blocks
 
 namespace mlc {
@@ -73,8 +76,6 @@ template <typename TX, typename TW, typename TY, int BM, int BN, int TM, int TN,
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restrict__ y, float* __restrict__ part,
                    int M, int N, int K) {
-    grid_launch_dependents();
-    grid_dependency_wait();
     constexpr int THREADS = (BM / TM) * (BN / TN);
     constexpr int XV = (BM * (LS_BK / 4) + THREADS - 1) / THREADS;       // 16-byte loads per thread and K step
     constexpr int WV = (BN * (LS_BK / 4) + THREADS - 1) / THREADS;
@@ -91,9 +92,9 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
     auto col_of = [&](int j) { return (j / GN) * (BN / (TN / GN)) + tx * GN + j % GN; };
     const bool x_vec = rows_vectorizable(x, K), w_vec = rows_vectorizable(w, K);
 
-    // the totals of the 64 x 64 tile lie in shared memory, a column per thread: its blocks are small, and what hides their
-    // loads is how many of them an SM's registers hold
-    constexpr bool PARKED = !PARTIAL && BM == 64;
+    // the totals of the 64 x 64 tile of 8 x 8 per thread lie in shared memory, a column per thread: its blocks are small, and
+    // what hides their loads is how many of them an SM's registers hold
+    constexpr bool PARKED = !PARTIAL && BM == 64 && TM == 8;
     __shared__ float parked[PARKED ? TM * TN : 1][PARKED ? THREADS : 1];
     float total[PARKED ? 1 : TM][PARKED ? 1 : TN], acc[TM][TN];
 #pragma unroll
@@ -189,8 +190,6 @@ linear_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __res
 // y = the chunks' sums added in ascending order into a total that starts at zero.
 template <typename TY>
 __global__ void linear_simt_add_chunks_kernel(const float* __restrict__ part, TY* __restrict__ y, long long MN, int n_chunks) {
-    grid_launch_dependents();
-    grid_dependency_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= MN) return;
     float total = 0.0f;
@@ -427,19 +426,28 @@ static int launch_few_rows(const float* x, const float* w, TY* y, int M, int N, 
     return launch_few<TY, 16>(x, w, y, M, N, K, status, n_sms, s);
 }
 
-// The tile of a product of more than 16 rows: 128 x 128 where those fill the GPU four times over (a block has an SM almost
-// for itself, so a short last wave costs a whole tile), else 64 x 64; and whether its blocks take single chunks of K: below six
-// tiles an SM (a request with prompts of 230 tokens, 608 tiles in the widest product: 30.4 ms, 30.7 with the line at three).
-struct TilePlan { bool large; bool chunks; long long scratch; };
+// The form of a product of more than 16 rows.  Lone blocks take 37 us a chunk of K with 128 x 128 tiles, 22 with 64 x 64 tiles of
+// 8 x 8 per thread and 13 with 64 x 64 tiles of 4 x 4 (four warps a scheduler instead of one half), B200; a GPU full of
+// them 31, 37 and 31 TFLOP/s.  So
+//   TILES_128    more than 64 rows (64 rows of a 128-row tile are work for nothing: 64 x 151,936 x 896 1,170 us, 64 x 64 tiles
+//                527) where such tiles fill the GPU four times over;
+//   TILES_4X4    one or two chunks of K and at most three tiles an SM, where a lone block's time is what counts (64 x 500 x 300
+//                18 us, 8 x 8 per thread 28, in chunks 31; 700 x 2,000 x 128 17, 21);
+//   CHUNKS       single chunks of K a block and a second kernel that adds them, where whole tiles would fill less than 78 % of
+//                their waves of six an SM (9,728 columns of K = 896, whole and in chunks: 256 rows, 608 tiles 160, 149 us; 300 rows,
+//                760 tiles 169, 176; 400 rows, 1,064 tiles 294, 238; 700 rows, 1,672 tiles 333, 383);
+//   TILES        whole tiles otherwise.
+enum TileForm { TILES_128, TILES, TILES_4X4, CHUNKS };
+struct TilePlan { TileForm form; long long scratch; };
 constexpr long long LS_MAX_SCRATCH = 32LL << 20;          // floats: 128 MB
 static TilePlan tile_plan(int M, int N, int K, int n_sms) {
     const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128), t64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
     const int n_chunks = (K + LS_CHUNK - 1) / LS_CHUNK;
-    const long long need = (long long)n_chunks * M * N;
-    TilePlan p{t128 >= 4LL * n_sms, false, 0};
-    p.chunks = !p.large && t64 < 6LL * n_sms && n_chunks > 1 && n_chunks <= 65535 && need <= LS_MAX_SCRATCH;
-    if (p.chunks) p.scratch = need;
-    return p;
+    if ((M > 64 && t128 >= 4LL * n_sms) || (M + 63) / 64 > 65535) return TilePlan{TILES_128, 0};
+    if (n_chunks <= 2 && t64 <= 3LL * n_sms) return TilePlan{TILES_4X4, 0};
+    const long long need = (long long)n_chunks * M * N, slots = 6LL * n_sms, waves = (t64 + slots - 1) / slots;
+    if (n_chunks > 1 && n_chunks <= 65535 && 100 * t64 < 78 * waves * slots && need <= LS_MAX_SCRATCH) return TilePlan{CHUNKS, need};
+    return TilePlan{TILES, 0};
 }
 
 template <typename TX, typename TW, typename TY>
@@ -453,17 +461,18 @@ static int launch_linear(const void* x, const void* w, void* y, float* scratch, 
     bool chunks = false;
     if (M > 16) {
         const TilePlan p = tile_plan(M, N, K, n_sms);
-        chunks = p.chunks && scratch != nullptr && scratch_floats >= p.scratch;
-        if (p.large || (M + 63) / 64 > 65535) {
+        chunks = p.form == CHUNKS && scratch != nullptr && scratch_floats >= p.scratch;
+        const dim3 g64((N + 63) / 64, (M + 63) / 64, chunks ? n_chunks : 1);
+        if (p.form == TILES_128) {
             dim3 grid((N + 127) / 128, (M + 127) / 128);
             if (grid.y > 65535) return MLC_ERR_BAD_SIZE;
-            launch_pdl(linear_simt_kernel<TX, TW, TY, 128, 128, 8, 8, false>, grid, dim3(256), 0, s, xp, wp, yp, nullptr, M, N, K);
+            linear_simt_kernel<TX, TW, TY, 128, 128, 8, 8, false><<<grid, 256, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
         } else if (chunks) {
-            dim3 grid((N + 63) / 64, (M + 63) / 64, n_chunks);
-            launch_pdl(linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, true>, grid, dim3(64), 0, s, xp, wp, yp, scratch, M, N, K);
+            linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, true><<<g64, 64, 0, s>>>(xp, wp, yp, scratch, M, N, K);
+        } else if (p.form == TILES_4X4) {
+            linear_simt_kernel<TX, TW, TY, 64, 64, 4, 4, false><<<g64, 256, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
         } else {
-            dim3 grid((N + 63) / 64, (M + 63) / 64);
-            launch_pdl(linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, false>, grid, dim3(64), 0, s, xp, wp, yp, nullptr, M, N, K);
+            linear_simt_kernel<TX, TW, TY, 64, 64, 8, 8, false><<<g64, 64, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
         }
     } else {
         if constexpr (sizeof(TX) == 4 && sizeof(TW) == 4) {
@@ -474,15 +483,15 @@ static int launch_linear(const void* x, const void* w, void* y, float* scratch, 
         chunks = tiles < 4 * n_sms && n_chunks > 1 && n_chunks <= 65535 && scratch != nullptr && scratch_floats >= n_chunks * MN;
         if (chunks) {
             dim3 grid(tiles, 1, n_chunks);
-            launch_pdl(linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, true>, grid, dim3(128), 0, s, xp, wp, yp, scratch, M, N, K);
+            linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, true><<<grid, 128, 0, s>>>(xp, wp, yp, scratch, M, N, K);
         } else {
             dim3 grid(tiles, 1);
-            launch_pdl(linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, false>, grid, dim3(128), 0, s, xp, wp, yp, nullptr, M, N, K);
+            linear_simt_kernel<TX, TW, TY, 16, 64, 2, 4, false><<<grid, 128, 0, s>>>(xp, wp, yp, nullptr, M, N, K);
         }
     }
     MLC_LAUNCH_CHECK();
     if (chunks) {
-        launch_pdl(linear_simt_add_chunks_kernel<TY>, dim3((unsigned)((MN + 255) / 256)), dim3(256), 0, s, scratch, yp, MN, n_chunks);
+        linear_simt_add_chunks_kernel<TY><<<(unsigned)((MN + 255) / 256), 256, 0, s>>>(scratch, yp, MN, n_chunks);
         MLC_LAUNCH_CHECK();
     }
     return 0;

@@ -31,3 +31,20 @@ def test_same_sum_whatever_the_rows(n, k):
     odd = torch.empty(n * k + 1, device=DEV)[1:].view(n, k)
     odd.copy_(w)
     assert torch.equal(product(3, odd), whole[:3])
+
+
+# (columns, K) of 17 to 64 rows on 148 SMs: tiles of 4 x 4 per thread up to 444 tiles of one or two chunks, single chunks below
+# 78 % of a wave of 888 tiles, whole tiles from there on, single chunks again in the second wave
+@pytest.mark.parametrize("n,k", [(1, 512), (500, 300), (28416, 512), (28417, 512), (44288, 512), (44353, 512), (56833, 300), (64, 600),
+                                 (3000, 200), (30000, 256)])
+def test_same_sum_in_every_form_of_17_to_64_rows(n, k):
+    g = torch.Generator().manual_seed(n * 31 + k)
+    x, w = torch.randn(65, k, generator=g).to(DEV), torch.randn(n, k, generator=g).to(DEV)
+
+    def product(rows):
+        y = torch.full((len(rows), n), float("nan"), device=DEV)
+        kernels.linear_simt(rows, w, y)
+        return y
+    want = torch.cat([product(x[i:i + 13]) for i in range(0, 65, 13)])           # five steps of few rows
+    for rows in (17, 33, 64, 65):
+        assert torch.equal(product(x[:rows]), want[:rows]), rows
