@@ -280,7 +280,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int s = 0; s < early; ++s, next()) ask(s, false, true);
     }
 
-    int slot = 0, round = 0, done = 0, parity = 0;
+    int slot = 0, round = 0, done = 0, asked = early, parity = 0;     // stages used and asked for, of all tiles
     bool ok = true;
     for (int tile = first_tile; tile < tiles; tile += tile_step, parity ^= 1) {
         float* const mine = sums + ((parity * warps + warp) * pw) * TOKENS * LF_ROWS;
@@ -325,6 +325,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             if (lane == 0 && done + LF_SLOTS < total_stages) {
                 ask(slot, true, true);
                 next();
+                ++asked;
             }
             ++done;
             if (++slot == LF_SLOTS) {
@@ -346,6 +347,16 @@ linear_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
             }
         }
         ok = all_ok;
+    }
+    // A wait ran out: nobody leaves while a copy into its shared memory may still be under way (bounded waits again).
+    if (!ok && lane == 0) {
+        for (; done < asked; ++done) {
+            mbar_wait(bars + 8u * (unsigned)slot, (unsigned)round & 1u, status, 61);
+            if (++slot == LF_SLOTS) {
+                slot = 0;
+                ++round;
+            }
+        }
     }
     if (cluster > 1) {                                               // one tile per cluster; its blocks share out the outputs
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
