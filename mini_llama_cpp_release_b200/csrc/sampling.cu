@@ -260,12 +260,19 @@ __device__ __forceinline__ void for_each_key(const float* __restrict__ row, int 
 
 // Top-k sampling: find the k largest keys (ties by lowest id), sort them by (logit descending, id ascending), walk.
 //
-// A row is read twice.  First every thread takes the largest key of its share: the k-th largest of these 1,024 is a key that
-// at least k of the row's keys reach, and of a row in no particular order not many more than k.  Then all keys that
-// reach it are gathered and sorted.  Where they are more than the room for them (ties without end, a k close to 1,024) the
-// k-th key is found by its digits instead, eight bits per pass.  24 steps of 64 rows of 151,936 with k = 40, B200: 47.9 ms
-// with the digits alone (244 us a step in this kernel), 42.9 with two reads.
+// The k largest are found by reading the row twice, or by their digits.
+// Two reads: every thread takes the largest key of its share (1,024 shares from 4,096 logits on, vocab / 4 at least); the
+// k-th largest of these is a key that at least k of the row's keys reach, and of a row in no particular order not many more
+// than k; then all keys that reach it are gathered and sorted.  Digits: the k-th key eight bits per pass over the row, four
+// passes, and a pass that gathers.
+// Of S shares of a row in no particular order some -S ln(1 - k/S) keys reach the k-th: 1,560 at k = 800, but 2,160 at 900, more
+// than the room for them; and in short rows the sort of the shares costs more than the passes it saves.  So two reads where
+// they are sure to be enough and to pay, the digits elsewhere.  In a row most of whose keys are one and the same (a mask over
+// the vocabulary) the k-th share's key is that one: found out from the sorted shares, and left to the digits as well.
+// B200, us a launch, digits and two reads: 64 rows of 151,936, k = 40 217, 37, k = 600 228, 56; of 32,000, k = 800 80, 52; one row of 4,000,
+// k = 100 17, 22, k = 800 31, 46; of 1,000, k = 40 18, 27.  A masked row (k = 40 of 20 logits that are not -inf) 192, 252 in vain, 199 so.
 constexpr int TOPK_ROOM = 2048;
+constexpr int TOPK_TWO_READS_VOCAB = 2048, TOPK_TWO_READS_SHARE = 16, TOPK_TWO_READS_MAX = 800, TOPK_TIES = 512;
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_top_k_kernel(const float* __restrict__ logits, int vocab, float temperature, int top_k,
@@ -286,44 +293,52 @@ sample_top_k_kernel(const float* __restrict__ logits, int vocab, float temperatu
     const float* row = logits + (long long)blockIdx.x * vocab;
     const int k = min(top_k, vocab);
 
-    // --- the largest key of every thread's share, and the k-th of them
-    unsigned int most = 0;
-    for_each_key(row, vocab, [&](unsigned int key, int) { most = max(most, key); });
-    room_k[threadIdx.x] = most;
-    room_i[threadIdx.x] = threadIdx.x;
-    if (threadIdx.x == 0) n_greater = 0;
-    __syncthreads();
-    block_sort_keys(room_k, room_i, SAMPLE_THREADS);
-    const unsigned int reach = vocab >= SAMPLE_THREADS ? room_k[k - 1] : 0u;      // (a thread without a share has no key)
-    __syncthreads();
-    // --- all keys that reach it
-    for_each_key(row, vocab, [&](unsigned int key, int i) {
-        if (key >= reach) {
-            const int slot = atomicAdd(&n_greater, 1);
-            if (slot < TOPK_ROOM) {
-                room_k[slot] = key;
-                room_i[slot] = i;
+    bool found_all = false;                    // the same for the whole block
+    if (vocab >= TOPK_TWO_READS_VOCAB && k <= TOPK_TWO_READS_MAX && k <= vocab / TOPK_TWO_READS_SHARE) {
+        // --- the largest key of every thread's share, and the k-th of them
+        unsigned int most = 0;                 // a thread without a share has no key
+        for_each_key(row, vocab, [&](unsigned int key, int) { most = max(most, key); });
+        room_k[threadIdx.x] = most;
+        room_i[threadIdx.x] = threadIdx.x;
+        if (threadIdx.x == 0) n_greater = 0;
+        __syncthreads();
+        block_sort_keys(room_k, room_i, SAMPLE_THREADS);
+        const unsigned int reach = room_k[k - 1];
+        const bool tied = room_k[min(k - 1 + TOPK_TIES, SAMPLE_THREADS - 1)] == reach;
+        __syncthreads();
+        if (!tied) {
+            // --- all keys that reach it
+            for_each_key(row, vocab, [&](unsigned int key, int i) {
+                if (key >= reach) {
+                    const int slot = atomicAdd(&n_greater, 1);
+                    if (slot < TOPK_ROOM) {
+                        room_k[slot] = key;
+                        room_i[slot] = i;
+                    }
+                }
+            });
+            __syncthreads();
+            const int found = n_greater;
+            __syncthreads();
+            if (found <= TOPK_ROOM) {
+                int n_room = 1;
+                while (n_room < found) n_room <<= 1;
+                for (int i = found + threadIdx.x; i < n_room; i += blockDim.x) {
+                    room_k[i] = 0;
+                    room_i[i] = 0x7fffffff;
+                }
+                __syncthreads();
+                block_sort_keys(room_k, room_i, n_room);
+                for (int i = threadIdx.x; i < k; i += blockDim.x) {
+                    cand_i[i] = room_i[i];
+                    cand_v[i] = row[room_i[i]];
+                }
+                __syncthreads();
+                found_all = true;
             }
         }
-    });
-    __syncthreads();
-    const int found = n_greater;
-    __syncthreads();
-    if (found <= TOPK_ROOM) {                  // the same for the whole block
-        int n_room = 1;
-        while (n_room < found) n_room <<= 1;
-        for (int i = found + threadIdx.x; i < n_room; i += blockDim.x) {
-            room_k[i] = 0;
-            room_i[i] = 0x7fffffff;
-        }
-        __syncthreads();
-        block_sort_keys(room_k, room_i, n_room);
-        for (int i = threadIdx.x; i < k; i += blockDim.x) {
-            cand_i[i] = room_i[i];
-            cand_v[i] = row[room_i[i]];
-        }
-        __syncthreads();
-    } else {
+    }
+    if (!found_all) {
         // --- the k-th largest key, 8 bits at a time from the top
         unsigned int prefix = 0, mask = 0;
         int remaining = k;

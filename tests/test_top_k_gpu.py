@@ -23,10 +23,14 @@ def test_pick_lies_where_the_sorted_row_has_it(vocab, k, kind):
         rows = torch.arange(vocab).float().expand(5, vocab).contiguous() / vocab
     elif kind == "one_share":
         rows[:, : min(vocab, 4000):4] += 30.0         # the largest in few threads' shares
+    _check(rows, k)
+
+
+def _check(rows, k):
     ids, pos = list(range(5)), [3, 9, 27, 81, 243]
     sampler = DeviceSampler(SamplingParams(0.7, k, 11), torch.device(DEV))
     got = sampler.sample(rows.to(DEV), ids, pos)
-    kk = min(k, vocab)
+    kk = min(k, rows.shape[1])
     for b in range(5):
         # larger first, lower ids first among equal ones
         order = torch.argsort(rows[b].double(), descending=True, stable=True)[:kk]
@@ -38,3 +42,16 @@ def test_pick_lies_where_the_sorted_row_has_it(vocab, k, kind):
         r = kernels.uniform_of(11, ids[b], pos[b])
         # a float32 running sum of up to 1,024 weights
         assert (cum[i - 1] if i else 0.0) <= r + 1e-4 and cum[i] >= r - 1e-4, (b, i, r)
+
+
+@pytest.mark.parametrize("vocab,k", [(2047, 127), (2048, 128), (2048, 129), (4096, 256), (4097, 257), (12800, 800), (12816, 801), (40000, 800)])
+@pytest.mark.parametrize("kind", ["normal", "masked", "few_kept"])
+def test_both_ways_of_finding_the_largest_at_the_lines_between_them(vocab, k, kind):
+    """Two reads up to a sixteenth of the row and 800, from 2,048 logits on; the digits elsewhere, and where one value fills the row."""
+    g = torch.Generator().manual_seed(vocab * 3 + k)
+    rows = torch.randn(5, vocab, generator=g)
+    if kind == "masked":
+        rows[:, torch.randperm(vocab, generator=g)[: vocab - 2 * k]] = float("-inf")
+    elif kind == "few_kept":
+        rows[:, torch.randperm(vocab, generator=g)[: vocab - k // 2]] = torch.finfo(torch.float32).min
+    _check(rows, k)
