@@ -474,14 +474,23 @@ extern "C" int mlc_sample(const float* logits, int rows, int vocab, float temper
     if (rows <= 0) return 0;
     if (vocab <= 0 || !(temperature > 0.0f) || top_k < 0 || top_k == 1) return MLC_ERR_BAD_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
+    // Many rows: blocks that start ahead of the kernel before come to lie two to an SM (64 rows of 151,936 a launch: k = 40 44.7
+    // us, 36.8 in the ordinary way, the whole vocabulary 101, 79; one row 35.3, 36.1).
+    const bool early = rows <= 16;
     if (top_k == 0) {
-        launch_pdl(sample_temperature_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, s, logits, vocab, temperature, seed, seed_ptr, seq_ids,
-                                                                  positions, out);
+        if (early)
+            launch_pdl(sample_temperature_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, s, logits, vocab, temperature, seed, seed_ptr, seq_ids,
+                       positions, out);
+        else
+            sample_temperature_kernel<<<rows, SAMPLE_THREADS, 0, s>>>(logits, vocab, temperature, seed, seed_ptr, seq_ids, positions, out);
     } else {
         const int k = top_k < vocab ? top_k : vocab;
         if (k > TOPK_MAX) return MLC_ERR_UNSUPPORTED;
-        launch_pdl(sample_top_k_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, s, logits, vocab, temperature, top_k, seed, seed_ptr, seq_ids,
-                                                            positions, out);
+        if (early)
+            launch_pdl(sample_top_k_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, s, logits, vocab, temperature, top_k, seed, seed_ptr, seq_ids,
+                       positions, out);
+        else
+            sample_top_k_kernel<<<rows, SAMPLE_THREADS, 0, s>>>(logits, vocab, temperature, top_k, seed, seed_ptr, seq_ids, positions, out);
     }
     MLC_LAUNCH_CHECK();
     return 0;
