@@ -19,6 +19,7 @@ from .batch import MiniBatch, SequenceChunk
 from .decode_runner import DecodeRunner, capturing, padded_batch
 from .model import Model
 from .step_info import StepInfo
+from .step_shapes import StepShapes
 
 
 class ContextOverflow(ValueError):
@@ -165,26 +166,21 @@ class Context:
             page_tables=page_tables, slots_long=slots_dev.long() if self.cache.has_state else None,
         )
 
-    # A step is some two hundred launches issued from Python; when its kernels are fast the host
-    # becomes the limit.  A shape of step that comes again (the same numbers of tokens and sequences, the same
-    # longest lengths: fixed-size prompts, a benchmark, chunks of a fixed size) is therefore captured into a CUDA
-    # graph the second time it is seen (below 64 tokens the eighth time: lengths of short prompts are many and each comes
-    # again soon) and replayed from then on; everything that may differ between two such
-    # steps (tokens, positions, lengths, pages) lies in the description buffer the graph reads.
-    # A capture costs a step several times over (a run to warm up, the collector, two synchronisations), so it has to be worth it:
-    #   - a step of more tokens than STEP_GRAPH_MAX_TOKENS is not captured: its kernels take longer than issuing
-    #     them does (8,191 tokens at the 0.5B sizes still gain 1 %: 12.02 ms replayed, 12.10 issued);
-    #   - a captured shape gives way to another only when it was not used for STEP_GRAPH_IDLE steps: more shapes in turn than
-    #     are kept would otherwise be captured at every single step.
-    # Sixteen ragged prompts of up to 2,048 tokens (1.5B sizes), whose pieces take turns in shape, B200: 159 ms a request with
-    # captures at nearly every step, 94 without.
-    STEP_GRAPHS = 8                     # captured shapes kept
+    # A shape of step that comes again (the same numbers of tokens and sequences, the same longest lengths: fixed-size prompts,
+    # a benchmark, chunks of a fixed size) is captured into a CUDA graph and replayed from then on; everything that may
+    # differ between two such steps (tokens, positions, lengths, pages) lies in the description buffer the graph reads.
+    # Which shapes: step_shapes.py.  Steps of at least STEP_GRAPH_LONG tokens are captured the second time they are
+    # seen, shorter ones the eighth time (lengths of short prompts are many and each comes again soon).  The two have places of
+    # their own, so that a stream of short prompts, or of single tokens, each of another shape, takes none from the long steps.
+    # Steps of more than STEP_GRAPH_MAX_TOKENS are issued every time: a replay saves them 0 to 3 %, and a capture costs ten such
+    # steps and more, and the step's scratch memory for as long as the shape is kept.  ms, issued and replayed, B200, at the
+    # Qwen2-0.5B and 1.5B sizes and in 6 Betepel layers: one prompt of 4,096 tokens 4.99, 4.80; 12.8, 11.8; 5.15, 4.95; one of 8,191 11.5,
+    # 11.5; 26.7, 27.1; 9.60, 9.43; 12 of 1,024 11.7, 11.8; 32.2, 32.1; 13.7, 13.6; 8 of 2,048 17.1, 16.9; 46.1, 46.2; 18.6, 18.3.
+    # Captures took 70 to 860.
     STEP_GRAPH_MAX_TOKENS = 8192
-    STEP_GRAPH_IDLE = 64
-
-    @staticmethod
-    def _sights_to_capture(n_tokens: int) -> int:
-        return 2 if n_tokens >= 64 else 8
+    STEP_GRAPHS = 8                     # captured shapes kept, of either kind
+    STEP_GRAPH_LONG = 64
+    STEP_GRAPH_IDLE = 64                # steps of its kind after which an unused shape gives its place to any other
 
     def forward_batch(self, batch: MiniBatch) -> torch.Tensor:
         """Run the batch's tokens; returns float32 logits [number of wanted places, vocab], in
@@ -219,8 +215,7 @@ class Context:
         """One step: all of the batch's tokens at once."""
         dev = self.model.runtime.device
         with torch.cuda.device(dev):
-            n_new = sum(len(c.tokens) for c in batch.chunks)
-            if self.use_graphs and n_new <= self.STEP_GRAPH_MAX_TOKENS:
+            if self.use_graphs and batch.n_tokens <= self.STEP_GRAPH_MAX_TOKENS:
                 logits = self._forward_maybe_replayed(batch)
             else:
                 step = self.describe(batch)
@@ -234,24 +229,19 @@ class Context:
 
     def _forward_maybe_replayed(self, batch: MiniBatch) -> torch.Tensor:
         graphs = self.__dict__.setdefault("_step_graphs", {})
-        seen = self.__dict__.setdefault("_step_shapes_seen", {})
         dev = self.model.runtime.device
         layout = self._describe_host(batch)
         key = self._step_key(layout)
+        long = layout["n_tokens"] >= self.STEP_GRAPH_LONG
+        shapes = self.__dict__.setdefault("_step_shapes", {}).setdefault(long, StepShapes(2 if long else 8))
+        capture, leaving = shapes.coming(key, self.STEP_GRAPHS, self.STEP_GRAPH_IDLE)
         entry = graphs.get(key)
-        self._graph_clock = now = getattr(self, "_graph_clock", 0) + 1
         if entry is not None:
-            entry["used"] = now
             self._upload(layout, into=entry["dev"])
             entry["graph"].replay()
-            graphs[key] = graphs.pop(key)                                     # most recently used last
             return entry["logits"].clone()
-        seen[key] = seen.pop(key, 0) + 1
-        if len(seen) > 64:
-            seen.pop(next(iter(seen)))
         own = self._upload(layout)
-        room = len(graphs) < self.STEP_GRAPHS or now - next(iter(graphs.values()))["used"] > self.STEP_GRAPH_IDLE
-        if seen[key] < self._sights_to_capture(layout["n_tokens"]) or not room:
+        if not capture:
             return self.model.forward(self._step_over(own, layout), self.cache)
         # worth a capture: run it once more eagerly on a side stream (what capture needs), then capture and replay
         stream = torch.cuda.Stream(device=dev)
@@ -267,9 +257,9 @@ class Context:
         with capturing(graph, stream):
             logits = self.model.forward(self._step_over(own, layout), self.cache)
         torch.cuda.synchronize(dev)
-        while len(graphs) >= self.STEP_GRAPHS:
-            graphs.pop(next(iter(graphs)))
-        graphs[key] = dict(graph=graph, dev=own, logits=logits, used=now)
+        shapes.keep(key, leaving)
+        graphs.pop(leaving, None)
+        graphs[key] = dict(graph=graph, dev=own, logits=logits)
         graph.replay()
         return logits.clone()
 
