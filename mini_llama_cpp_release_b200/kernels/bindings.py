@@ -1620,26 +1620,36 @@ def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> 
     chains of like kernels at the Qwen2-0.5B, 1.5B and 7B sizes (us, against the tcgen05 form, with its norm where there is one):
       ADD      blocks x splits of about two an SM, at least 7 and at most 26 units a split.  8 rows: 896 x 896 1.5 against
                2.3, 896 x 4,864 2.7 against 3.5, 1,536 x 8,960 5.8 against 6.6, 3,584 x 3,584 5.3 against 6.7; but 3,584 x
-               18,944 25.5 against 24.0: not above 40 M weights.  16 rows: 896 x 4,864 3.2 against 3.7, but 3,584 x 3,584 7.8
+               18,944 25.5 against 24.0: not above 40 M weights, and 4,096 x 4,096 7.9 against 7.5: not above 16 M where tiles
+               are more than SMs.  16 rows: 896 x 4,864 3.2 against 3.7, but 3,584 x 3,584 7.8
                against 6.8 and 1,536 x 8,960 7.9 against 6.7: not above 5 M.  32 rows: 896 x 4,864 4.2 against 4.7.
+               A whole K of up to 14 units is a warp a unit (1,024 x 256, 8 and 16 rows: 1.8 and 2.3, two units a warp 2.2 and
+               3.3), and left to the tcgen05 form where so few warps take long over the outputs of the rows (1,024 x 128: 8
+               rows 2.2 against 2.3, 9 rows 2.8 against 2.3; 1,024 x 256: 24 rows 3.0 against 3.1, 32 rows 3.5 against 3.2).
       QKV      a block per tile (at most one an SM).  8 rows: 1,152 x 896 2.5 against 6.6, 2,048 x 1,536 3.8 against 8.3,
                4,608 x 3,584 9.2 against 13.5; 16 rows: 3.0, 4.6, 12.2 against 6.7, 8.5, 13.3; 32 rows: 1,152 x 896 5.2
                against 7.0.
       others   8 rows: 9,728 x 896 with SiLU 5.2 against 7.5, 17,920 x 1,536 10.6 against 13.1, 37,888 x 3,584 44.9 against
                48.1, the head's 151,936 x 896 44.6 against 47.4; 16 rows: 6.4 against 7.5, 12.6 against 13.6, 3,584
-               columns slower; 24 rows: 9.1 against 8.9."""
+               columns slower; 24 rows: 9.1 against 8.9; a single unit of K: three tiles at a time for
+               the one warp 2.7 against 2.4 (256 x 64, 8 rows), so one."""
     if n_tok < 1 or n_tok > 32 or k < 64 or k % 64:
         return None
     units, tiles = k // 64, (n_out + 15) // 16
     if epilogue == EPI_ADD:
-        if n_out * k > (40_000_000 if n_tok <= 8 else 5_000_000):
+        if n_out * k > (5_000_000 if n_tok > 8 else 16_000_000 if tiles >= n_sms else 40_000_000):
             return None
         splits = (units + 27) // 28 if tiles >= n_sms else max(1, min(units // 7, 2 * n_sms // tiles), (units + 25) // 26)
         per = (units + splits - 1) // splits
         splits = (units + per - 1) // per
-        uw = max(1 if per <= 2 else 2, (per + 13) // 14)
+        short = splits == 1 and per <= (6 if n_tok <= 8 else 14)
+        uw = 1 if short or per <= 2 else max(2, (per + 13) // 14)
         if uw > 2:
             return None
+        if splits == 1:
+            rounds = (tiles + n_sms - 1) // n_sms
+            if rounds * n_tok > 2 * ((per + uw - 1) // uw) * (3 if n_tok > 16 and rounds == 1 else 2):
+                return None
         rt = 2 if tiles < n_sms and tiles * splits > 2 * n_sms else 1
         return ((per + uw - 1) // uw, uw, rt, min((tiles + rt - 1) // rt, n_sms), splits)
     if epilogue == EPI_QKV:
@@ -1650,7 +1660,7 @@ def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> 
     uw = (units + 15) // 16
     if uw > (4 if n_tok <= 8 else 2 if n_tok <= 16 else 0):
         return None
-    rt = {1: 3, 2: 2}.get(uw, 1) if n_tok <= 8 else 1
+    rt = {1: 3, 2: 2}.get(uw, 1) if n_tok <= 8 and units > 1 else 1
     blocks = n_sms if n_tok <= 8 and uw > 1 else 2 * n_sms
     return ((units + uw - 1) // uw, uw, rt, min((tiles + rt - 1) // rt, blocks), 1)
 

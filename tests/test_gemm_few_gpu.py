@@ -133,3 +133,26 @@ def test_few_rows_refuses_what_it_does_not_take():
     big = torch.zeros(33, 128, dtype=torch.bfloat16, device=DEV)
     with pytest.raises(kernels.KernelError, match="size"):
         kernels.gemm_few(big, w, torch.empty(33, 32, device=DEV), STORE, (2, 1, 1, 2, 1))
+
+
+def test_short_inner_sizes_go_to_the_few_row_product_only_where_its_few_warps_keep_up():
+    for n_tok, n_out, k, few in ((8, 1024, 128, True), (9, 1024, 128, False), (8, 1024, 64, False), (1, 1024, 64, True), (17, 1024, 256, True),
+                                 (32, 1024, 256, False), (16, 4096, 256, False), (4, 4096, 256, True), (32, 1024, 512, True), (8, 4096, 4096, False)):
+        assert (bindings.gemm_few_plan(n_tok, n_out, k, ADD, 148) is not None) is few, (n_tok, n_out, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [64, 192, 320, 448, 896])
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 32])
+def test_adding_products_of_short_inner_sizes(T, K):
+    for N in (16, 1000, 4100):
+        plan = bindings.gemm_few_plan(T, N, K, ADD, 148)
+        x, w, gain, want = operands(T, N, K, False)
+        out = torch.ones(T, N, device=DEV)
+        if plan is not None:
+            run(x, w, out, ADD, plan, gain)
+            close(out, want + 1, F32)
+        store = bindings.gemm_few_plan(T, N, K, STORE, 148)
+        if store is not None:
+            run(x, w, out, STORE, store, gain)
+            close(out, want, F32)
