@@ -325,7 +325,7 @@ static int launch_few_epilogue(const FewArgs& g, int epilogue, bool norm, int bl
 
 template <int NT>
 static int launch_few_shape(const FewArgs& g, int uw, int rt, int epilogue, bool norm, int blocks, int splits, int warps, cudaStream_t s) {
-    switch (uw * 8 + rt) {     // the shapes gemm_few_plan in kernels/bindings.py gives
+    switch (uw * 8 + rt) {     // what gemm_few_plan in kernels/bindings.py gives, and the shapes beside those that a caller's own plan may name
         case 9: return launch_few_epilogue<NT, 1, 1>(g, epilogue, norm, blocks, splits, warps, s);
         case 10: return launch_few_epilogue<NT, 1, 2>(g, epilogue, norm, blocks, splits, warps, s);
         case 11: if constexpr (NT == 1) return launch_few_epilogue<NT, 1, 3>(g, epilogue, norm, blocks, splits, warps, s); break;

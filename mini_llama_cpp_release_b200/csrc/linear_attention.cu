@@ -208,7 +208,9 @@ gla_walk_kernel(GlaArgs a) {
 
 // Steps of one token per sequence: a warp per (sequence, head, eight columns), a column's rows spread over its lanes, so that
 // the state streams through in whole lines and nothing but a warp's sum stands between its arrival and the output.  Bound by
-// the state's bytes: B200, 8 sequences, 6 heads of 128 x 257 (12.6 MB in and out), 5.5 us, the walk 32 us.
+// that chain (the boundary, one trip for the state, the sums) in small batches, by the state's bytes in large ones: B200, 6
+// heads of 128 x 257, 8 sequences (12.6 MB in and out) 5.5 us = 2.3 TB/s, the walk 32; of 128 x 256, 64 sequences 24 us = 4.2
+// TB/s, the walk 144; 256 sequences 102 us, 394.
 constexpr int GLS_COLS = 8;
 
 template <int RPL, bool SILU>          // rows of a column per lane: dim <= 32 * RPL

@@ -5,8 +5,12 @@ Which kernel runs is decided by the operand types and sizes, never by the model:
   * any float32 operand (the whole 32-bit path, or a tensor the checkpoint stores in
     32-bit while the engine computes in bfloat16): the float32 multiply-add kernel of
     csrc/linear_simt.cu.  No tensor-core mode takes part.
-  * bfloat16 × bfloat16 with an inner size that is a multiple of 8: the tcgen05/TMA kernel of
-    csrc/gemm_tcgen05.cu, always when an epilogue is fused (Q/K/V with bias, rotation and
+  * bfloat16 × bfloat16 of up to 32 rows, with an inner size that is a multiple of 64 and where
+    `kernels.gemm_few_plan` has a plan (by rows, sizes and epilogue): the few-row product of
+    csrc/gemm_few.cu, which also forms the RMS norm of its input on the way where a part may leave it
+    to it (`of_norm`).
+  * other bfloat16 × bfloat16 products with an inner size that is a multiple of 8: the tcgen05/TMA
+    kernel of csrc/gemm_tcgen05.cu, when an epilogue is fused (Q/K/V with bias, rotation and
     cache write; gate/up with SiLU·mul), and for plain products of up to 64 rows (decoding),
     where the K range is split over blocks and the partial sums are left to the consumer.
   * plain bfloat16 products of more rows (prompts): the tokens-as-M tcgen05 kernels, one SM
