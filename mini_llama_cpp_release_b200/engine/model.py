@@ -136,4 +136,4 @@ class Model:
             rows_x = rt.empty(n_want, x.shape[1], dtype=torch.float32)
             rows_p = rt.empty(n_want, x.shape[1], dtype=torch.float32) if pending is not None else None
             kernels.gather_rows(x, pending, step.want_rows, rows_x, rows_p)
-        return self.parts.head.forward(norm_into(self.parts.final_norm, self.parts.head, rows_x, rows_p))
+        return self.parts.head.forward(norm_into(self.parts.final_norm, self.parts.head, rows_x, rows_p, n_want))

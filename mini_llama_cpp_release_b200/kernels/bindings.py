@@ -14,7 +14,7 @@ from ..csrc import build as _build
 __all__ = [
     "KernelError", "KVView", "require_cuda", "dtype_code", "embed", "add_rmsnorm", "rope_table", "qkv_post",
     "attention_simt", "silu_mul", "gather_rows", "linear_simt", "argmax", "sample", "uniform_of", "core",
-    "launch_count", "reset_launch_count", "library_launch_count", "count_library_launches", "attention_mma_available", "attention_mma", "attention_mma_plan", "attention_decode_cluster_limit", "attention_decode_splits", "attention_decode_clusters_resident", "attention_tcgen05", "attention_tcgen05_takes", "attention_tcgen05_blocks", "attention_library", "gemm_tcgen05", "gemm_few", "gemm_few_plan", "gemm_qkv_cluster_splits", "gemm_qkv_clusters_resident", "gemm_tcgen05_rows", "gemm_rows_takes", "gemm_rows_add_plan", "gemm_add_plan", "gemm_tcgen05_pair", "gemm_pair_takes", "gemm_prompt", "library_gemm", "gemm_status", "check_gemm_status", "set_pdl", "PinnedCopy", "decode_advance",
+    "launch_count", "reset_launch_count", "library_launch_count", "count_library_launches", "attention_mma_available", "attention_mma", "attention_mma_plan", "attention_decode_cluster_limit", "attention_decode_splits", "attention_decode_clusters_resident", "attention_tcgen05", "attention_tcgen05_takes", "attention_tcgen05_blocks", "attention_library", "gemm_tcgen05", "gemm_few", "gemm_few_plan", "FEW_ROWS", "gemm_qkv_cluster_splits", "gemm_qkv_clusters_resident", "gemm_tcgen05_rows", "gemm_rows_takes", "gemm_rows_add_plan", "gemm_add_plan", "gemm_tcgen05_pair", "gemm_pair_takes", "gemm_prompt", "library_gemm", "gemm_status", "check_gemm_status", "set_pdl", "PinnedCopy", "decode_advance",
     "layernorm", "qk_norm_rope_cache", "softcap", "convert", "causal_conv", "gated_delta_rule", "gated_rmsnorm", "block_gates",
     "linear_scan", "gates_scan_step", "gates_scan_step_takes",
     "moe_route", "moe_plan", "moe_plan_rows", "grouped_linear", "gemm_few_grouped", "gemm_few_grouped_takes", "moe_gather", "moe_combine", "scaled_add", "scaled_add_experts", "gla", "gla_slices", "latent_prepare",
@@ -1611,6 +1611,9 @@ def gemm_qkv_cluster_splits(n_tok: int, n_out: int, k: int, resident: tuple = No
     return 1
 
 
+FEW_ROWS = 32             # the most rows the few-row product takes
+
+
 @functools.lru_cache(maxsize=4096)
 def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> Optional[tuple]:
     """How csrc/gemm_few.cu takes a product (`plan` of `gemm_few`), or None where the tcgen05 form is the better one.
@@ -1633,7 +1636,7 @@ def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> 
                48.1, the head's 151,936 x 896 44.6 against 47.4; 16 rows: 6.4 against 7.5, 12.6 against 13.6, 3,584
                columns slower; 24 rows: 9.1 against 8.9; a single unit of K: three tiles at a time for
                the one warp 2.7 against 2.4 (256 x 64, 8 rows), so one."""
-    if n_tok < 1 or n_tok > 32 or k < 64 or k % 64:
+    if n_tok < 1 or n_tok > FEW_ROWS or k < 64 or k % 64:
         return None
     units, tiles = k // 64, (n_out + 15) // 16
     if epilogue == EPI_ADD:

@@ -105,12 +105,15 @@ class GQAttention(Part):
         return b + (self.bias.numel() * 4 if self.bias is not None else 0)
 
     def _few_plan(self, n: int, rows: int):
-        return kernels.gemm_few_plan(n, rows, self.hidden, kernels.bindings.EPI_QKV, self.runtime.n_sms) if self.fused else None
+        if n > kernels.FEW_ROWS or not self.fused:       # (a prompt asks a few times a layer)
+            return None
+        return kernels.gemm_few_plan(n, rows, self.hidden, kernels.bindings.EPI_QKV, self.runtime.n_sms)
 
     def takes_normed_stream(self, n: int) -> bool:
         """Whether `forward` may be given a `NormedStream` of n rows: whichever rows of the projection it will use.  (Another
         `forward` is given finished rows.)"""
-        return runs_plain(self.forward, GQAttention._plain_forward) and all(self._few_plan(n, r) is not None for r in (self.H * self.hd, (self.H + 2 * self.KV) * self.hd))
+        return (runs_plain(self, GQAttention._plain_forward) and self._few_plan(n, self.H * self.hd) is not None
+                and self._few_plan(n, (self.H + 2 * self.KV) * self.hd) is not None)
 
     # ---- the step
     accumulates = True        # forward(..., residual=x) may add the branch into the float32 stream and return None

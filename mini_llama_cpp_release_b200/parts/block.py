@@ -18,10 +18,10 @@ from ..config.specs import PartSpec
 from .base import MixerMemory, Part, TensorSpec
 
 
-def norm_into(norm, reader, x: torch.Tensor, pending: Optional[torch.Tensor]):
-    """The norm of the stream (which takes `pending` first) for the part that reads it; with nothing pending the reader's
-    product may form the norm itself."""
-    if pending is None and hasattr(norm, "into"):
+def norm_into(norm, reader, x: torch.Tensor, pending: Optional[torch.Tensor], n: int):
+    """The norm of the stream's n rows (which takes `pending` first) for the part that reads it; with nothing pending and few
+    rows the reader's product may form the norm itself."""
+    if n <= kernels.FEW_ROWS and pending is None and hasattr(norm, "into"):
         return norm.into(reader, x)
     return norm.forward(x, pending)
 
@@ -61,11 +61,11 @@ class PreNormBlock(Part):
         else:
             if left is not None:
                 left.finish()
-            h = norm_into(self.mixer_norm, mixer, x, pending)
+            h = norm_into(self.mixer_norm, mixer, x, pending, step.n_tokens)
         a = mixer.forward(h, step, memory, residual=x) if getattr(mixer, "accumulates", False) else mixer.forward(h, step, memory)
         if ffn is None:
             return x, a
-        h2 = norm_into(self.feed_forward_norm, ffn, x, a)
+        h2 = norm_into(self.feed_forward_norm, ffn, x, a, step.n_tokens)
         if getattr(ffn, "defers_sum", False) and not getattr(ffn, "identity", 0) and not getattr(ffn, "sum_is_plain", False):
             step.handover[DEFERRED] = DeferredBranch(x, expert_rows=ffn.forward(h2, step, deferred=True))
             return x, None

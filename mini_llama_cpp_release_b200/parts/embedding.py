@@ -82,7 +82,7 @@ class LinearHead(Part):
     def takes_normed_stream(self, n: int) -> bool:
         """Whether `forward` may be given a `NormedStream` of n rows.  (Another `forward`, and another product than `Linear` in
         `proj`, are given finished rows.)"""
-        return runs_plain(self.forward, LinearHead._plain_forward) and type(self.proj) is Linear and self.proj.few_plan(n) is not None
+        return runs_plain(self, LinearHead._plain_forward) and type(self.proj) is Linear and self.proj.few_plan(n) is not None
 
     def forward(self, h) -> torch.Tensor:
         h, gain, eps = normed_rows(h)

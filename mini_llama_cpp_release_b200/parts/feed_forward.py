@@ -62,11 +62,13 @@ class SwiGLU(Part):
     accumulates = True        # forward(..., residual=x) may add the branch into the float32 stream and return None
 
     def _few_plan(self, n: int):
-        return kernels.gemm_few_plan(n, 2 * self.inter, self.hidden, kernels.bindings.EPI_SILU_MUL, self.runtime.n_sms) if self.fused else None
+        if n > kernels.FEW_ROWS or not self.fused:       # (a prompt asks a few times a layer)
+            return None
+        return kernels.gemm_few_plan(n, 2 * self.inter, self.hidden, kernels.bindings.EPI_SILU_MUL, self.runtime.n_sms)
 
     def takes_normed_stream(self, n: int) -> bool:
         """Whether `forward` may be given a `NormedStream` of n rows.  (Another `forward` is given finished rows.)"""
-        return runs_plain(self.forward, SwiGLU._plain_forward) and self._few_plan(n) is not None
+        return runs_plain(self, SwiGLU._plain_forward) and self._few_plan(n) is not None
 
     def forward(self, h, step=None, residual=None):
         rt = self.runtime

@@ -74,7 +74,7 @@ class Linear:
 
     def few_plan(self, n_rows: int, epilogue: int = 0):
         """The plan of the few-row product (csrc/gemm_few.cu), or None where another kernel takes these rows."""
-        if not self.tensor_core_ok:
+        if n_rows > kernels.FEW_ROWS or not self.tensor_core_ok:
             return None
         return kernels.gemm_few_plan(n_rows, self.out_features, self.in_features, epilogue, self.runtime.n_sms)
 

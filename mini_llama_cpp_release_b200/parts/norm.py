@@ -30,10 +30,10 @@ def normed_rows(h):
     return (h.x, h.gain, h.eps) if isinstance(h, NormedStream) else (h, None, 0.0)
 
 
-def runs_plain(method, plain) -> bool:
-    """Whether the bound `method` is the function `plain` itself: not one that a subclass, the object or a later assignment to
-    the class put in its place."""
-    return getattr(method, "__func__", None) is plain
+def runs_plain(part, forward) -> bool:
+    """Whether the part's `forward` is this function: not one that a subclass, the object or a later assignment to the class
+    put in its place."""
+    return type(part).forward is forward and "forward" not in part.__dict__
 
 
 @register_part("norm", "rmsnorm")
@@ -75,7 +75,7 @@ class RMSNorm(Part):
         can form the norm itself (`takes_normed_stream`), and only the norm above: a norm whose `forward` is another one is asked for
         its output."""
         takes = getattr(reader, "takes_normed_stream", None)
-        if (takes is not None and self.runtime.dtype == torch.bfloat16 and runs_plain(self.forward, RMSNorm._plain_forward)
+        if (takes is not None and self.runtime.dtype == torch.bfloat16 and runs_plain(self, RMSNorm._plain_forward)
                 and takes(x.shape[0])):
             return NormedStream(x, self.gain, self.eps)
         return self.forward(x)

@@ -41,7 +41,7 @@ TAKES = SimpleNamespace(takes_normed_stream=lambda n: True)
 
 def test_the_plain_norm_is_left_to_a_reader_that_takes_it():
     x = torch.randn(4, 128)
-    h = norm_into(_norm(), TAKES, x, None)
+    h = norm_into(_norm(), TAKES, x, None, 4)
     assert isinstance(h, NormedStream) and h.x is x
 
 
@@ -51,17 +51,17 @@ def test_another_forward_is_called(monkeypatch):
     class Own(RMSNorm):
         def forward(self, x, delta=None, out_dtype=None):
             return marker
-    assert norm_into(_norm(Own), TAKES, x, None) is marker
+    assert norm_into(_norm(Own), TAKES, x, None, 4) is marker
 
     class OwnBelow(Own):
         pass
-    assert norm_into(_norm(OwnBelow), TAKES, x, None) is marker
+    assert norm_into(_norm(OwnBelow), TAKES, x, None, 4) is marker
     wrapped = _norm()
     wrapped.forward = lambda *a, **k: marker
-    assert norm_into(wrapped, TAKES, x, None) is marker
+    assert norm_into(wrapped, TAKES, x, None, 4) is marker
     plain = _norm()
     monkeypatch.setattr(RMSNorm, "forward", lambda self, *a, **k: marker)
-    assert norm_into(plain, TAKES, x, None) is marker
+    assert norm_into(plain, TAKES, x, None, 4) is marker
 
 
 def _readers():
