@@ -18,10 +18,10 @@ from ..config.specs import PartSpec
 from .base import MixerMemory, Part, TensorSpec
 
 
-def norm_into(norm, reader, x: torch.Tensor, pending: Optional[torch.Tensor], n: int):
-    """The norm of the stream's n rows (which takes `pending` first) for the part that reads it; with nothing pending and few
-    rows the reader's product may form the norm itself."""
-    if n <= kernels.FEW_ROWS and pending is None and hasattr(norm, "into"):
+def norm_into(norm, reader, x: torch.Tensor, pending: Optional[torch.Tensor], n: Optional[int] = None):
+    """The norm of the stream's rows (n of them, if the caller knows) which takes `pending` first, for the part that reads it;
+    with nothing pending and few rows the reader's product may form the norm itself."""
+    if pending is None and (x.shape[0] if n is None else n) <= kernels.FEW_ROWS and hasattr(norm, "into"):
         return norm.into(reader, x)
     return norm.forward(x, pending)
 

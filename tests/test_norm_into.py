@@ -41,7 +41,7 @@ TAKES = SimpleNamespace(takes_normed_stream=lambda n: True)
 
 def test_the_plain_norm_is_left_to_a_reader_that_takes_it():
     x = torch.randn(4, 128)
-    h = norm_into(_norm(), TAKES, x, None, 4)
+    h = norm_into(_norm(), TAKES, x, None)
     assert isinstance(h, NormedStream) and h.x is x
 
 
