@@ -21,7 +21,7 @@
 //                of the row's columns.
 // A block has one tile in flight per team and the scores of those after them: a team finds its next
 // scores complete when it has handed over its probabilities, and neither issuing thread waits for the other's
-// products (an issue costs its thread some 60 clocks and a barrier wait twice that, whatever the product's size).
+// products (a barrier wait costs its thread some 120 clocks, whatever the product's size).
 // Every barrier has one waiting thread, or a team's threads in step, and a waiter knows the phase before the one
 // it waits for to be complete: a parity wait cannot tell a phase from the one two before or after it.
 //
@@ -130,7 +130,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const unsigned tmem_slot = bar_base + 8u * (B_SF + 4 * A_AHEAD + 2);
     volatile unsigned* tmem_slot_ptr = reinterpret_cast<volatile unsigned*>(smem_generic + bar_off + 8 * (B_SF + 4 * A_AHEAD + 2));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < A_K_STAGES; ++s) {
             mbar_init(k_full(s), 1);
@@ -178,7 +178,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
     if (warp == 0) {
         // ---------------- TMA producer
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0 && elect_one()) {
             // a box is heads_per_block x tokens_per_block rows whatever part of it lies outside the tensor; rows of the
             // tile past the box are not written, and nothing reads their results
             mbar_expect_tx(q_full, (unsigned)(A_KB * a.heads_per_block * a.tokens_per_block * 128));
@@ -226,7 +226,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     } else if (warp == 1) {
         // ---------------- scores: S_j into buffer j mod A_AHEAD as soon as K_j has landed and the product that read the
         // buffer's last probabilities is complete; the commits hand S_j to its team and the K stage back to the loader
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0 && elect_one()) {
             constexpr unsigned idesc_s = umma_idesc(A_BN);
             bool ok = mbar_wait_polling(q_full, 0, a.status, 12);
             for (int j = 0; j < n_tiles && ok; ++j) {
@@ -252,7 +252,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // ---------------- outputs: the team's O += P_j V_j once V_j has landed and the team has written P_j (and rescaled
         // its output where needed); the commits tell that the tile's buffer is free for other scores and the team's O at
         // rest again, and hand the V stage back to the loader
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0 && elect_one()) {
             constexpr unsigned idesc_o = umma_idesc(A_HD, true);
             bool ok = true;
             for (int j = 0; j < n_tiles && ok; ++j) {

@@ -8,8 +8,8 @@
 // 128-byte swizzle span per row) through a ring of shared-memory stages:
 //     warp 0   one thread issues the TMA loads of the W tile and the activation tile;
 //     warp 1   allocates tensor memory, one thread issues tcgen05.mma and commits; for tiles of up to 32 tokens a
-//              thread of each of warps 2-4 issues too: the four take K steps in turn into accumulators of their own (an issue
-//              costs its thread about sixty clocks however small the product, and one thread's rate would bound the
+//              thread of each of warps 2-4 issues too: the four take K steps in turn into accumulators of their own (a wait on a stage's
+//              barrier costs its thread more than so small a product takes, and one thread's rate would bound the
 //              K loop);
 //     the next four warps (eight for tiles of 64 tokens and more) read the accumulators with tcgen05.ld (each warp its
 //              32 lanes), add the issuers' accumulators and run the epilogue.
@@ -81,9 +81,8 @@ template <int BN, int EPI> struct GemmShape {
     static constexpr int B_BYTES = BN * G_BK * 2;
     static constexpr int STAGE_BYTES = G_A_BYTES + B_BYTES;
     static constexpr int EPI_GROUPS = (BN >= 64) ? 2 : 1;            // epilogue warps: four per group, groups share out the tokens
-    // Threads that issue tcgen05.mma.  An issue costs the thread some sixty clocks and a wait on a stage's barrier twice
-    // that, whatever the size of the product: with few tokens (tiny products) one thread's issue rate, not the tensor
-    // cores, bounds the K loop.  Four threads then take K steps in turn, each into accumulators of its own; the epilogue
+    // Threads that issue tcgen05.mma.  A wait on a stage's barrier costs the thread some 120 clocks, whatever the size of the
+    // product: with few tokens (tiny products) one thread's issue rate, not the tensor cores, bounds the K loop.  Four threads then take K steps in turn, each into accumulators of its own; the epilogue
     // adds them.
     static constexpr int ISSUERS = (BN <= 32) ? 4 : 1;
     static constexpr int THREADS = 32 + 32 * ISSUERS + 128 * EPI_GROUPS;
@@ -170,7 +169,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     int* tok_pos = reinterpret_cast<int*>(smem_generic + bar_off + S::BAR_BYTES);                         // [BN]
     long long* tok_off = reinterpret_cast<long long*>(tok_pos + BN);                                      // [BN]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int n_tiles_total = g.m_tiles * g.n_tiles * g.n_splits;
     unsigned long long* const stamps = MLC_STAMPS_OR_NULL(g.timing == nullptr ? nullptr : g.timing + 8ull * blockIdx.x);
     if (stamps != nullptr && threadIdx.x == 0) stamps[0] = global_ns();                 // block start
@@ -214,7 +213,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (clustered) cluster_sync_all();       // every block's barriers exist before any block arrives on another's
         grid_dependency_wait();
         if (lane < early) tma_load_2d(b_base + lane * S::B_BYTES, &map_x, (c0.kb_begin + lane) * G_BK, c0.n0, full_bar(lane));
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < n_tiles_total && alive; t += gridDim.x) {
@@ -239,7 +238,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // ---------------- MMA issuers: tile j accumulates in buffer j % 2 (of each issuer) once the epilogue has emptied
         // it; issuer u takes the tile's K steps u, u + ISSUERS, ...
         if (clustered) cluster_sync_all();
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr unsigned idesc = umma_idesc(BN);
             const int u = warp - 1;
             int it = 0, j = 0;

@@ -74,7 +74,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const unsigned tmem_slot = bar_base + 8u * 28;
     volatile unsigned* tmem_slot_ptr = reinterpret_cast<volatile unsigned*>(smem_generic + bar_off + 8 * 28);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int n_tiles_total = g.m_tiles * g.n_tiles * g.n_splits;           // m_tiles counts tiles of 256 tokens
     auto tile_m0 = [&](int t) { return (t % g.m_tiles) * 2 * R_BM + (int)rank * R_BM; };             // this block's 128 tokens
@@ -108,7 +108,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (warp == 0) {
         // ---------------- TMA producer of this block: its 128 tokens and its BN/2 rows of W.  The first ring of W tiles
         // is requested before the wait for the kernels before this one, the token tiles after it.
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             bool alive = true;
             for (int t = pair; t < n_tiles_total && alive; t += n_pairs) {
@@ -137,7 +137,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     } else if (warp == 1 && rank == 1) {
         // ---------------- second block: every stage that has landed here is reported to the first block, whose
         // products read it: a second arrival on the first block's barrier of that stage
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             bool ok = true;
             unsigned remote[S::STAGES];
@@ -159,7 +159,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     } else if (warp == 1) {
         // ---------------- first block: the pair's products.  Tile j accumulates in buffer j % 2 of both blocks once
         // both epilogues have emptied it.
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr unsigned idesc = umma_idesc_pair(BN);
             int it = 0, j = 0;
             bool ok = true;

@@ -59,7 +59,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const unsigned tmem_slot = bar_base + 8u * 20;
     volatile unsigned* tmem_slot_ptr = reinterpret_cast<volatile unsigned*>(smem_generic + bar_off + 8 * 20);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int n_tiles_total = g.m_tiles * g.n_tiles * g.n_splits;
     // consecutive blocks take the token tiles of one W tile: the W tile is fetched from memory once and then found in L2
     auto tile_m0 = [&](int t) { return (t % g.m_tiles) * R_BM; };
@@ -94,7 +94,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (warp == 0) {
         // ---------------- TMA producer.  The weights do not depend on the kernels before this one: the first ring of W
         // tiles is requested before the wait for those kernels, the token tiles after it.
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             bool alive = true;
             if (grouped) grid_dependency_wait();
@@ -125,7 +125,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: tile j accumulates in buffer j % 2 once the epilogue has emptied it
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr unsigned idesc = umma_idesc(BN);
             int it = 0, j = 0;
             bool ok = true;
