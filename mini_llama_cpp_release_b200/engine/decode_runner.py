@@ -110,6 +110,10 @@ class DecodeRunner:
         end = self.offsets["sample_pos"][0] + B                     # tokens, positions, start_pos, sample_pos lie first
         self._copy_step_in = kernels.PinnedCopy(self.dev_buf[:end], self.host_buf[:end])
         self._copy_chosen_out = kernels.PinnedCopy(self.chosen_host, self.chosen_dev)
+        # the page tables likewise, one per group
+        areas = [slice(self.offsets[f"pages{g}"][0], sum(self.offsets[f"pages{g}"])) for g in range(n_groups)]
+        self._np_pages = [self.host_np[a].reshape(B, self.pages_per_seq) for a in areas]
+        self._copy_pages_in = [kernels.PinnedCopy(self.dev_buf[a], self.host_buf[a]) for a in areas]
         self._np_step = {n: self.host_np[self.offsets[n][0]:self.offsets[n][0] + B]
                          for n in ("tokens", "positions", "start_pos", "sample_pos")}
         self.sync_stream = torch.cuda.current_stream(dev)
@@ -200,32 +204,32 @@ class DecodeRunner:
         self.loaded_ids = list(seq_ids[:self.n_live])
         self._padded_slots = list(slots)
 
-    def _fill_pages(self, slots: Sequence[int]) -> None:
+    def _fill_pages(self, slots: Sequence[int], rows: Optional[Sequence[int]] = None) -> None:
+        """The page lists of `slots` into the host's tables (only those of `rows`, if given)."""
         P = self.pages_per_seq
-        for g in range(len(self.cache.groups)):
-            t = self.host_view(f"pages{g}").view(self.B, P)
-            for b, s in enumerate(slots):
-                pl = self.cache.page_lists[s][g]
+        for g, table in enumerate(self._np_pages):
+            for b in range(len(slots)) if rows is None else rows:
+                pl = self.cache.page_lists[slots[b]][g]
                 if len(pl) > P:
                     raise RuntimeError("decode runner: a sequence outgrew the runner's page table")
-                t[b, :len(pl)] = torch.tensor(pl, dtype=torch.int32)
-                t[b, len(pl):] = -1
+                table[b, :len(pl)] = pl
+                table[b, len(pl):] = -1
         self.page_versions = [self.cache.page_version[s] for s in slots]
 
     def refresh_pages(self, slots: Sequence[int]) -> int:
         """Copy the page tables again if any sequence's pages are not the ones copied last (it got or lost a page, or
-        its slot was given back and taken again by another sequence); returns bytes copied."""
+        its slot was given back and taken again by another sequence); returns bytes copied.  Only the rows that changed
+        are written anew: of 64 sequences of unequal lengths one gets a page at nearly every step, and the device stands idle
+        meanwhile."""
         version = self.cache.page_version
         slots = self._padded_slots
-        if self.page_versions == [version[s] for s in slots]:
+        rows = [b for b, s in enumerate(slots) if self.page_versions[b] != version[s]]
+        if not rows:
             return 0
-        self._fill_pages(slots)
-        n = 0
-        for g in range(len(self.cache.groups)):
-            o, cnt = self.offsets[f"pages{g}"]
-            self.dev_buf[o:o + cnt].copy_(self.host_buf[o:o + cnt], non_blocking=True)
-            n += cnt * 4
-        return n
+        self._fill_pages(slots, rows)
+        for copy in self._copy_pages_in:
+            copy()
+        return sum(copy.nbytes for copy in self._copy_pages_in)
 
     def load_step(self, tokens: Sequence[int], lengths: Sequence[int]) -> int:
         """The per-step inputs from the host: tokens and positions.  Returns bytes copied."""
