@@ -16,6 +16,7 @@ struct RowsArgs {
     int n_tok;
     int k_blocks;              // ceil(K / 64)
     int m_tiles, n_tiles;
+    int n_first;               // tiles of one token tile follow one another (1), or those of one tile of W's rows (0)
     int n_splits;              // blocks that share out a tile's K range (ADD only); 1: none
     int k_blocks_per_split;
     int* status;
@@ -72,10 +73,46 @@ __device__ __forceinline__ unsigned pack2(float a, float b) {
     return *reinterpret_cast<unsigned*>(&h);
 }
 
+// Tile number t of a product.  Consecutive blocks take tiles that share one operand's piece, which is then fetched from memory
+// once by all of them together, while the other operand is walked whole for each such piece: it comes from L2 if it fits there,
+// so it is the smaller one (n_first: W is).
+struct TileWalk {
+    int m, n, split;
+};
+__device__ __forceinline__ TileWalk tile_walk(const RowsArgs& g, int t) {
+    TileWalk w;
+    const int inner = g.n_first ? g.n_tiles : g.m_tiles, outer = g.n_first ? g.m_tiles : g.n_tiles;
+    const int i = t % inner, r = t / inner, o = r % outer;
+    w.m = g.n_first ? o : i;
+    w.n = g.n_first ? i : o;
+    w.split = r / outer;
+    return w;
+}
+
+// A warp's 32 tokens x 32 accumulator columns on their way into a float32 output through `buf`, 4 KiB of shared memory of
+// the warp's own: a thread writes its token's 128 bytes (16-byte pieces in the order of the 128-byte swizzle, so that eight
+// lanes hit all banks), one lane hands the tile to TMA.  ADD: added to what is there, a line at a time, where 16-byte atomic adds by
+// the threads themselves touch 32 lines an instruction.  B200, us, those adds with x walked whole, and this with the walk above:
+// 16,384 tokens 896 x 4,864 143, 119; 1,536 x 8,960 381, 320; 1,536 x 1,536 103, 76; 8,191 tokens 896 x 896 19.8, 16.2; 896 x 4,864 64.3,
+// 58.4; 2,048 tokens 896 x 896 7.5, 7.0; 1,536 x 8,960 42.3, 40.4.
+constexpr int R_OUT_BYTES = 32 * 32 * 4;
+template <int EPI>
+__device__ __forceinline__ void rows_tile_out(const CUtensorMap* map, const float (&v)[32], unsigned buf, int lane, int n, int tok0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 128 + ((u ^ (lane & 7)) << 4)), "f"(v[4 * u]),
+                     "f"(v[4 * u + 1]), "f"(v[4 * u + 2]), "f"(v[4 * u + 3]) : "memory");
+    fence_async_shared();
+    __syncwarp();
+    if (lane == 0) {
+        if (EPI == R_EPI_ADD) tma_add_2d(map, n, tok0, buf);
+        else tma_store_2d(map, n, tok0, buf);
+        tma_store_commit();
+    }
+}
+
 // One token's 32 (or, at the matrix's edge, 16) accumulator columns n .. n+31 leave the block.  `second`: the upper 16
-// exist too.  STORE: y as float32 or bfloat16; ADD: added into the float32 stream with 16-byte atomic adds (one
-// per element and launch unless the K range is shared out over blocks); SILU_MUL: columns alternate gate_j, up_j
-// and gate·sigmoid(gate)·up goes to [token][n/2].
+// exist too.  STORE: y as float32 or bfloat16; SILU_MUL: columns alternate gate_j, up_j and gate·sigmoid(gate)·up goes to [token][n/2].
 template <int EPI>
 __device__ __forceinline__ void rows_epilogue_chunk(const RowsArgs& g, const float (&vin)[32], int tok, int n, bool second) {
     float v[32];
@@ -96,11 +133,6 @@ __device__ __forceinline__ void rows_epilogue_chunk(const RowsArgs& g, const flo
             for (int u = 0; u < 8; ++u)
                 if (u < 4 || second) dst[u] = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
         }
-    } else if (EPI == R_EPI_ADD) {                    // a reduction that returns nothing: the thread does not wait for the old value
-        float4* dst = reinterpret_cast<float4*>((float*)g.out + (long long)tok * g.n_out + n);
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (u < 4 || second) atomicAdd(dst + u, make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]));
     } else {                                          // SILU_MUL: columns alternate gate_j, up_j
         float act[16];
         // the kind is tested once per chunk, outside the unrolled loops

@@ -20,15 +20,16 @@
 
 namespace mlc {
 
-template <int BN> struct PairShape {
+template <int BN, int EPI> struct PairShape {
     static constexpr int B_BYTES = (BN / 2) * R_BK * 2;              // this block's half of the W tile
     static constexpr int STAGE_BYTES = R_A_BYTES + B_BYTES;
-    static constexpr int STAGES_FIT = (227 * 1024 - 512 - 1024) / STAGE_BYTES;
+    static constexpr int OUT_BYTES = (EPI == R_EPI_ADD) ? 8 * 2 * R_OUT_BYTES : 0;       // two tiles on their way out per epilogue warp
+    static constexpr int STAGES_FIT = (227 * 1024 - 512 - 1024 - OUT_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_FIT < 7 ? STAGES_FIT : 7;
     static constexpr int THREADS = 64 + 256;
     static constexpr int TMEM_COLS = (2 * BN <= 256) ? 256 : 512;    // two accumulators of BN columns
     static constexpr int BAR_BYTES = 512;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024 /* alignment slack */;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES + BAR_BYTES + 1024 /* alignment slack */;
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a block");
     static_assert(BN % 32 == 0 && BN >= 128 && BN <= 256, "rows of W per tile");
     static_assert(STAGES >= 3 && STAGES <= 8, "stage ring");
@@ -56,16 +57,18 @@ __host__ __device__ constexpr unsigned umma_idesc_pair(int n) {
 }
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(PairShape<BN>::THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, RowsArgs g) {
-    using S = PairShape<BN>;
+__global__ void __launch_bounds__(PairShape<BN, EPI>::THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                 const __grid_constant__ CUtensorMap map_out, RowsArgs g) {
+    using S = PairShape<BN, EPI>;
     extern __shared__ unsigned char smem_dyn[];
     const unsigned rank = cluster_rank();                  // 0: the block that issues the pair's products
     const unsigned base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char* smem_generic = smem_dyn + (base - smem_u32(smem_dyn));
     const unsigned a_base = base;
     const unsigned b_base = base + S::STAGES * R_A_BYTES;
-    constexpr unsigned bar_off = S::STAGES * S::STAGE_BYTES;
+    constexpr unsigned out_off = S::STAGES * S::STAGE_BYTES;
+    constexpr unsigned bar_off = out_off + S::OUT_BYTES;
     const unsigned bar_base = base + bar_off;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };                // this block's stage has landed
     auto empty_bar = [&](int s) { return bar_base + 8u * (8 + s); };         // the pair's products have read the stage (both blocks)
@@ -77,10 +80,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     const int warp = warp_number(), lane = threadIdx.x & 31;
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int n_tiles_total = g.m_tiles * g.n_tiles * g.n_splits;           // m_tiles counts tiles of 256 tokens
-    auto tile_m0 = [&](int t) { return (t % g.m_tiles) * 2 * R_BM + (int)rank * R_BM; };             // this block's 128 tokens
-    auto tile_n0 = [&](int t) { return ((t / g.m_tiles) % g.n_tiles) * BN; };
-    auto tile_kb0 = [&](int t) { return (t / (g.m_tiles * g.n_tiles)) * g.k_blocks_per_split; };
-    auto tile_nkb = [&](int t) { return min(g.k_blocks, tile_kb0(t) + g.k_blocks_per_split) - tile_kb0(t); };
+    auto tile_nkb = [&](int t) {
+        const int kb0 = (t / (g.m_tiles * g.n_tiles)) * g.k_blocks_per_split;
+        return min(g.k_blocks, kb0 + g.k_blocks_per_split) - kb0;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) {
@@ -112,7 +115,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             int it = 0;
             bool alive = true;
             for (int t = pair; t < n_tiles_total && alive; t += n_pairs) {
-                const int m0 = tile_m0(t), w0 = tile_n0(t) + (int)rank * (BN / 2), kb0 = tile_kb0(t), n_kb = tile_nkb(t);
+                const TileWalk at = tile_walk(g, t);
+                const int m0 = (2 * at.m + (int)rank) * R_BM, w0 = at.n * BN + (int)rank * (BN / 2);     // this block's 128 tokens, its half of the W rows
+                const int kb0 = at.split * g.k_blocks_per_split, n_kb = tile_nkb(t);
                 int i = 0;
                 if (it == 0) {
                     const int early = min(n_kb, S::STAGES);
@@ -192,12 +197,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // tile's columns each
         const int q = warp & 3;
         const int eg = (warp - 2) >> 2;
-        constexpr int COLS_PER_GROUP = BN / 2;
+        constexpr bool WHOLE = EPI == R_EPI_ADD;                             // the groups take whole chunks of 32 columns
+        constexpr int COLS_PER_GROUP = WHOLE ? (BN / 32 + 1) / 2 * 32 : BN / 2;
+        const int cols = WHOLE ? min(COLS_PER_GROUP, BN - eg * COLS_PER_GROUP) : COLS_PER_GROUP;
         grid_dependency_wait();                // the output may come from earlier kernels
-        int j = 0;
+        const unsigned out_buf = base + out_off + (unsigned)((warp - 2) * 2 * R_OUT_BYTES);
+        int j = 0, n_out_tiles = 0;
         bool ok = true;
         for (int t = pair; t < n_tiles_total && ok; t += n_pairs, ++j) {
-            const int m0 = tile_m0(t), n0 = tile_n0(t);
+            const TileWalk at = tile_walk(g, t);
+            const int m0 = (2 * at.m + (int)rank) * R_BM, n0 = at.n * BN;
             const int buf = j & 1;
             const int tok = m0 + q * 32 + lane;
             const bool tok_ok = tok < g.n_tok;
@@ -207,14 +216,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const unsigned t_addr = tmem_base + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN + eg * COLS_PER_GROUP);
             const int col_base = n0 + eg * COLS_PER_GROUP;
 #pragma unroll 1
-            for (int c0 = 0; c0 < COLS_PER_GROUP; c0 += 32) {
+            for (int c0 = 0; c0 < cols; c0 += 32) {
                 const int n = col_base + c0;
                 if (n >= g.n_out) break;
                 float v[32];
                 tmem_load32(t_addr + (unsigned)c0, v);
-                const bool second = n + 16 < g.n_out && c0 + 32 <= COLS_PER_GROUP;
-                if (!tok_ok) continue;
-                rows_epilogue_chunk<EPI>(g, v, tok, n, second);
+                if constexpr (EPI == R_EPI_ADD) {
+                    if (m0 + q * 32 >= g.n_tok) break;
+                    // the buffer of two chunks before has been read (the warp's first lane asked for both copies)
+                    if (lane == 0) tma_store_wait_read<1>();
+                    __syncwarp();
+                    rows_tile_out<EPI>(&map_out, v, out_buf + (unsigned)((n_out_tiles++ & 1) * R_OUT_BYTES), lane, n, m0 + q * 32);
+                } else {
+                    const bool second = n + 16 < g.n_out && c0 + 32 <= COLS_PER_GROUP;
+                    if (!tok_ok) continue;
+                    rows_epilogue_chunk<EPI>(g, v, tok, n, second);
+                }
             }
             // the accumulator has been read here: once the other block's has been too, the tensor cores may fill it again
             tcgen05_fence_before();
@@ -224,6 +241,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 else mbar_arrive_remote(cluster_map(acc_empty_bar(buf), 0));
             }
         }
+        if (EPI == R_EPI_ADD && lane == 0) tma_store_wait<0>();
     }
 
     tcgen05_fence_before();
@@ -237,8 +255,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 }
 
 template <int BN, int EPI>
-static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const RowsArgs& g, int n_sms, cudaStream_t s) {
-    using S = PairShape<BN>;
+static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const RowsArgs& g, int n_sms, cudaStream_t s) {
+    using S = PairShape<BN, EPI>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
@@ -261,17 +279,17 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const RowsA
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, EPI>, mx, mw, g);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, EPI>, mx, mw, mo, g);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
 template <int EPI>
-static int dispatch_pair(int bn, const CUtensorMap& mx, const CUtensorMap& mw, const RowsArgs& g, int n_sms, cudaStream_t s) {
-    if (bn == 128) return launch_pair<128, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 160) return launch_pair<160, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 192) return launch_pair<192, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 224) return launch_pair<224, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 256) return launch_pair<256, EPI>(mx, mw, g, n_sms, s);
+static int dispatch_pair(int bn, const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const RowsArgs& g, int n_sms, cudaStream_t s) {
+    if (bn == 128) return launch_pair<128, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 160) return launch_pair<160, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 192) return launch_pair<192, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 224) return launch_pair<224, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 256) return launch_pair<256, EPI>(mx, mw, mo, g, n_sms, s);
     return MLC_ERR_BAD_SIZE;
 }
 
@@ -307,15 +325,18 @@ extern "C" int mlc_gemm_tcgen05_pair(const void* x, const void* w, void* out, in
     g.n_splits = n_splits;
     g.k_blocks_per_split = (g.k_blocks + n_splits - 1) / n_splits;
     if ((long long)(n_splits - 1) * g.k_blocks_per_split >= g.k_blocks) return MLC_ERR_BAD_SIZE;   // an empty split
+    g.n_first = n_tok > n_out;                 // x has more rows than W: see tile_walk
     g.status = status;
-    CUtensorMap mx, mw;
+    CUtensorMap mx, mw, mo;
     int rc = cached_map_2d(&mx, x, n_tok, K, R_BK, R_BM);
     if (rc) return rc;
     rc = cached_map_2d(&mw, w, n_out, K, R_BK, block_rows / 2);
     if (rc) return rc;
+    mo = mx;
+    if (epilogue == R_EPI_ADD && (rc = cached_map_2d(&mo, out, n_tok, n_out, 32, 32, true))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (epilogue == R_EPI_STORE) return dispatch_pair<R_EPI_STORE>(block_rows, mx, mw, g, n_sms, s);
-    if (epilogue == R_EPI_SILU_MUL) return dispatch_pair<R_EPI_SILU_MUL>(block_rows, mx, mw, g, n_sms, s);
-    if (epilogue == R_EPI_ADD) return dispatch_pair<R_EPI_ADD>(block_rows, mx, mw, g, n_sms, s);
+    if (epilogue == R_EPI_STORE) return dispatch_pair<R_EPI_STORE>(block_rows, mx, mw, mo, g, n_sms, s);
+    if (epilogue == R_EPI_SILU_MUL) return dispatch_pair<R_EPI_SILU_MUL>(block_rows, mx, mw, mo, g, n_sms, s);
+    if (epilogue == R_EPI_ADD) return dispatch_pair<R_EPI_ADD>(block_rows, mx, mw, mo, g, n_sms, s);
     return MLC_ERR_UNSUPPORTED;
 }

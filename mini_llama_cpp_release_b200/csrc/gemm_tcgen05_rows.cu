@@ -18,8 +18,8 @@
 //   QKV       rows of each head alternate dim i, dim i + hd/2: adds the bias, rotates q and k by the token's
 //             position (src/ops.cpp:125-141), writes q as [token][head][hd] and k, v into the token's place in
 //             the paged cache (src/forward.cpp:553);
-//   ADD       adds y into a float32 [token][row] tensor, the residual stream (src/forward.cpp:772, 779), with 16-byte
-//             atomic adds: nothing comes back, so a thread does not wait for the stream's old values, and the K
+//   ADD       adds y into a float32 [token][row] tensor, the residual stream (src/forward.cpp:772, 779), tile by tile with
+//             TMA's adding copies: nothing comes back, so nobody waits for the stream's old values, and the K
 //             range can be shared out over blocks (for products whose tiles alone would leave most SMs idle).
 //
 // Every wait on an mbarrier is bounded by a clock; a wait that runs out records a code in `status` (21 loader,
@@ -28,29 +28,32 @@
 
 namespace mlc {
 
-template <int BN> struct RowsShape {
+template <int BN, int EPI> struct RowsShape {
     static constexpr int B_BYTES = BN * R_BK * 2;
     static constexpr int STAGE_BYTES = R_A_BYTES + B_BYTES;
-    static constexpr int STAGES_FIT = (227 * 1024 - 256 - 1024) / STAGE_BYTES;
+    static constexpr int OUT_BYTES = (EPI == R_EPI_ADD) ? 8 * R_OUT_BYTES : 0;           // a tile on its way out per epilogue warp
+    static constexpr int STAGES_FIT = (227 * 1024 - 256 - 1024 - OUT_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_FIT < 6 ? STAGES_FIT : 6;
     static constexpr int THREADS = 64 + 256;
     static constexpr int TMEM_COLS = (2 * BN <= 256) ? 256 : 512;    // two accumulators of BN columns; allocations are powers of two
     static constexpr int BAR_BYTES = 256;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024 /* alignment slack */;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES + BAR_BYTES + 1024 /* alignment slack */;
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a block");
     static_assert(BN % 32 == 0 && BN >= 128 && BN <= 256, "rows of W per tile");
 };
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(RowsShape<BN>::THREADS, 1)
-gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, RowsArgs g) {
-    using S = RowsShape<BN>;
+__global__ void __launch_bounds__(RowsShape<BN, EPI>::THREADS, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                 const __grid_constant__ CUtensorMap map_out, RowsArgs g) {
+    using S = RowsShape<BN, EPI>;
     extern __shared__ unsigned char smem_dyn[];
     const unsigned base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char* smem_generic = smem_dyn + (base - smem_u32(smem_dyn));
     const unsigned a_base = base;
     const unsigned b_base = base + S::STAGES * R_A_BYTES;
-    constexpr unsigned bar_off = S::STAGES * S::STAGE_BYTES;
+    constexpr unsigned out_off = S::STAGES * S::STAGE_BYTES;
+    constexpr unsigned bar_off = out_off + S::OUT_BYTES;
     const unsigned bar_base = base + bar_off;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (8 + s); };
@@ -61,14 +64,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 
     const int warp = warp_number(), lane = threadIdx.x & 31;
     const int n_tiles_total = g.m_tiles * g.n_tiles * g.n_splits;
-    // consecutive blocks take the token tiles of one W tile: the W tile is fetched from memory once and then found in L2
-    auto tile_m0 = [&](int t) { return (t % g.m_tiles) * R_BM; };
-    auto tile_n0 = [&](int t) { return ((t / g.m_tiles) % g.n_tiles) * BN; };
-    auto tile_kb0 = [&](int t) { return (t / (g.m_tiles * g.n_tiles)) * g.k_blocks_per_split; };       // first K block of the tile's share
-    auto tile_nkb = [&](int t) { return min(g.k_blocks, tile_kb0(t) + g.k_blocks_per_split) - tile_kb0(t); };
+    auto tile_nkb = [&](int t) {
+        const int kb0 = (t / (g.m_tiles * g.n_tiles)) * g.k_blocks_per_split;
+        return min(g.k_blocks, kb0 + g.k_blocks_per_split) - kb0;
+    };
     const bool grouped = g.tile_group != nullptr;
     // the group of tile t's tokens (0 when the product is not grouped); a negative group: no role touches the tile
-    auto tile_grp = [&](int t) { return grouped ? __ldg(g.tile_group + t % g.m_tiles) : 0; };
+    auto tile_grp = [&](int t) { return grouped ? __ldg(g.tile_group + t % g.m_tiles) : 0; };       // (grouped products walk with n_first 0)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) {
@@ -101,7 +103,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             for (int t = blockIdx.x; t < n_tiles_total && alive; t += gridDim.x) {
                 const int grp = tile_grp(t);
                 if (grp < 0) continue;
-                const int m0 = tile_m0(t), n0 = tile_n0(t) + grp * g.n_out, kb0 = tile_kb0(t), n_kb = tile_nkb(t);
+                const TileWalk at = tile_walk(g, t);
+                const int m0 = at.m * R_BM, n0 = at.n * BN + grp * g.n_out, kb0 = at.split * g.k_blocks_per_split, n_kb = tile_nkb(t);
                 int i = 0;
                 if (it == 0 && !grouped) {
                     const int early = min(n_kb, S::STAGES);
@@ -160,13 +163,17 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // ---------------- epilogue: a thread is one token; the two groups of warps take half of the tile's columns each
         const int q = warp & 3;
         const int eg = (warp - 2) >> 2;
-        constexpr int COLS_PER_GROUP = BN / 2;
+        constexpr bool WHOLE = EPI == R_EPI_ADD;                             // the groups take whole chunks of 32 columns
+        constexpr int COLS_PER_GROUP = WHOLE ? (BN / 32 + 1) / 2 * 32 : BN / 2;
+        const int cols = WHOLE ? min(COLS_PER_GROUP, BN - eg * COLS_PER_GROUP) : COLS_PER_GROUP;
+        const unsigned out_buf = base + out_off + (unsigned)((warp - 2) * R_OUT_BYTES);
         grid_dependency_wait();                // positions, page lists and the output may come from earlier kernels
         int j = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < n_tiles_total && ok; t += gridDim.x) {
             if (tile_grp(t) < 0) continue;
-            const int m0 = tile_m0(t), n0 = tile_n0(t);
+            const TileWalk at = tile_walk(g, t);
+            const int m0 = at.m * R_BM, n0 = at.n * BN;
             const int buf = j & 1;
             const int tok = m0 + q * 32 + lane;
             const bool tok_ok = tok < g.n_tok;
@@ -241,11 +248,18 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
             } else {
 #pragma unroll 1
-                for (int c0 = 0; c0 < COLS_PER_GROUP; c0 += 32) {
+                for (int c0 = 0; c0 < cols; c0 += 32) {
                     const int n = col_base + c0;
                     if (n >= g.n_out) break;
                     float v[32];
                     tmem_load32(t_addr + (unsigned)c0, v);
+                    if constexpr (EPI == R_EPI_ADD) {
+                        if (m0 + q * 32 >= g.n_tok) break;
+                        if (lane == 0) tma_store_wait_read<0>();       // the warp's tile before has been read
+                        __syncwarp();
+                        rows_tile_out<EPI>(&map_out, v, out_buf, lane, n, m0 + q * 32);
+                        continue;
+                    }
                     // n_out and the group's share of the tile are multiples of 16: the chunk has 16 or 32 columns
                     const bool second = n + 16 < g.n_out && c0 + 32 <= COLS_PER_GROUP;
                     if (!tok_ok) continue;
@@ -257,6 +271,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_arrive(acc_empty_bar(buf));
             ++j;
         }
+        if (EPI == R_EPI_ADD && lane == 0) tma_store_wait<0>();
     }
 
     tcgen05_fence_before();
@@ -272,8 +287,8 @@ static int rows_map(CUtensorMap* map, const void* ptr, long long rows, long long
 }
 
 template <int BN, int EPI>
-static int launch_rows(const CUtensorMap& mx, const CUtensorMap& mw, const RowsArgs& g, int n_sms, cudaStream_t s) {
-    using S = RowsShape<BN>;
+static int launch_rows(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const RowsArgs& g, int n_sms, cudaStream_t s) {
+    using S = RowsShape<BN, EPI>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
@@ -282,17 +297,17 @@ static int launch_rows(const CUtensorMap& mx, const CUtensorMap& mw, const RowsA
     }
     const long long tiles = (long long)g.m_tiles * g.n_tiles * g.n_splits;
     const unsigned blocks = (unsigned)(tiles < n_sms ? tiles : n_sms);
-    cudaError_t e = launch_pdl(gemm_rows_kernel<BN, EPI>, dim3(blocks), dim3(S::THREADS), (size_t)S::SMEM_BYTES, s, mx, mw, g);
+    cudaError_t e = launch_pdl(gemm_rows_kernel<BN, EPI>, dim3(blocks), dim3(S::THREADS), (size_t)S::SMEM_BYTES, s, mx, mw, mo, g);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
 template <int EPI>
-static int dispatch_rows(int bn, const CUtensorMap& mx, const CUtensorMap& mw, const RowsArgs& g, int n_sms, cudaStream_t s) {
-    if (bn == 128) return launch_rows<128, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 160) return launch_rows<160, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 192) return launch_rows<192, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 224) return launch_rows<224, EPI>(mx, mw, g, n_sms, s);
-    if (bn == 256) return launch_rows<256, EPI>(mx, mw, g, n_sms, s);
+static int dispatch_rows(int bn, const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo, const RowsArgs& g, int n_sms, cudaStream_t s) {
+    if (bn == 128) return launch_rows<128, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 160) return launch_rows<160, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 192) return launch_rows<192, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 224) return launch_rows<224, EPI>(mx, mw, mo, g, n_sms, s);
+    if (bn == 256) return launch_rows<256, EPI>(mx, mw, mo, g, n_sms, s);
     return MLC_ERR_BAD_SIZE;
 }
 
@@ -332,6 +347,7 @@ extern "C" int mlc_gemm_tcgen05_rows(const void* x, const void* w, void* out, in
     g.n_splits = n_splits;
     g.k_blocks_per_split = (g.k_blocks + n_splits - 1) / n_splits;
     if ((long long)(n_splits - 1) * g.k_blocks_per_split >= g.k_blocks) return MLC_ERR_BAD_SIZE;   // an empty split
+    g.n_first = n_tok > n_out;                 // x has more rows than W: see tile_walk
     g.status = status;
     if (epilogue == R_EPI_QKV) {
         if (out_dtype != MLC_DTYPE_BF16) return MLC_ERR_BAD_DTYPE;
@@ -354,10 +370,12 @@ extern "C" int mlc_gemm_tcgen05_rows(const void* x, const void* w, void* out, in
     rc = rows_map(&mw, w, n_out, K, block_rows);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (epilogue == R_EPI_STORE) return dispatch_rows<R_EPI_STORE>(block_rows, mx, mw, g, n_sms, s);
-    if (epilogue == R_EPI_SILU_MUL) return dispatch_rows<R_EPI_SILU_MUL>(block_rows, mx, mw, g, n_sms, s);
-    if (epilogue == R_EPI_QKV) return block_rows == 128 ? launch_rows<128, R_EPI_QKV>(mx, mw, g, n_sms, s) : MLC_ERR_BAD_SIZE;
-    if (epilogue == R_EPI_ADD) return dispatch_rows<R_EPI_ADD>(block_rows, mx, mw, g, n_sms, s);
+    if (epilogue == R_EPI_STORE) return dispatch_rows<R_EPI_STORE>(block_rows, mx, mw, mx, g, n_sms, s);
+    if (epilogue == R_EPI_SILU_MUL) return dispatch_rows<R_EPI_SILU_MUL>(block_rows, mx, mw, mx, g, n_sms, s);
+    if (epilogue == R_EPI_QKV) return block_rows == 128 ? launch_rows<128, R_EPI_QKV>(mx, mw, mx, g, n_sms, s) : MLC_ERR_BAD_SIZE;
+    CUtensorMap mo;
+    if (epilogue == R_EPI_ADD && (rc = cached_map_2d(&mo, out, n_tok, n_out, 32, 32, true))) return rc;
+    if (epilogue == R_EPI_ADD) return dispatch_rows<R_EPI_ADD>(block_rows, mx, mw, mo, g, n_sms, s);
     return MLC_ERR_UNSUPPORTED;
 }
 
@@ -400,6 +418,6 @@ extern "C" int mlc_gemm_tcgen05_rows_grouped(const void* x, const void* w, void*
     rc = rows_map(&mw, w, (long long)n_groups * n_out, K, block_rows);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (epilogue == R_EPI_STORE) return dispatch_rows<R_EPI_STORE>(block_rows, mx, mw, g, n_sms, s);
-    return dispatch_rows<R_EPI_SILU_MUL>(block_rows, mx, mw, g, n_sms, s);
+    if (epilogue == R_EPI_STORE) return dispatch_rows<R_EPI_STORE>(block_rows, mx, mw, mx, g, n_sms, s);
+    return dispatch_rows<R_EPI_SILU_MUL>(block_rows, mx, mw, mx, g, n_sms, s);
 }

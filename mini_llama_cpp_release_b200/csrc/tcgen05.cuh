@@ -115,6 +115,21 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
+// A tile in shared memory leaves for a tensor in global memory, stored or (float32) added to what is there; what lies outside
+// the tensor is left out.  Copies are asked for and waited for by one thread, in groups.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int c0, int c1, unsigned src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(map), "r"(c0), "r"(c1), "r"(src) : "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, int c0, int c1, unsigned src) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(map), "r"(c0), "r"(c1), "r"(src) : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// All but the latest N groups have read their shared memory / are complete.
+template <int N> __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+template <int N> __device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
+
 __device__ __forceinline__ void tcgen05_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -265,41 +280,42 @@ static PFN_cuTensorMapEncodeTiled encode_tiled() {
     return fn;
 }
 
-// A bfloat16 tensor of `rank` dimensions (innermost first; strides in bytes for dimensions 1...) read in boxes
-// whose innermost extent is 64 elements, with the 128-byte swizzle; reads outside the tensor give zeros.
+// A tensor of `rank` dimensions (innermost first; strides in bytes for dimensions 1...) read or written in boxes whose
+// innermost extent is 128 bytes, with the 128-byte swizzle; reads outside the tensor give zeros.
 static int make_tensor_map(CUtensorMap* map, const void* ptr, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
-                           const cuuint32_t* box) {
+                           const cuuint32_t* box, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
     PFN_cuTensorMapEncodeTiled fn = encode_tiled();
     if (fn == nullptr) return MLC_ERR_UNSUPPORTED;
     cuuint32_t elem[5] = {1, 1, 1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(ptr), dims, strides, box, elem,
+    CUresult r = fn(map, type, (cuuint32_t)rank, const_cast<void*>(ptr), dims, strides, box, elem,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : MLC_ERR_BAD_SIZE;
 }
 
-// The map of a row-major bfloat16 matrix [rows][cols] read in boxes of box_rows x box_cols, remembered by what defines
+// The map of a row-major matrix [rows][cols] (bfloat16, or float32) read or written in boxes of box_rows x box_cols, remembered by what defines
 // it: a step launches hundreds of products over the same weights, and its scratch tensors come back at the same
 // addresses step after step, so the driver is asked once per matrix, not once per launch.
-static int cached_map_2d(CUtensorMap* map, const void* ptr, long long rows, long long cols, int box_cols, int box_rows) {
+static int cached_map_2d(CUtensorMap* map, const void* ptr, long long rows, long long cols, int box_cols, int box_rows, bool f32 = false) {
     struct Key {
         const void* ptr;
         long long rows, cols;
         int box_cols, box_rows;
+        bool f32;
         bool operator==(const Key& o) const {
-            return ptr == o.ptr && rows == o.rows && cols == o.cols && box_cols == o.box_cols && box_rows == o.box_rows;
+            return ptr == o.ptr && rows == o.rows && cols == o.cols && box_cols == o.box_cols && box_rows == o.box_rows && f32 == o.f32;
         }
     };
     struct Hash {
         size_t operator()(const Key& k) const {
             size_t h = std::hash<const void*>()(k.ptr);
             h = h * 1000003u ^ std::hash<long long>()(k.rows * 131 + k.cols);
-            return h * 1000003u ^ std::hash<int>()(k.box_cols * 1024 + k.box_rows);
+            return h * 1000003u ^ std::hash<int>()((k.box_cols * 1024 + k.box_rows) * 2 + k.f32);
         }
     };
     static std::unordered_map<Key, CUtensorMap, Hash> cache;
     static std::mutex lock;
-    const Key key{ptr, rows, cols, box_cols, box_rows};
+    const Key key{ptr, rows, cols, box_cols, box_rows, f32};
     {
         std::lock_guard<std::mutex> guard(lock);
         auto it = cache.find(key);
@@ -309,9 +325,9 @@ static int cached_map_2d(CUtensorMap* map, const void* ptr, long long rows, long
         }
     }
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * (f32 ? 4 : 2)};
     cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-    const int rc = make_tensor_map(map, ptr, 2, dims, strides, box);
+    const int rc = make_tensor_map(map, ptr, 2, dims, strides, box, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
     if (rc == 0) {
         std::lock_guard<std::mutex> guard(lock);
         if (cache.size() > 8192) cache.clear();

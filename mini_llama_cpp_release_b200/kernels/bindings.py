@@ -1458,10 +1458,11 @@ def gemm_prompt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
 
 
 # What an adding prompt product costs in microseconds, by form: a launch, per K step a part that grows with the tile's
-# width and one that does not, per tile the write-out, and per megabyte of 16-byte atomic adds what the L2 takes for
-# them.  Fitted (12 % rms) to 600 measurements on a B200: 512, 2,048 and 8,192 tokens, nine weight shapes from
-# 896 x 896 to 4,096 x 11,008, every width and split below; the plan it picks is the fastest measured one in half of
-# the 27 cases and within 4 % of it in all but four (at most 9 %).
+# width and one that does not, per tile the write-out, and per megabyte of adds what the L2 takes for them.  Fitted (12 % rms) to 600 measurements on a B200: 512, 2,048 and 8,192 tokens, nine weight shapes from
+# 896 x 896 to 4,096 x 11,008, every width and split below; the plan it picks was the fastest measured one in half of
+# the 27 cases.  Since then the adds leave by TMA and cost half of what the constants say, but the choice holds: over 34 cases of 100 to
+# 16,384 tokens it is 1.2 % slower than the fastest on average, at most 7 % (4,088 tokens 896 x 4,864: 30.2 against 28.1 us);
+# constants fitted anew choose worse (2.2 %, at most 12 %).
 _ADD_COST = {"rows": (128, 1, 2.34, 0.00090, 0.183, 2.19, 0.372),
              "pair": (256, 2, 3.41, 0.00061, 0.219, 2.24, 0.360)}
 _ADD_WIDTHS = {"rows": (128, 160, 192, 224, 256), "pair": (192, 224, 256)}
@@ -1514,7 +1515,7 @@ def gemm_tcgen05_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilo
                       kv: Optional[KVView] = None, n_sms: int = 0, glu=None) -> None:
     """The tcgen05 product for prompts (csrc/gemm_tcgen05_rows.cu): bfloat16 x [n, K] times bfloat16 w [rows, K]
     transposed, tiles of 128 tokens x `block_rows` (128 to 256 in steps of 32) rows of w, the same epilogues as `gemm_tcgen05`;
-    EPI_ADD adds into `out` (float32 [n, rows]) with 16-byte atomic adds, the K range shared out over `n_splits` blocks per
+    EPI_ADD adds into `out` (float32 [n, rows]) with TMA's adding copies, the K range shared out over `n_splits` blocks per
     tile (the plan's choice if neither tile width nor splits are given)."""
     require_cuda(x, w, out, bias, positions, tok_seq, rope)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
