@@ -351,19 +351,25 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             m = m_new;
 
             // probabilities, their sum, P as pairs of bfloat16 over the first half of the scores' columns
-            float ls4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            // (two keys an instruction where there is one: prompts of 8,191 tokens, 14 heads of 64, 179 -> 169 us)
+            float2x sum[2] = {pair_of(0.0f, 0.0f), pair_of(0.0f, 0.0f)};
+            const float2x scale2 = pair_of(a.scale_log2, a.scale_log2), shift2 = pair_of(-m_use, -m_use);
             unsigned pk[A_BN / 2];
 #pragma unroll
             for (int c = 0; c < A_BN / 2; ++c) {
-                const float p0 = fast_exp2(fmaf(sc[2 * c], a.scale_log2, -m_use));
-                const float p1 = fast_exp2(fmaf(sc[2 * c + 1], a.scale_log2, -m_use));
-                ls4[(2 * c) & 3] += p0;
-                ls4[(2 * c + 1) & 3] += p1;
+                float p0, p1;
+                unpair(pair_fma(pair_of(sc[2 * c], sc[2 * c + 1]), scale2, shift2), p0, p1);
+                p0 = fast_exp2(p0);
+                p1 = fast_exp2(p1);
+                sum[c & 1] = pair_add(sum[c & 1], pair_of(p0, p1));
                 __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);        // key 2c in the low half
                 pk[c] = *reinterpret_cast<unsigned*>(&hh);
             }
             tmem_store32_words(s_taddr, pk);
-            l = l * corr + ((ls4[0] + ls4[1]) + (ls4[2] + ls4[3]));
+            float s0, s1, s2, s3;
+            unpair(sum[0], s0, s1);
+            unpair(sum[1], s2, s3);
+            l = l * corr + ((s0 + s1) + (s2 + s3));
             MLC_PHASE(2)                                   // exponentials, writing P
 
             if (j == n_tiles - 1 && key0 + A_BN - 1 > seq_last) {
