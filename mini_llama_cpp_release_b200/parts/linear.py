@@ -5,7 +5,7 @@ Which kernel runs is decided by the operand types and sizes, never by the model:
   * any float32 operand (the whole 32-bit path, or a tensor the checkpoint stores in
     32-bit while the engine computes in bfloat16): the float32 multiply-add kernel of
     csrc/linear_simt.cu.  No tensor-core mode takes part.
-  * bfloat16 × bfloat16 of up to 32 rows, with an inner size that is a multiple of 64 and where
+  * bfloat16 × bfloat16 of up to 32 rows (16 where the product adds into the stream), with an inner size that is a multiple of 64 and where
     `kernels.gemm_few_plan` has a plan (by rows, sizes and epilogue): the few-row product of
     csrc/gemm_few.cu, which also forms the RMS norm of its input on the way where a part may leave it
     to it (`of_norm`).
@@ -36,6 +36,12 @@ SMALL_BATCH = 64          # up to this many rows a plain product runs on the tcg
 MAX_SPLITS = 8            # partial sums the consumer has to add
 ADD_MAX_SPLITS = 24       # splits of a product that adds into the stream atomically (nobody has to add them up)
 ADD_MAX_SPLITS_SOME = 10  # the same for 2 to 16 rows
+ADD_MAX_SPLITS_MORE = 12  # the same for 17 to 64 rows
+# Rows up to which an adding product takes the few-row form where that has a plan.  B200, us in a chain, few-row form and tcgen05 form with
+# its splits: 896 x 4,864 17 rows 3.51, 3.47, 24 rows 3.84, 3.52, 32 rows 4.36, 3.56; 896 x 896 2.47, 2.38; 2.64, 2.47; 2.91, 2.49; 1,536 x
+# 1,536 3.03, 2.90; 3.35, 2.92; 3.54, 2.99; below, 8 rows, 2.67, 3.15; 1.53, 2.15; 1.75, 2.54.  Requests of 20 prompts of 100 tokens with 24
+# tokens each (0.5B sizes) 19.1 -> 18.0 ms, of 30 (1.5B sizes) 35.8 -> 35.6.
+ADD_FEW_ROWS = 16
 
 
 def add_split_cap(n_tok: int) -> int:
@@ -44,8 +50,11 @@ def add_split_cap(n_tok: int) -> int:
     the kernel after it cannot start early to ask for its own weights.  Measured on whole decode steps of 24 and 28
     layers on a B200, caps of 8 / 10 / 12 / 24: 0.733 / 0.710 / 0.717 / 0.722 ms at 8 rows and 1.271 against 1.300 ms
     (10 against 24) at 16 rows of the Qwen2-1.5B sizes, but 0.735 / 0.703 / 0.704 / 0.683 ms at one row and
-    1.039 / 1.044 / 1.016 / 1.009 ms at 64 rows; at the 7B sizes the cap does not bind."""
-    return ADD_MAX_SPLITS_SOME if 2 <= n_tok <= 16 else ADD_MAX_SPLITS
+    1.039 / 1.044 / 1.016 / 1.009 ms at 64 rows; at the 7B sizes the cap does not bind.  With issues through elect.sync (us in a
+    chain, 64 rows): 896 x 4,864 3.60 with 10 splits, 3.84 with 19; 1,536 x 8,960 6.81 with 10, 6.51 with 12, 6.71 with 24."""
+    if n_tok < 2:
+        return ADD_MAX_SPLITS
+    return ADD_MAX_SPLITS_SOME if n_tok <= 16 else ADD_MAX_SPLITS_MORE
 
 
 def split_count(n_out: int, k: int, n_tok: int, n_sms: int, max_splits: int = 0) -> int:
@@ -102,7 +111,7 @@ class Linear:
         if m > SMALL_BATCH:
             kernels.library_gemm(x, self.weight, stream, accumulate=True)
             return
-        if (plan := self.few_plan(m, kernels.bindings.EPI_ADD)) is not None:
+        if m <= ADD_FEW_ROWS and (plan := self.few_plan(m, kernels.bindings.EPI_ADD)) is not None:
             kernels.gemm_few(x, self.weight, stream, kernels.bindings.EPI_ADD, plan)
             return
         splits = split_count(self.out_features, self.in_features, m, self.runtime.n_sms, max_splits=add_split_cap(m))
