@@ -5,7 +5,7 @@ Which kernel runs is decided by the operand types and sizes, never by the model:
   * any float32 operand (the whole 32-bit path, or a tensor the checkpoint stores in
     32-bit while the engine computes in bfloat16): the float32 multiply-add kernel of
     csrc/linear_simt.cu.  No tensor-core mode takes part.
-  * bfloat16 × bfloat16 of up to 32 rows (16 where the product adds into the stream), with an inner size that is a multiple of 64 and where
+  * bfloat16 × bfloat16 of up to 32 rows, with an inner size that is a multiple of 64 and where
     `kernels.gemm_few_plan` has a plan (by rows, sizes and epilogue): the few-row product of
     csrc/gemm_few.cu, which also forms the RMS norm of its input on the way where a part may leave it
     to it (`of_norm`).
@@ -37,11 +37,6 @@ MAX_SPLITS = 8            # partial sums the consumer has to add
 ADD_MAX_SPLITS = 24       # splits of a product that adds into the stream atomically (nobody has to add them up)
 ADD_MAX_SPLITS_SOME = 10  # the same for 2 to 16 rows
 ADD_MAX_SPLITS_MORE = 12  # the same for 17 to 64 rows
-# Rows up to which an adding product takes the few-row form where that has a plan.  B200, us in a chain, few-row form and tcgen05 form with
-# its splits: 896 x 4,864 17 rows 3.51, 3.47, 24 rows 3.84, 3.52, 32 rows 4.36, 3.56; 896 x 896 2.47, 2.38; 2.64, 2.47; 2.91, 2.49; 1,536 x
-# 1,536 3.03, 2.90; 3.35, 2.92; 3.54, 2.99; below, 8 rows, 2.67, 3.15; 1.53, 2.15; 1.75, 2.54.  Requests of 20 prompts of 100 tokens with 24
-# tokens each (0.5B sizes) 19.1 -> 18.0 ms, of 30 (1.5B sizes) 35.8 -> 35.6.
-ADD_FEW_ROWS = 16
 
 
 def add_split_cap(n_tok: int) -> int:
@@ -111,7 +106,7 @@ class Linear:
         if m > SMALL_BATCH:
             kernels.library_gemm(x, self.weight, stream, accumulate=True)
             return
-        if m <= ADD_FEW_ROWS and (plan := self.few_plan(m, kernels.bindings.EPI_ADD)) is not None:
+        if (plan := self.few_plan(m, kernels.bindings.EPI_ADD)) is not None:
             kernels.gemm_few(x, self.weight, stream, kernels.bindings.EPI_ADD, plan)
             return
         splits = split_count(self.out_features, self.in_features, m, self.runtime.n_sms, max_splits=add_split_cap(m))

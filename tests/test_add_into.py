@@ -1,0 +1,60 @@
+"""A product that adds into the stream (parts/linear.py: Linear.add_into): which kernel takes which rows, and what comes out on both sides of
+every line between them."""
+import pytest
+import torch
+
+from mini_llama_cpp_release_b200 import kernels
+from mini_llama_cpp_release_b200.parts import linear
+
+
+class _Runtime:
+    n_sms = 148
+
+
+def route(monkeypatch, n_tok, n_out, k):
+    """("few" or "tcgen05", blocks that share the K range), without launching anything."""
+    seen = []
+    monkeypatch.setattr(kernels, "gemm_few", lambda x, w, out, epilogue, plan, *a, **kw: seen.append(("few", plan[4])))
+    monkeypatch.setattr(kernels, "gemm_tcgen05", lambda x, w, out, epilogue, n_splits=1, *a, **kw: seen.append(("tcgen05", n_splits)))
+    layer = linear.Linear(torch.empty(n_out, k, dtype=torch.bfloat16), _Runtime())
+    layer.add_into(torch.empty(n_tok, k, dtype=torch.bfloat16), torch.empty(n_tok, n_out))
+    assert len(seen) == 1
+    return seen[0]
+
+
+@pytest.mark.parametrize("n_out,k", [(512, 512), (640, 640), (1024, 256), (1536, 768), (2048, 832), (1024, 448)])
+def test_a_whole_inner_size_is_added_by_one_block(monkeypatch, n_out, k):
+    """17 to 32 rows: one plain add per element, so that the same bits come out every time."""
+    for n_tok in (16, 17, 24):
+        assert route(monkeypatch, n_tok, n_out, k) == ("few", 1), n_tok
+
+
+def test_larger_products_leave_the_few_row_form_at_17_rows(monkeypatch):
+    for n_out, k in ((896, 896), (896, 4864), (1536, 1536)):
+        assert route(monkeypatch, 16, n_out, k)[0] == "few"
+        for n_tok in (17, 32, 33, 64):
+            assert route(monkeypatch, n_tok, n_out, k)[0] == "tcgen05"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_out,k", [(512, 512), (896, 896), (896, 4864), (208, 1000), (130, 1024), (1536, 768)])
+@pytest.mark.parametrize("n_tok", [1, 16, 17, 24, 32, 33, 63, 64, 65])
+def test_added_products_on_both_sides_of_the_lines(n_tok, n_out, k):
+    """Against float64: sums of K products of 16-bit numbers in float32, each partial sum rounded by 2^-24 (3e-6 of the largest output, as
+    for the kernels by themselves); a row beyond the output stays as it was; products that one block adds repeat bit for bit."""
+    g = torch.Generator().manual_seed(n_tok + n_out + k)
+    x = (torch.randn(n_tok, k, generator=g) * 0.5).bfloat16().cuda()
+    layer = linear.Linear((torch.randn(n_out, k, generator=g) * 0.3).bfloat16().cuda(), _Runtime())
+    before = torch.randn(n_tok + 1, n_out, generator=g).cuda()
+    want = before[:n_tok].double() + x.double() @ layer.weight.double().T
+    plan = layer.few_plan(n_tok, kernels.bindings.EPI_ADD)
+    outs = []
+    for _ in range(4):
+        stream = before.clone()
+        layer.add_into(x, stream[:n_tok])
+        outs.append(stream)
+        assert float((stream[:n_tok].double() - want).abs().max()) <= 3e-6 * float(want.abs().max())
+        assert torch.equal(stream[n_tok], before[n_tok])
+    if plan is not None and plan[4] == 1:
+        assert all(torch.equal(o, outs[0]) for o in outs[1:])
+    kernels.check_gemm_status(torch.device("cuda"))
