@@ -1627,8 +1627,10 @@ def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> 
                18,944 25.5 against 24.0: not above 40 M weights, and 4,096 x 4,096 7.9 against 7.5: not above 16 M where tiles
                are more than SMs.  16 rows: 896 x 4,864 3.2 against 3.7, but 3,584 x 3,584 7.8
                against 6.8 and 1,536 x 8,960 7.9 against 6.7: not above 5 M.  17 to 32 rows: where one block has the whole K
-               (one plain add an element: the same bits every run, at 24 rows 1,536 x 768 2.3 against 2.4, at 32 3.0 against 2.5);
-               shared out, 24 and 32 rows of 896 x 896 take 2.8 and 3.2 against 2.4, of 896 x 4,864 4.0 and 4.3 against 3.7.
+               (one plain add an element: the same bits every run; at 24 rows 1,536 x 768 2.3 against 2.4, at 32 3.0 against 2.5),
+               and where the tcgen05 form's tiles are few or short: up to 128 rows of w (128 x 8,192 17 rows 2.6 against 3.0, 32
+               rows 3.2 and 3.2) or 600,000 weights (256 x 1,024 2.0 against 2.4, 32 rows 2.4 and 2.4); else not: 24 and 32 rows
+               of 896 x 896 2.8 and 3.2 against 2.4, of 896 x 4,864 4.0 and 4.3 against 3.6.
                A whole K of up to 14 units is a warp a unit (1,024 x 256, 8 and 16 rows: 1.8 and 2.3, two units a warp 2.2 and
                3.3), and left to the tcgen05 form where so few warps take long over the outputs of the rows (1,024 x 128: 8
                rows 2.2 against 2.3, 9 rows 2.8 against 2.3; 1,024 x 256: 24 rows 3.0 against 3.1, 32 rows 3.5 against 3.2).
@@ -1652,7 +1654,7 @@ def gemm_few_plan(n_tok: int, n_out: int, k: int, epilogue: int, n_sms: int) -> 
         uw = 1 if short or per <= 2 else max(2, (per + 13) // 14)
         if uw > 2:
             return None
-        if splits > 1 and n_tok > 16:
+        if n_tok > 16 and splits > 1 and n_out > 128 and n_out * k > 600_000:
             return None
         if splits == 1:
             rounds = (tiles + n_sms - 1) // n_sms

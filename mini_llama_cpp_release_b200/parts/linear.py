@@ -36,20 +36,7 @@ SMALL_BATCH = 64          # up to this many rows a plain product runs on the tcg
 MAX_SPLITS = 8            # partial sums the consumer has to add
 ADD_MAX_SPLITS = 24       # splits of a product that adds into the stream atomically (nobody has to add them up)
 ADD_MAX_SPLITS_SOME = 10  # the same for 2 to 16 rows
-ADD_MAX_SPLITS_MORE = 12  # the same for 17 to 64 rows
-
-
-def add_split_cap(n_tok: int) -> int:
-    """The most blocks that share the K range of a few-row product that adds into the stream.  More blocks stream the
-    weights faster, but every block adds its part with one atomic per row and column, and its blocks are SMs on which
-    the kernel after it cannot start early to ask for its own weights.  Measured on whole decode steps of 24 and 28
-    layers on a B200, caps of 8 / 10 / 12 / 24: 0.733 / 0.710 / 0.717 / 0.722 ms at 8 rows and 1.271 against 1.300 ms
-    (10 against 24) at 16 rows of the Qwen2-1.5B sizes, but 0.735 / 0.703 / 0.704 / 0.683 ms at one row and
-    1.039 / 1.044 / 1.016 / 1.009 ms at 64 rows; at the 7B sizes the cap does not bind.  With issues through elect.sync (us in a
-    chain, 64 rows): 896 x 4,864 3.60 with 10 splits, 3.84 with 19; 1,536 x 8,960 6.81 with 10, 6.51 with 12, 6.71 with 24."""
-    if n_tok < 2:
-        return ADD_MAX_SPLITS
-    return ADD_MAX_SPLITS_SOME if n_tok <= 16 else ADD_MAX_SPLITS_MORE
+ADD_SPLIT_STEPS = 8       # 64-element K steps that a split of 17 to 64 rows has at least, once half of the SMs have one
 
 
 def split_count(n_out: int, k: int, n_tok: int, n_sms: int, max_splits: int = 0) -> int:
@@ -62,6 +49,27 @@ def split_count(n_out: int, k: int, n_tok: int, n_sms: int, max_splits: int = 0)
     s = max(1, min(n_sms // max(1, row_tiles), k_blocks // 2, max_splits or MAX_SPLITS))
     per = (k_blocks + s - 1) // s
     return (k_blocks + per - 1) // per
+
+
+def add_split_count(n_out: int, k: int, n_tok: int, n_sms: int) -> int:
+    """The blocks that share the K range of a product of up to 64 rows that adds into the stream.  More blocks stream the weights
+    faster, but every block adds its part with one atomic per row and column, and its blocks are SMs on which the kernel after it
+    cannot start early to ask for its own weights.
+
+    Up to 16 rows, measured on whole decode steps of 24 and 28 layers on a B200, caps of 8 / 10 / 12 / 24: 0.733 / 0.710 / 0.717 /
+    0.722 ms at 8 rows and 1.271 against 1.300 ms (10 against 24) at 16 rows of the Qwen2-1.5B sizes, but 0.735 / 0.703 / 0.704 /
+    0.683 ms at one row; at the 7B sizes the cap does not bind.
+
+    17 to 64 rows: as many as fill half of the SMs, and more only where each still has eight K steps.  us in a chain, weights from
+    memory, 32 rows (17 to 64 alike): 896 x 4,864 10 splits 3.63, 7 4.56, 19 4.00; 1,536 x 1,536 6 2.93, 12 3.27; 2,048 x 2,048 4 3.65,
+    8 3.92; 4,096 x 1,024 2 3.56, 4 4.01; 1,280 x 5,120 10 4.30, 7 4.81, 14 4.61; 1,024 x 8,192 16 5.12, 9 5.63; 256 x 8,192 22 3.20,
+    12 4.18; 512 x 4,096 16 2.92, 11 3.18; 1,536 x 8,960 (the SMs allow 12) 6.55, 6 7.27."""
+    if n_tok <= 16:
+        cap = ADD_MAX_SPLITS if n_tok < 2 else ADD_MAX_SPLITS_SOME
+    else:
+        tiles = (n_out + 127) // 128
+        cap = min(ADD_MAX_SPLITS, max(1, n_sms // (2 * tiles), (k + 63) // 64 // ADD_SPLIT_STEPS))
+    return split_count(n_out, k, n_tok, n_sms, max_splits=cap)
 
 
 class Linear:
@@ -109,7 +117,7 @@ class Linear:
         if (plan := self.few_plan(m, kernels.bindings.EPI_ADD)) is not None:
             kernels.gemm_few(x, self.weight, stream, kernels.bindings.EPI_ADD, plan)
             return
-        splits = split_count(self.out_features, self.in_features, m, self.runtime.n_sms, max_splits=add_split_cap(m))
+        splits = add_split_count(self.out_features, self.in_features, m, self.runtime.n_sms)
         kernels.gemm_tcgen05(x, self.weight, stream, kernels.bindings.EPI_ADD, splits, n_sms=self.runtime.n_sms)
 
     def __call__(self, x: torch.Tensor, out_dtype: torch.dtype = torch.float32, partial_ok: bool = False) -> torch.Tensor:

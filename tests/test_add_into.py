@@ -36,6 +36,25 @@ def test_larger_products_leave_the_few_row_form_at_17_rows(monkeypatch):
             assert route(monkeypatch, n_tok, n_out, k)[0] == "tcgen05"
 
 
+@pytest.mark.parametrize("n_out,k", [(128, 8192), (64, 2048), (256, 1024), (512, 1024)])
+def test_products_with_few_weights_stay_in_the_few_row_form(monkeypatch, n_out, k):
+    for n_tok in (17, 32):
+        assert route(monkeypatch, n_tok, n_out, k)[0] == "few"
+
+
+@pytest.mark.parametrize("n_out,k,splits", [(256, 8192, 22), (512, 4096, 16), (128, 8192, 22), (896, 4864, 10), (1536, 1536, 6), (1536, 8960, 12),
+                                            (2048, 2048, 4), (3584, 3584, 5), (1000, 136, 1), (896, 896, 7), (151936, 896, 1), (2, 8, 1)])
+def test_blocks_that_share_an_inner_size(monkeypatch, n_out, k, splits):
+    """33 to 64 rows: half of the SMs or eight K steps a block, whichever are more blocks; never an empty one."""
+    for n_tok in (33, 64):
+        assert route(monkeypatch, n_tok, n_out, k) == ("tcgen05", splits)
+    steps = (k + 63) // 64
+    for n_sms in (148, 132, 16, 1):
+        for n_tok in (1, 2, 16, 17, 64):
+            n = linear.add_split_count(n_out, k, n_tok, n_sms)
+            assert 1 <= n <= steps and (n - 1) * -(-steps // n) < steps
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_out,k", [(512, 512), (896, 896), (896, 4864), (208, 1000), (130, 1024), (1536, 768)])
 @pytest.mark.parametrize("n_tok", [1, 16, 17, 24, 32, 33, 63, 64, 65])
