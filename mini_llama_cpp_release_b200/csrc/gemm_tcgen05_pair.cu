@@ -23,7 +23,9 @@ namespace mlc {
 template <int BN, int EPI> struct PairShape {
     static constexpr int B_BYTES = (BN / 2) * R_BK * 2;              // this block's half of the W tile
     static constexpr int STAGE_BYTES = R_A_BYTES + B_BYTES;
-    static constexpr int OUT_BYTES = (EPI == R_EPI_ADD) ? 8 * 2 * R_OUT_BYTES : 0;       // two tiles on their way out per epilogue warp
+    // A tile on its way out per epilogue warp.  One and not two: the ring then has six stages of the widest tiles and not five, which long
+    // inner sizes need.  B200, us, two and one: 8,191 tokens 3,584 x 18,944 932, 877; 1,536 x 8,960 195, 181; 2,048 tokens 45.3, 42.0.
+    static constexpr int OUT_BYTES = (EPI == R_EPI_ADD) ? 8 * R_OUT_BYTES : 0;
     static constexpr int STAGES_FIT = (227 * 1024 - 512 - 1024 - OUT_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_FIT < 7 ? STAGES_FIT : 7;
     static constexpr int THREADS = 64 + 256;
@@ -32,7 +34,7 @@ template <int BN, int EPI> struct PairShape {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_BYTES + BAR_BYTES + 1024 /* alignment slack */;
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a block");
     static_assert(BN % 32 == 0 && BN >= 128 && BN <= 256, "rows of W per tile");
-    static_assert(STAGES >= 3 && STAGES <= 8, "stage ring");
+    static_assert(STAGES >= 6 && STAGES <= 8, "stage ring");
 };
 
 // A remote arrival (mbar_arrive_remote) without ordering of this thread's own earlier writes (it has none to publish): what the arrival reports was
@@ -201,8 +203,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         constexpr int COLS_PER_GROUP = WHOLE ? (BN / 32 + 1) / 2 * 32 : BN / 2;
         const int cols = WHOLE ? min(COLS_PER_GROUP, BN - eg * COLS_PER_GROUP) : COLS_PER_GROUP;
         grid_dependency_wait();                // the output may come from earlier kernels
-        const unsigned out_buf = base + out_off + (unsigned)((warp - 2) * 2 * R_OUT_BYTES);
-        int j = 0, n_out_tiles = 0;
+        const unsigned out_buf = base + out_off + (unsigned)((warp - 2) * R_OUT_BYTES);
+        int j = 0;
         bool ok = true;
         for (int t = pair; t < n_tiles_total && ok; t += n_pairs, ++j) {
             const TileWalk at = tile_walk(g, t);
@@ -223,10 +225,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_load32(t_addr + (unsigned)c0, v);
                 if constexpr (EPI == R_EPI_ADD) {
                     if (m0 + q * 32 >= g.n_tok) break;
-                    // the buffer of two chunks before has been read (the warp's first lane asked for both copies)
-                    if (lane == 0) tma_store_wait_read<1>();
+                    if (lane == 0) tma_store_wait_read<0>();           // the warp's tile before has been read
                     __syncwarp();
-                    rows_tile_out<EPI>(&map_out, v, out_buf + (unsigned)((n_out_tiles++ & 1) * R_OUT_BYTES), lane, n, m0 + q * 32);
+                    rows_tile_out<EPI>(&map_out, v, out_buf, lane, n, m0 + q * 32);
                 } else {
                     const bool second = n + 16 < g.n_out && c0 + 32 <= COLS_PER_GROUP;
                     if (!tok_ok) continue;
