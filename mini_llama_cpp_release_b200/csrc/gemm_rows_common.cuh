@@ -74,8 +74,8 @@ __device__ __forceinline__ unsigned pack2(float a, float b) {
 }
 
 // Tile number t of a product.  Consecutive blocks take tiles that share one operand's piece, which is then fetched from memory
-// once by all of them together, while the other operand is walked whole for each such piece: it comes from L2 if it fits there,
-// so it is the smaller one (n_first: W is).
+// once by all of them together, while the other operand is walked whole for each such piece, out of L2 if it stays there
+// (n_first: the shared pieces are x's).
 struct TileWalk {
     int m, n, split;
 };
@@ -87,6 +87,17 @@ __device__ __forceinline__ TileWalk tile_walk(const RowsArgs& g, int t) {
     w.n = g.n_first ? i : o;
     w.split = r / outer;
     return w;
+}
+
+// Whether a product's walk shares x's pieces and goes through W for each of them (n_first).  That pays where x does not stay in
+// L2 from one piece of W to the next: beyond some 60 MB, half of the 126 MB that two dies share; an adding product's output is
+// fetched and written there too and counts half.  Below, sharing W's pieces is as fast or faster.  B200, us, W's pieces shared
+// and x's: QKV 1,536 x 512 2,048 tokens 14.8, 17.4; 4,608 x 3,584 8,191 (59 MB) 265, 267, 16,384 641, 548; STORE 1,152 x 896
+// 16,384 (29 MB) 31.8, 34.0; 4,096 x 4,096 8,191 (67 MB) 203, 198, 16,384 424, 351; ADD 1,536 x 1,536 8,191 (25 + 25 MB) 33.0,
+// 33.5; 2,560 x 2,560 4,500 (23 + 23 MB) 47.6, 49.5, 16,384 191, 174; 896 x 4,864 8,191 (80 + 15 MB) 63.7, 60.7; 2,048 x 512
+// 16,384 (17 + 67 MB) 66.0, 59.7.
+static bool walk_shares_x(long long n_tok, long long n_out, long long K, int epilogue) {
+    return n_tok > n_out && n_tok * K * 2 + (epilogue == R_EPI_ADD ? n_tok * n_out * 2 : 0) > 60000000;
 }
 
 // A warp's 32 tokens x 32 accumulator columns on their way into a float32 output through `buf`, 4 KiB of shared memory of

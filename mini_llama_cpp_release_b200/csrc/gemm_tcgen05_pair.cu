@@ -326,7 +326,7 @@ extern "C" int mlc_gemm_tcgen05_pair(const void* x, const void* w, void* out, in
     g.n_splits = n_splits;
     g.k_blocks_per_split = (g.k_blocks + n_splits - 1) / n_splits;
     if ((long long)(n_splits - 1) * g.k_blocks_per_split >= g.k_blocks) return MLC_ERR_BAD_SIZE;   // an empty split
-    g.n_first = n_tok > n_out;                 // x has more rows than W: see tile_walk
+    g.n_first = walk_shares_x(n_tok, n_out, K, epilogue);
     g.status = status;
     CUtensorMap mx, mw, mo;
     int rc = cached_map_2d(&mx, x, n_tok, K, R_BK, R_BM);

@@ -37,3 +37,50 @@ def test_added_and_stored_tiles(form, width, n_tok, n_out, k):
     assert float((out[:n_tok].double() - want).abs().max()) <= TOL * float(want.abs().max())
     assert torch.equal(out[n_tok], before[n_tok])
     kernels.check_gemm_status(torch.device(DEV))
+
+
+# x of 60.2 MB: its pieces are shared by consecutive blocks; of half as many tokens W's are
+LONG, LONG_K = 30100, 1000
+
+
+@pytest.mark.parametrize("epilogue", [bindings.EPI_STORE, bindings.EPI_SILU_MUL, bindings.EPI_ADD])
+@pytest.mark.parametrize("form,width", [("rows", 128), ("rows", 224), ("pair", 256)])
+def test_both_walks_give_the_same_bits(form, width, epilogue):
+    """An output's sum runs over K in the same order wherever its tile stands: all tokens at once and half of them at a time agree."""
+    n_out, half = 208, LONG // 2
+    g = torch.Generator().manual_seed(5)
+    x = (torch.randn(LONG, LONG_K, generator=g) * 0.5).bfloat16().to(DEV)
+    w = (torch.randn(n_out, LONG_K, generator=g) * 0.1).bfloat16().to(DEV)
+    run = kernels.gemm_tcgen05_pair if form == "pair" else kernels.gemm_tcgen05_rows
+    before = torch.randn(LONG, n_out // 2 if epilogue == bindings.EPI_SILU_MUL else n_out, device=DEV)
+    whole, parts = before.clone(), before.clone()
+    run(x, w, whole, epilogue, width, 1)
+    for part in (slice(0, half), slice(half, LONG)):
+        run(x[part], w, parts[part], epilogue, width, 1)
+    kernels.check_gemm_status(torch.device(DEV))
+    assert torch.equal(whole, parts)
+    if epilogue == bindings.EPI_STORE:
+        want = x.double() @ w.double().T
+        assert float((whole.double() - want).abs().max()) <= TOL * float(want.abs().max())
+
+
+def test_both_walks_of_the_qkv_product_give_the_same_bits():
+    H, KV, hd, half = 4, 1, 64, LONG // 2
+    g = torch.Generator().manual_seed(6)
+    x = (torch.randn(LONG, LONG_K, generator=g) * 0.5).bfloat16().to(DEV)
+    w = (torch.randn((H + 2 * KV) * hd, LONG_K, generator=g) * 0.1).bfloat16().to(DEV)
+    pos = torch.arange(LONG, dtype=torch.int32, device=DEV)
+    seq = torch.zeros(LONG, dtype=torch.int32, device=DEV)
+    rope = torch.randn(LONG, hd // 2, 2, generator=g).to(DEV)
+    pages = (LONG + 63) // 64
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, pages)
+    got = []
+    for cuts in ((0, LONG), (0, half, LONG)):
+        kv = kernels.KVView(*(torch.zeros(1, pages, KV, 64, hd, dtype=torch.bfloat16, device=DEV) for _ in range(2)), 0, table, 64, KV, hd)
+        q = torch.empty(LONG, H * hd, dtype=torch.bfloat16, device=DEV)
+        for a, b in zip(cuts, cuts[1:]):
+            kernels.gemm_tcgen05_rows(x[a:b], w, q[a:b], bindings.EPI_QKV, positions=pos[a:b], tok_seq=seq[a:b], rope=rope, q_heads=H,
+                                      kv_heads=KV, head_dim=hd, kv=kv)
+        got.append((q, kv.k_pool, kv.v_pool))
+    kernels.check_gemm_status(torch.device(DEV))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and bool(got[0][1].any()) and bool(got[0][2].any())
