@@ -36,7 +36,7 @@ SMALL_BATCH = 64          # up to this many rows a plain product runs on the tcg
 MAX_SPLITS = 8            # partial sums the consumer has to add
 ADD_MAX_SPLITS = 24       # splits of a product that adds into the stream atomically (nobody has to add them up)
 ADD_MAX_SPLITS_SOME = 10  # the same for 2 to 16 rows
-ADD_SPLIT_STEPS = 8       # 64-element K steps that a split of 17 to 64 rows has at least, once half of the SMs have one
+ADD_SPLIT_STEPS = 7       # 64-element K steps that no split of 17 to 64 rows has more of, where the SMs allow it
 
 
 def split_count(n_out: int, k: int, n_tok: int, n_sms: int, max_splits: int = 0) -> int:
@@ -60,15 +60,17 @@ def add_split_count(n_out: int, k: int, n_tok: int, n_sms: int) -> int:
     0.722 ms at 8 rows and 1.271 against 1.300 ms (10 against 24) at 16 rows of the Qwen2-1.5B sizes, but 0.735 / 0.703 / 0.704 /
     0.683 ms at one row; at the 7B sizes the cap does not bind.
 
-    17 to 64 rows: as many as fill half of the SMs, and more only where each still has eight K steps.  us in a chain, weights from
-    memory, 32 rows (17 to 64 alike): 896 x 4,864 10 splits 3.63, 7 4.56, 19 4.00; 1,536 x 1,536 6 2.93, 12 3.27; 2,048 x 2,048 4 3.65,
-    8 3.92; 4,096 x 1,024 2 3.56, 4 4.01; 1,280 x 5,120 10 4.30, 7 4.81, 14 4.61; 1,024 x 8,192 16 5.12, 9 5.63; 256 x 8,192 22 3.20,
-    12 4.18; 512 x 4,096 16 2.92, 11 3.18; 1,536 x 8,960 (the SMs allow 12) 6.55, 6 7.27."""
+    17 to 64 rows: as many as fill half of the SMs, and more while a block has more than seven K steps.  Whole decode steps, us:
+    896 x 4,864 at the 0.5B sizes with 10 / 11 / 13 / 19 splits 20 rows 655 / 636 / 644 / 641, 48 rows 719 / 704 / 702 / 714, 64 rows
+    741 / 735 / 730 / 725; 1,536 x 1,536 at the 1.5B sizes with 4 / 6 / 8 / 12 20 rows 1,193 / 1,174 / 1,172 / 1,190, 64 rows 1,266 /
+    1,270 / 1,269 / 1,292.  us in a chain, weights from memory, 32 rows (17 to 64 alike): 2,048 x 2,048 5 splits 3.56, 8 3.92; 4,096 x
+    1,024 2 3.56, 4 4.01; 1,024 x 8,192 16 5.12, 9 5.63; 256 x 8,192 22 3.20, 12 4.18; 512 x 4,096 16 2.92, 11 3.18; 1,536 x 8,960
+    (the SMs allow 12) 6.55, 6 7.27."""
     if n_tok <= 16:
         cap = ADD_MAX_SPLITS if n_tok < 2 else ADD_MAX_SPLITS_SOME
     else:
         tiles = (n_out + 127) // 128
-        cap = min(ADD_MAX_SPLITS, max(1, n_sms // (2 * tiles), (k + 63) // 64 // ADD_SPLIT_STEPS))
+        cap = min(ADD_MAX_SPLITS, max(n_sms // (2 * tiles), -(-((k + 63) // 64) // ADD_SPLIT_STEPS)))
     return split_count(n_out, k, n_tok, n_sms, max_splits=cap)
 
 
@@ -97,13 +99,13 @@ class Linear:
         return out
 
     def can_add_into_stream(self, n_rows: int) -> bool:
-        """Whether `add_into` has a kernel for these operands: the tcgen05 products (atomic adds for few rows; plain or
-        atomic adds for more), else the library's product with the stream as the matrix it adds to."""
+        """Whether `add_into` has a kernel for these operands: the few-row and tcgen05 products (plain or atomic adds for
+        few rows, adding copies by TMA for more), else the library's product with the stream as the matrix it adds to."""
         return self.tensor_core_ok
 
     def add_into(self, x: torch.Tensor, stream: torch.Tensor) -> None:
-        """stream (float32 [n, out]) += x · Wᵀ.  Few rows: the weights-as-M tcgen05 product, the K range shared out over
-        as many blocks as is useful.  More rows: the tokens-as-M tcgen05 product, with a K split when its tiles alone
+        """stream (float32 [n, out]) += x · Wᵀ.  Few rows: the few-row product where it has a plan, else the weights-as-M tcgen05
+        product, the K range shared out over as many blocks as is useful.  More rows: the tokens-as-M tcgen05 product, with a K split when its tiles alone
         would leave SMs idle (the library's product only for a row count that kernel does not take: no multiple of
         16).  Either way the stream is updated in the product's epilogue, so the norm that follows has one tensor to
         read, not two."""

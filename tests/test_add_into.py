@@ -42,10 +42,10 @@ def test_products_with_few_weights_stay_in_the_few_row_form(monkeypatch, n_out, 
         assert route(monkeypatch, n_tok, n_out, k)[0] == "few"
 
 
-@pytest.mark.parametrize("n_out,k,splits", [(256, 8192, 22), (512, 4096, 16), (128, 8192, 22), (896, 4864, 10), (1536, 1536, 6), (1536, 8960, 12),
-                                            (2048, 2048, 4), (3584, 3584, 5), (1000, 136, 1), (896, 896, 7), (151936, 896, 1), (2, 8, 1)])
+@pytest.mark.parametrize("n_out,k,splits", [(256, 8192, 22), (512, 4096, 16), (128, 8192, 22), (896, 4864, 11), (1536, 1536, 6), (1536, 8960, 12),
+                                            (2048, 2048, 5), (3584, 3584, 5), (1000, 136, 1), (896, 896, 7), (151936, 896, 1), (2, 8, 1)])
 def test_blocks_that_share_an_inner_size(monkeypatch, n_out, k, splits):
-    """33 to 64 rows: half of the SMs or eight K steps a block, whichever are more blocks; never an empty one."""
+    """33 to 64 rows: half of the SMs or seven K steps a block, whichever are more blocks; never an empty one."""
     for n_tok in (33, 64):
         assert route(monkeypatch, n_tok, n_out, k) == ("tcgen05", splits)
     steps = (k + 63) // 64
@@ -77,3 +77,21 @@ def test_added_products_on_both_sides_of_the_lines(n_tok, n_out, k):
     if plan is not None and plan[4] == 1:
         assert all(torch.equal(o, outs[0]) for o in outs[1:])
     kernels.check_gemm_status(torch.device("cuda"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_tok,n_out,k,splits", [(17, 896, 4864, 11), (24, 896, 4864, 10), (32, 896, 896, 7), (32, 208, 1000, 6), (33, 896, 4864, 11),
+                                                  (63, 200, 1000, 8), (17, 130, 128, 1), (24, 300, 200, 2), (32, 1536, 1536, 12)])
+def test_the_tcgen05_form_with_shared_inner_sizes(n_tok, n_out, k, splits):
+    """Tiles of 32 and 64 tokens: a last split shorter than the others, splits of fewer K steps than threads that issue them, rows of w that
+    are no multiple of 128.  Tolerance as above."""
+    g = torch.Generator().manual_seed(n_tok + n_out + k)
+    x = (torch.randn(n_tok, k, generator=g) * 0.5).bfloat16().cuda()
+    w = (torch.randn(n_out, k, generator=g) * 0.3).bfloat16().cuda()
+    before = torch.randn(n_tok + 1, n_out, generator=g).cuda()
+    stream = before.clone()
+    kernels.gemm_tcgen05(x, w, stream[:n_tok], kernels.bindings.EPI_ADD, splits)
+    kernels.check_gemm_status(torch.device("cuda"))
+    want = before[:n_tok].double() + x.double() @ w.double().T
+    assert float((stream[:n_tok].double() - want).abs().max()) <= 3e-6 * float(want.abs().max())
+    assert torch.equal(stream[n_tok], before[n_tok])
