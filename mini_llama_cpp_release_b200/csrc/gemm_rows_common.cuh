@@ -89,26 +89,24 @@ __device__ __forceinline__ TileWalk tile_walk(const RowsArgs& g, int t) {
     return w;
 }
 
-// Whether a product's walk shares x's pieces and goes through W for each of them (n_first).  That pays where x does not stay in
-// L2 from one piece of W to the next: beyond some 60 MB, half of the 126 MB that two dies share; an adding product's output is
-// fetched and written there too and counts half.  Below, sharing W's pieces is as fast or faster.  B200, us, W's pieces shared
-// and x's: QKV 1,536 x 512 2,048 tokens 14.8, 17.4; 4,608 x 3,584 8,191 (59 MB) 265, 267, 16,384 641, 548; STORE 1,152 x 896
-// 16,384 (29 MB) 31.8, 34.0; 4,096 x 4,096 8,191 (67 MB) 203, 198, 16,384 424, 351; ADD 1,536 x 1,536 8,191 (25 + 25 MB) 33.0,
-// 33.5; 2,560 x 2,560 4,500 (23 + 23 MB) 47.6, 49.5, 16,384 191, 174; 896 x 4,864 8,191 (80 + 15 MB) 63.7, 60.7; 2,048 x 512
-// 16,384 (17 + 67 MB) 66.0, 59.7.
+// Whether a product's walk shares x's pieces and goes through W for each of them (n_first).  An adding product's does where x has
+// more rows than W: its output is fetched and written in L2 too, and consecutive blocks then work on the same tokens' rows.  B200,
+// us, W's pieces shared and x's: 2,048 x 512 16,384 tokens 66.0, 59.7; 896 x 4,864 8,191 63.7, 60.7, 16,384 141, 121; whole prompts
+// of the 0.5B sizes of 2,048 tokens 2,366, 2,349 (1,000 to 4,500 tokens by themselves the other way, by 2 %).  The others' does
+// where x does not stay in L2 from one piece of W to the next, beyond some 60 MB, half of the 126 MB that two dies share: STORE
+// 4,096 x 4,096 8,191 (67 MB) 203, 198, 16,384 424, 351; QKV 4,608 x 3,584 8,191 (59 MB) 265, 267, 16,384 641, 548; but QKV
+// 1,536 x 512 2,048 14.8, 17.4; STORE 1,152 x 896 16,384 (29 MB) 31.8, 34.0.
 static bool walk_shares_x(long long n_tok, long long n_out, long long K, int epilogue) {
-    return n_tok > n_out && n_tok * K * 2 + (epilogue == R_EPI_ADD ? n_tok * n_out * 2 : 0) > 60000000;
+    return n_tok > n_out && (epilogue == R_EPI_ADD || n_tok * K * 2 > 60000000);
 }
 
-// A warp's 32 tokens x 32 accumulator columns on their way into a float32 output through `buf`, 4 KiB of shared memory of
-// the warp's own: a thread writes its token's 128 bytes (16-byte pieces in the order of the 128-byte swizzle, so that eight
-// lanes hit all banks), one lane hands the tile to TMA.  ADD: added to what is there, a line at a time, where 16-byte atomic adds by
-// the threads themselves touch 32 lines an instruction.  B200, us, those adds with x walked whole, and this with the walk above:
-// 16,384 tokens 896 x 4,864 143, 119; 1,536 x 8,960 381, 320; 1,536 x 1,536 103, 76; 8,191 tokens 896 x 896 19.8, 16.2; 896 x 4,864 64.3,
-// 58.4; 2,048 tokens 896 x 896 7.5, 7.0; 1,536 x 8,960 42.3, 40.4.
+// A warp's 32 tokens x 32 accumulator columns on their way into the float32 stream through `buf`, 4 KiB of shared memory of the
+// warp's own: a thread writes its token's 128 bytes (16-byte pieces in the order of the 128-byte swizzle, so that eight lanes hit
+// all banks), one lane hands the tile to TMA, which adds a line at a time; 16-byte atomic adds by the threads themselves touch 32
+// lines an instruction.  B200, us, those adds and these, the same walk: 896 x 4,864 512 tokens 8.7, 7.9, 2,048 18.2, 17.2; 896 x
+// 896 8,191 19.7, 15.9; 1,536 x 1,536 2,048 19.7, 17.4; 2,048 x 512 8,191 36.9, 26.6.
 constexpr int R_OUT_BYTES = 32 * 32 * 4;
-template <int EPI>
-__device__ __forceinline__ void rows_tile_out(const CUtensorMap* map, const float (&v)[32], unsigned buf, int lane, int n, int tok0) {
+__device__ __forceinline__ void rows_tile_add(const CUtensorMap* map, const float (&v)[32], unsigned buf, int lane, int n, int tok0) {
 #pragma unroll
     for (int u = 0; u < 8; ++u)
         asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 128 + ((u ^ (lane & 7)) << 4)), "f"(v[4 * u]),
@@ -116,8 +114,7 @@ __device__ __forceinline__ void rows_tile_out(const CUtensorMap* map, const floa
     fence_async_shared();
     __syncwarp();
     if (lane == 0) {
-        if (EPI == R_EPI_ADD) tma_add_2d(map, n, tok0, buf);
-        else tma_store_2d(map, n, tok0, buf);
+        tma_add_2d(map, n, tok0, buf);
         tma_store_commit();
     }
 }

@@ -227,7 +227,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     if (m0 + q * 32 >= g.n_tok) break;
                     if (lane == 0) tma_store_wait_read<0>();           // the warp's tile before has been read
                     __syncwarp();
-                    rows_tile_out<EPI>(&map_out, v, out_buf, lane, n, m0 + q * 32);
+                    rows_tile_add(&map_out, v, out_buf, lane, n, m0 + q * 32);
                 } else {
                     const bool second = n + 16 < g.n_out && c0 + 32 <= COLS_PER_GROUP;
                     if (!tok_ok) continue;

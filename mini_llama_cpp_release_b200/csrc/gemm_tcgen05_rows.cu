@@ -257,7 +257,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         if (m0 + q * 32 >= g.n_tok) break;
                         if (lane == 0) tma_store_wait_read<0>();       // the warp's tile before has been read
                         __syncwarp();
-                        rows_tile_out<EPI>(&map_out, v, out_buf, lane, n, m0 + q * 32);
+                        rows_tile_add(&map_out, v, out_buf, lane, n, m0 + q * 32);
                         continue;
                     }
                     // n_out and the group's share of the tile are multiples of 16: the chunk has 16 or 32 columns

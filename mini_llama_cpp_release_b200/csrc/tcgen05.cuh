@@ -21,9 +21,8 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)_
 // True in one lane of a warp whose lanes are all here.  A role that one thread plays is entered through this and not
 // through `lane == 0`: the operands of tcgen05.mma, its commits and TMA loads are registers that a warp has once, and under
 // a branch that the compiler must take for a divergent one it has to bring them there for whichever lanes are active (some
-// sixty clocks an issue were measured, more than a 128 x 64 x 16 product takes).  Measured on a B200, lane == 0 against this: prompt
-// attention of 8,191 tokens, 14 heads of 64, 201 against 179 us, 8 x 2,048 tokens with 12 heads of 128 158 against 141; products of
-// 512 tokens 1,152 x 896 7.6 against 6.2 us, 896 x 4,864 10.5 against 8.5; 2,048 tokens 896 x 896 9.1 against 7.5.
+// sixty clocks an issue were measured, more than a 128 x 64 x 16 product takes).  B200, us, lane == 0 and this: prompt
+// attention of 8,191 tokens, 14 heads of 64, 201, 179; products of 512 tokens 896 x 4,864 10.5, 8.5.
 __device__ __forceinline__ bool elect_one() {
     unsigned p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -115,12 +114,8 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
-// A tile in shared memory leaves for a tensor in global memory, stored or (float32) added to what is there; what lies outside
-// the tensor is left out.  Copies are asked for and waited for by one thread, in groups.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int c0, int c1, unsigned src) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
-                 ::"l"(map), "r"(c0), "r"(c1), "r"(src) : "memory");
-}
+// A tile in shared memory is added (float32) to a tensor in global memory; what lies outside the tensor is left out.  Copies are
+// asked for and waited for by one thread, in groups.
 __device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, int c0, int c1, unsigned src) {
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
                  ::"l"(map), "r"(c0), "r"(c1), "r"(src) : "memory");
@@ -280,7 +275,7 @@ static PFN_cuTensorMapEncodeTiled encode_tiled() {
     return fn;
 }
 
-// A tensor of `rank` dimensions (innermost first; strides in bytes for dimensions 1...) read or written in boxes whose
+// A tensor of `rank` dimensions (innermost first; strides in bytes for dimensions 1...) read or added to in boxes whose
 // innermost extent is 128 bytes, with the 128-byte swizzle; reads outside the tensor give zeros.
 static int make_tensor_map(CUtensorMap* map, const void* ptr, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
                            const cuuint32_t* box, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
@@ -293,9 +288,9 @@ static int make_tensor_map(CUtensorMap* map, const void* ptr, int rank, const cu
     return r == CUDA_SUCCESS ? 0 : MLC_ERR_BAD_SIZE;
 }
 
-// The map of a row-major matrix [rows][cols] (bfloat16, or float32) read or written in boxes of box_rows x box_cols, remembered by what defines
-// it: a step launches hundreds of products over the same weights, and its scratch tensors come back at the same
-// addresses step after step, so the driver is asked once per matrix, not once per launch.
+// The map of a row-major matrix [rows][cols] (bfloat16, or float32) read or added to in boxes of box_rows x box_cols,
+// remembered by what defines it: a step launches hundreds of products over the same weights, and its scratch tensors come back
+// at the same addresses step after step, so the driver is asked once per matrix, not once per launch.
 static int cached_map_2d(CUtensorMap* map, const void* ptr, long long rows, long long cols, int box_cols, int box_rows, bool f32 = false) {
     struct Key {
         const void* ptr;
