@@ -331,8 +331,9 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     sc[c] = a.cap_over_scale * (1.0f - __fdividef(2.0f, 1.0f + fast_exp2(sc[c] * a.cap_exponent)));
             }
             if (masked) {
-                // Which of the row's 64 keys are seen, a bit each: two comparisons a tile where there were three a key.  B200, us: one
-                // sequence of 23 tokens, 14 heads of 64 on 2, 4.8 -> 4.3, 2,048 tokens 17.8 -> 16.3, 64 sequences of 200 57 -> 50.
+                // Which of the row's 64 keys are seen, a bit each: three bounds a tile and a bit tested a key, where each key was
+                // compared with the three.  B200, us, before and with it: one sequence of 23 tokens, 14 heads of 64 on 2, 4.8, 4.3;
+                // 2,048 tokens 17.8, 16.3; 64 sequences of 200 57, 50.
                 const unsigned long long seen = low_bits(hi - key0 + 1) & (~low_bits(lo - key0) | low_bits(keep - key0));
                 const unsigned half[2] = {(unsigned)seen, (unsigned)(seen >> 32)};
 #pragma unroll
@@ -355,7 +356,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             m = m_new;
 
             // probabilities, their sum, P as pairs of bfloat16 over the first half of the scores' columns
-            // (two keys an instruction where there is one: prompts of 8,191 tokens, 14 heads of 64, 179 -> 169 us)
+            // (two keys an instruction where there is one: prompts of 8,191 tokens, 14 heads of 64, 169 us and 179 with one)
             float2x sum[2] = {pair_of(0.0f, 0.0f), pair_of(0.0f, 0.0f)};
             const float2x scale2 = pair_of(a.scale_log2, a.scale_log2), shift2 = pair_of(-m_use, -m_use);
             unsigned pk[A_BN / 2];

@@ -1432,9 +1432,10 @@ def gemm_tcgen05_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilo
 
 def gemm_pair_takes(n_tok: int, n_out: int, k: int, n_sms: int) -> bool:
     """Whether a prompt product is better off with a pair of SMs on every tile of 256 tokens x 256 rows of w
-    (csrc/gemm_tcgen05_pair.cu): when those tiles fill the GPU at least twice over.  Measured on a B200: gate/up of
-    2,048 tokens 29.1 against 30.8 us at the Qwen2-0.5B sizes, 79 against 87 us at the 1.5B sizes, 345 against 383 us
-    at the 7B sizes (1,612 TFLOP/s); with fewer tiles than that the one-SM form, which has twice as many, wins."""
+    (csrc/gemm_tcgen05_pair.cu): when there are as many of those tiles as SMs, two for each pair.  Measured on a B200, gate/up,
+    pair against one SM, us: 2,048 tokens 28.4, 29.2 at the Qwen2-0.5B sizes, 81, 90 at the 1.5B sizes, 348, 395 at the 7B sizes;
+    8,192 tokens of the 0.5B sizes 101, 133; 512 tokens (fewer tiles) 13.8, 10.8 and 27.1, 26.4.  (At 1,000 tokens of the 0.5B
+    sizes, 152 tiles, the pair takes 18.4 against 16.1.)"""
     if n_tok <= 64 or n_out % 16 or k % 8 or n_sms < 2:
         return False
     return ((n_tok + 255) // 256) * ((n_out + 255) // 256) >= n_sms
@@ -1457,12 +1458,12 @@ def gemm_prompt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: i
         gemm_tcgen05_rows(x, w, out, epilogue, n_sms=n_sms, glu=glu)
 
 
-# What an adding prompt product costs in microseconds, by form: a launch, per K step a part that grows with the tile's
-# width and one that does not, per tile the write-out, and per megabyte of adds what the L2 takes for them.  Fitted (12 % rms) to 600 measurements on a B200: 512, 2,048 and 8,192 tokens, nine weight shapes from
-# 896 x 896 to 4,096 x 11,008, every width and split below; the plan it picks was the fastest measured one in half of
-# the 27 cases.  Since then the adds leave by TMA and cost half of what the constants say, but the choice holds: over 34 cases of 100 to
-# 16,384 tokens it is 1.2 % slower than the fastest on average, at most 7 % (4,088 tokens 896 x 4,864: 30.2 against 28.1 us);
-# constants fitted anew choose worse (2.2 %, at most 12 %).
+# What ranks the plans of an adding prompt product, by form: a launch, per K step a part that grows with the tile's width and one that
+# does not, per tile the write-out, and per megabyte of adds what the L2 takes for them.  The constants were fitted to times of
+# tiles written by atomic adds; the adds by TMA cost about half of their terms, so the sums are no longer microseconds, but they rank
+# as well: over 47 cases on a B200 (100 to 16,384 tokens, 896 x 896 to 3,584 x 18,944) the plan picked is 0.6 % slower than the
+# fastest of the twenty best-ranked on average, at most 7 % (1,000 tokens 3,584 x 3,584: 23.3 against 21.8 us), and constants
+# fitted anew to tiles by TMA chose worse.
 _ADD_COST = {"rows": (128, 1, 2.34, 0.00090, 0.183, 2.19, 0.372),
              "pair": (256, 2, 3.41, 0.00061, 0.219, 2.24, 0.360)}
 _ADD_WIDTHS = {"rows": (128, 160, 192, 224, 256), "pair": (192, 224, 256)}
@@ -1497,8 +1498,9 @@ def gemm_rows_add_plan(n_tok: int, n_out: int, k: int, n_sms: int):
 @functools.lru_cache(maxsize=4096)
 def gemm_add_plan(n_tok: int, n_out: int, k: int, n_sms: int):
     """("rows" or "pair", rows of W per tile, K splits): the cheapest plan of either form by the fitted costs above.
-    The paired form wins from about 1,536 columns at 2,048 tokens on (43 against 47 us for 1,536 x 8,960, 198 against
-    206 us for 3,584 x 18,944) and everywhere at 8,192 tokens; below that the one-SM form has the tiles to fill the GPU."""
+    The paired form wins from about 1,536 columns at 2,048 tokens on (57 against 59 us for 1,536 x 8,960, 220 against 248 us for
+    3,584 x 18,944), at 8,192 tokens from long inner sizes on (896 x 4,864 62.5 against 67.6; 896 x 896 22.0 against 22.3, where
+    the one-SM form is picked); below that the one-SM form has the tiles to fill the GPU."""
     best = ("rows",) + tuple(gemm_rows_add_plan(n_tok, n_out, k, n_sms))
     if n_sms >= 2 and n_tok > 64 and n_out % 16 == 0 and k % 8 == 0:
         rows_cost = min(_add_plans("rows", n_tok, n_out, k, n_sms))[0]

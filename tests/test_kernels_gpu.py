@@ -502,7 +502,7 @@ def test_prompt_product_with_bias_rotation_and_cache_write(H, KV, hd, T, bn):
                                               (300, 464, 200, 224, 1), (2048, 896, 896, None, None), (300, 272, 1000, 160, 3),
                                               (129, 48, 4864, 128, 8), (1000, 896, 4864, 224, 5), (70, 144, 520, 128, 2)])
 def test_prompt_product_adding_into_the_stream(T, N, K, bn, splits):
-    """16-byte atomic adds into the stream, with and without a K split (given, or chosen by the plan when the tiles
+    """TMA's adding copies into the stream, with and without a K split (given, or chosen by the plan when the tiles
     alone would leave SMs idle).  A last split shorter than the others, tiles beyond the matrix's edge in both
     directions, more tiles than blocks."""
     g = torch.Generator().manual_seed(N + K)
