@@ -220,7 +220,8 @@ class DecodeRunner:
         """Copy the page tables again if any sequence's pages are not the ones copied last (it got or lost a page, or
         its slot was given back and taken again by another sequence); returns bytes copied.  Only the rows that changed
         are written anew: of 64 sequences of unequal lengths one gets a page at nearly every step, and the device stands idle
-        meanwhile (24 tokens each for 64 short prompts: 40.5 -> 30.8 ms with the products' tiles by TMA, most of it here)."""
+        meanwhile (64 ragged prompts of up to 384 tokens and 24 tokens each, 0.5B sizes, B200: 30.8 ms, and 39.9 with every row
+        written through small tensors)."""
         version = self.cache.page_version
         slots = self._padded_slots
         rows = [b for b, s in enumerate(slots) if self.page_versions[b] != version[s]]
